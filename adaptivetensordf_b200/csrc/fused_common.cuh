@@ -11,7 +11,7 @@
 namespace atdf {
 
 constexpr int kSegItem = 128;         // segments per work item
-constexpr int kLineWin = 64;          // line-gradient window entries per line
+constexpr int kMinItem = 8;           // smallest share of a slot that becomes an item
 constexpr int kSegTabArrays = 17;     // per-segment arrays of the per-item segment table
 constexpr int kSegMapCap = 4096;      // samples of an item covered by the sample -> segment map
 constexpr int kSegTabFloats = kSegTabArrays * (kSegItem + 4) + 16 + kSegMapCap / 4;  // + the item's box, the map
@@ -75,7 +75,7 @@ static size_t ws_layout(int64_t R, int max_depth, int64_t nslot, char* base, Ws*
     x.slot_cursor = (int32_t*)carve(p, (nslot + 1) * 4);
     x.item_offset = (int32_t*)carve(p, (nslot + 2) * 4);
     x.counters = (int32_t*)carve(p, 8 * 4);
-    x.item_queue = (int2*)carve(p, (nslot + 3 + cap / kSegItem) * 8);
+    x.item_queue = (int2*)carve(p, (nslot + 3 + cap / kMinItem) * 8);
     x.cap = cap;
     x.nslot = nslot;
     if (w) *w = x;
@@ -167,6 +167,7 @@ struct FusedParams {
     int plane_off[4];    // element offsets of the three planes in shared memory (+ total)
     int plane_pitch[3];  // texels per shared-memory row of each plane (>= plane_w)
     int gplane_off[4];   // float offsets of the unpadded FP32 plane-gradient copy (+ total)
+    int line_rep;      // FP32 adjoint: copies of the line gradients in the workspace (0: none)
     float roi_inv;     // 1 / (roi_max.x - roi_min.x) when a power of two, else 0
     // Caller-placed samples (null: the uniform per-node rule): t and weight
     // of every sample in canonical order, indexed by the ray's sample offset
@@ -282,10 +283,11 @@ __device__ __forceinline__ void init_item_queue(int* s_ctl)
     s_ctl[7] = 0;
 }
 
-// by_item (the forwards, which keep no per-slot state between items): work
-// is handed out by item from the item queue (the slot queue's order, each
-// slot's items in a row), so the items of a large slot spread over several
-// CTAs; a CTA stages a slot's planes when its next item is of another slot.
+// by_item (kernels that keep no per-slot state between items): work is handed
+// out by item from the item queue (the slot queue's order, each slot's items
+// in a row), so the items of a large slot spread over several CTAs; a CTA
+// stages a slot's planes when its next item is of another slot. bar null: the
+// kernel reads the planes from global memory, nothing is staged.
 __device__ __forceinline__ ItemInfo next_item(const FusedParams& p, int queue, float* sm, SegTab tab, uint64_t* bar,
                                               int* s_ctl, bool want_dI, int map_cap = kSegMapCap,
                                               bool by_item = false)
@@ -303,7 +305,7 @@ __device__ __forceinline__ ItemInfo next_item(const FusedParams& p, int queue, f
                 if (slot != s_ctl[4]) {
                     s_ctl[4] = slot;
                     flags |= 1;
-                    if (slot < w.nslot) {
+                    if (slot < w.nslot && bar) {
                         const int esz = p.field.dtype == ATDF_BF16 ? 2 : 4;
                         uint32_t bytes = 0;
                         for (int m = 0; m < 3; ++m)

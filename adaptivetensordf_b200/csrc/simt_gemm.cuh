@@ -1,0 +1,105 @@
+// Register-tiled FP32 products of small matrices in shared memory, for the
+// decoder MLP on the CUDA cores (fused_simt.cuh, ops.cu).
+//
+// Every operand is stored with the contraction index contiguous, so a thread
+// loads four of its values per row with one 16-byte load and multiplies them
+// as two packed pairs (fma.rn.f32x2): a pair accumulates the even and the odd
+// terms, added at the end. Each lane is a plain FP32 fma.
+//
+// Lanes of a warp: lane / 4 picks the rows (A), lane % 4 the columns (B). On
+// sm_100a a warp's 16-byte shared load takes 2 cycles when neighbouring lanes
+// read the same address (A) and 4 otherwise (B; measured 2.06 and 3.9 cycles
+// an SM), so an 8 x 4 tile of outputs per thread costs 8 * 2 + 4 * 4 = 32
+// load cycles per 4 steps of the contraction against 32 cycles of its 128
+// FMAs per lane at 128 a cycle: both pipes are near balance, and a smaller
+// tile would be bound by the loads. Rows and columns of a thread are
+// interleaved (row i * groups + group), and the pitches are 4 mod 32 floats
+// (or 12, 20, 28) apart, so the distinct addresses of a load fall into
+// distinct banks.
+#pragma once
+
+#include <stdint.h>
+
+namespace atdf {
+
+__device__ __forceinline__ uint64_t ffma2(uint64_t a, uint64_t b, uint64_t c)
+{
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+
+__device__ __forceinline__ uint64_t pack2(float lo, float hi)
+{
+    uint64_t d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+    return d;
+}
+
+__device__ __forceinline__ void unpack2(uint64_t v, float& lo, float& hi)
+{
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+
+__device__ __forceinline__ float sum2(uint64_t v)
+{
+    float lo, hi;
+    unpack2(v, lo, hi);
+    return lo + hi;
+}
+
+// acc[i][j] += sum_k a[i * a_step + k] * b[j * b_step + k] over K (a multiple
+// of 4) contiguous k; a and b point at the thread's first row and column.
+template <int RM, int CN, int K>
+__device__ __forceinline__ void gemm_k(uint64_t (&acc)[RM][CN], const float* a, int a_step, const float* b,
+                                       int b_step)
+{
+#pragma unroll 2
+    for (int k = 0; k < K; k += 4) {
+        ulonglong2 av[RM], bv[CN];
+#pragma unroll
+        for (int i = 0; i < RM; ++i) av[i] = *reinterpret_cast<const ulonglong2*>(a + i * a_step + k);
+#pragma unroll
+        for (int j = 0; j < CN; ++j) bv[j] = *reinterpret_cast<const ulonglong2*>(b + j * b_step + k);
+#pragma unroll
+        for (int i = 0; i < RM; ++i)
+#pragma unroll
+            for (int j = 0; j < CN; ++j) {
+                acc[i][j] = ffma2(av[i].x, bv[j].x, acc[i][j]);
+                acc[i][j] = ffma2(av[i].y, bv[j].y, acc[i][j]);
+            }
+    }
+}
+
+// acc[i][j] += sum_s (a[s][2 i], a[s][2 i + 1]) * b[s][j]: a weight gradient
+// over S samples, both operands sample-major with 2 RP and CN contiguous
+// values per thread; the pairs run along a's columns.
+template <int RP, int CN>
+__device__ __forceinline__ void gemm_s(uint64_t (&acc)[RP][CN], const float* a, int a_pitch, const float* b,
+                                       int b_pitch, int S)
+{
+    static_assert(RP % 2 == 0 && CN == 4, "16-byte loads");
+#pragma unroll 4
+    for (int s = 0; s < S; ++s) {
+        ulonglong2 av[RP / 2];
+#pragma unroll
+        for (int i = 0; i < RP / 2; ++i) av[i] = *reinterpret_cast<const ulonglong2*>(a + s * a_pitch + 4 * i);
+        const float4 bv = *reinterpret_cast<const float4*>(b + s * b_pitch);
+        const uint64_t bb[4] = {pack2(bv.x, bv.x), pack2(bv.y, bv.y), pack2(bv.z, bv.z), pack2(bv.w, bv.w)};
+#pragma unroll
+        for (int i = 0; i < RP; ++i)
+#pragma unroll
+            for (int j = 0; j < CN; ++j) acc[i][j] = ffma2(i & 1 ? av[i / 2].y : av[i / 2].x, bb[j], acc[i][j]);
+    }
+}
+
+template <int RM, int CN>
+__device__ __forceinline__ void zero2(uint64_t (&acc)[RM][CN])
+{
+#pragma unroll
+    for (int i = 0; i < RM; ++i)
+#pragma unroll
+        for (int j = 0; j < CN; ++j) acc[i][j] = 0ull;
+}
+
+}  // namespace atdf

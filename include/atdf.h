@@ -547,7 +547,7 @@ int atdf_tone_response_loss(int32_t response_params, const float* response, floa
  * For callers that cannot call cudaMalloc (a plugin whose host framework owns
  * every device allocation, or a loop where an allocation would synchronise
  * the device): atdf_project_forward with its workspace taken from a static
- * device array of ATDF_NOALLOC_SCRATCH_BYTES (16 MiB) that every GPU loading
+ * device array of ATDF_NOALLOC_SCRATCH_BYTES (17 MiB) that every GPU loading
  * the library holds until exit. A problem whose workspace
  * (atdf_project_workspace_size) exceeds it is rejected with
  * ATDF_ERR_WORKSPACE before any launch; at depth 4 that is about 10,000
@@ -559,7 +559,7 @@ int atdf_tone_response_loss(int32_t response_params, const float* response, floa
  * atdf_project_forward. It is forward only: the segments it leaves in the
  * array are not a workspace that atdf_project_backward can take, so a caller
  * that needs gradients uses atdf_project_forward with its own workspace. */
-#define ATDF_NOALLOC_SCRATCH_BYTES (16u << 20)
+#define ATDF_NOALLOC_SCRATCH_BYTES (17u << 20)
 int atdf_project_forward_noalloc(const atdf_tree_t* tree, const atdf_field_t* field, const atdf_mlp_t* mlp,
                                  const float* ray_origin, const float* ray_direction, int64_t num_rays,
                                  int32_t max_samples_per_node, uint64_t jitter_seed, float* image,
