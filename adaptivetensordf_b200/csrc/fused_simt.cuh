@@ -226,44 +226,6 @@ __device__ __forceinline__ void load_weights(const FusedParams& p, float* sm)
     if (threadIdx.x == 0) sm[S::bl] = m.bias[NH][0];
 }
 
-// Logistic function from the approximate exponential and reciprocal (a few
-// ulp; without the denormal handling of __expf and __fdividef, which changes
-// nothing here: 1 + e^-x is never denormal, and e^-x is added to 1).
-__device__ __forceinline__ float sigmoid_ftz(float x)
-{
-    float e, r;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(x * -1.4426950408889634f));
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + e));
-    return r;
-}
-
-// Hidden activation and derivative. SiLU, the decoder's default, is inlined
-// (one exponential and one divide for both); the others go through a call.
-__device__ __noinline__ float2 act_pair_any(int a, float x, float beta)
-{
-    return make_float2(act_fwd(a, x, beta), act_grad(a, x, beta));
-}
-
-__device__ __forceinline__ void act_pair(int a, float x, float beta, float& h, float& g)
-{
-    if (a == ATDF_ACT_SILU) {
-        const float s = sigmoid_ftz(x);
-        h = x * s;
-        g = s * (1.0f + x * (1.0f - s));
-    } else {
-        const float2 v = act_pair_any(a, x, beta);
-        h = v.x;
-        g = v.y;
-    }
-}
-
-__device__ __noinline__ float act_any(int a, float x, float beta) { return act_fwd(a, x, beta); }
-
-__device__ __forceinline__ float act_hidden(int a, float x, float beta)
-{
-    return a == ATDF_ACT_SILU ? x * sigmoid_ftz(x) : act_any(a, x, beta);
-}
-
 // The thread's place in the [T][H] tile map: rows rg + i * RG, columns cg + j * CG.
 template <class K>
 __device__ __forceinline__ void tile_place(int& rg, int& cg, int& cw)

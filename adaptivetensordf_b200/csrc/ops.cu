@@ -9,6 +9,8 @@
 // hyperacorn/csrc/geometry/geometry_tensor_qo.cpp:257-380, Modules.h:23-149,
 // geometry.cpp:33-53,176-253,977-1019.
 
+#include <algorithm>
+
 #include "atdf_common.cuh"
 
 namespace atdf {
@@ -151,181 +153,251 @@ __global__ void gradcorr_bwd_kernel(const float* __restrict__ dir, const int64_t
 }
 
 // ---------------------------------------------------------------------------
-// VM feature field, FP32, channels-last (one thread per sample)
+// VM feature field, FP32, channels-last. A thread takes N pieces of V channels
+// of one sample (V = 4 with 16-byte accesses when the channel count and the
+// pointers allow it, else 1; N = 2 for channel counts that are multiples of 8,
+// which halves the threads that repeat a sample's geometry). Neighbouring
+// threads read and write neighbouring pieces: one thread per sample walking
+// its channels left every access of a warp in a cache line of its own.
 // ---------------------------------------------------------------------------
-__global__ void vm_fwd_kernel(atdf_field_t f, const float* __restrict__ pmin, const float* __restrict__ pmax,
-                              int64_t num_nodes, const float* __restrict__ pos, const int64_t* __restrict__ node,
-                              int64_t S, float* __restrict__ out, int32_t* err)
+template <int V>
+struct Vec {
+    float v[V];
+};
+
+template <int V>
+__device__ __forceinline__ Vec<V> load_vec(const float* p)
 {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= S) return;
-    const int C = f.channels;
-    const int F = f.mode ? 3 * C : C;
-    float* o = out + i * F;
+    Vec<V> r;
+    if constexpr (V == 4) {
+        const float4 t = __ldg(reinterpret_cast<const float4*>(p));
+        r.v[0] = t.x;
+        r.v[1] = t.y;
+        r.v[2] = t.z;
+        r.v[3] = t.w;
+    } else {
+        r.v[0] = __ldg(p);
+    }
+    return r;
+}
+
+template <int V>
+__device__ __forceinline__ void store_vec(float* p, const Vec<V>& r)
+{
+    if constexpr (V == 4)
+        *reinterpret_cast<float4*>(p) = make_float4(r.v[0], r.v[1], r.v[2], r.v[3]);
+    else
+        *p = r.v[0];
+}
+
+// p[0..V) += w * r in global memory.
+template <int V>
+__device__ __forceinline__ void add_vec(float* p, float w, const Vec<V>& r)
+{
+    if constexpr (V == 4)
+        asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(__cvta_generic_to_global(p)),
+                     "f"(__fmul_rn(w, r.v[0])), "f"(__fmul_rn(w, r.v[1])), "f"(__fmul_rn(w, r.v[2])),
+                     "f"(__fmul_rn(w, r.v[3]))
+                     : "memory");
+    else
+        atomicAdd(p, __fmul_rn(w, r.v[0]));
+}
+
+// Slot and coordinates of sample i; slot -1 (zero features) for a bad index
+// (which sets the error bit) and outside the ROI.
+__device__ __forceinline__ int64_t vm_sample(const atdf_field_t& f, const float* __restrict__ pmin,
+                                             const float* __restrict__ pmax, int64_t num_nodes,
+                                             const float* __restrict__ pos, const int64_t* __restrict__ node,
+                                             int64_t i, SampleGeo& g, int32_t* err)
+{
     const int64_t nd = node[i];
     if (nd < 0 || nd >= num_nodes) {
         set_err(err, ATDF_DEVERR_INDEX);
-        for (int c = 0; c < F; ++c) o[c] = 0.0f;
-        return;
+        return -1;
     }
     const int64_t slot = f.leaf_slot[nd];
     if (slot < 0 || slot >= f.num_slots) {
         if (slot >= f.num_slots) set_err(err, ATDF_DEVERR_INDEX);
-        for (int c = 0; c < F; ++c) o[c] = 0.0f;
-        return;
+        return -1;
     }
     const float p[3] = {pos[3 * i], pos[3 * i + 1], pos[3 * i + 2]};
-    const SampleGeo g = sample_geo(p, pmin + 3 * nd, pmax + 3 * nd, f.roi_min, f.roi_max);
-    for (int m = 0; m < 3; ++m) {
-        const int H = f.plane_h[m], W = f.plane_w[m], L = f.line_len[m];
-        const Corner2 k = corners2(g.pu[m], g.pv[m], H, W);
-        const Corner1 l = corners1(g.lu[m], L);
-        const float* P = (const float*)f.plane[m] + slot * (int64_t)H * W * C;
-        const float* V = (const float*)f.line[m];
-        for (int c = 0; c < C; ++c) {
-            const float mat = bilerp(k, P[(k.y0 * W + k.x0) * C + c], P[(k.y0 * W + k.x1) * C + c],
-                                     P[(k.y1 * W + k.x0) * C + c], P[(k.y1 * W + k.x1) * C + c]);
-            const float vec = lerp1(l, V[l.x0 * C + c], V[l.x1 * C + c]);
-            const float prod = __fmul_rn(mat, vec);
-            if (f.mode)
-                o[m * C + c] = prod;
-            else
-                o[c] = m == 0 ? prod : __fadd_rn(o[c], prod);
-        }
+    g = sample_geo(p, pmin + 3 * nd, pmax + 3 * nd, f.roi_min, f.roi_max);
+    return slot;
+}
+
+// Bilinear value of plane m (P: the slot's plane) and linear value of line m.
+template <int V>
+__device__ __forceinline__ void vm_values(const Corner2& k, const Corner1& l, const float* P, const float* L, int W,
+                                          int C, int c0, Vec<V>& mat, Vec<V>& vec)
+{
+    const Vec<V> nw = load_vec<V>(P + (k.y0 * W + k.x0) * C + c0), ne = load_vec<V>(P + (k.y0 * W + k.x1) * C + c0),
+                 sw = load_vec<V>(P + (k.y1 * W + k.x0) * C + c0), se = load_vec<V>(P + (k.y1 * W + k.x1) * C + c0),
+                 v0 = load_vec<V>(L + l.x0 * C + c0), v1 = load_vec<V>(L + l.x1 * C + c0);
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+        mat.v[i] = bilerp(k, nw.v[i], ne.v[i], sw.v[i], se.v[i]);
+        vec.v[i] = lerp1(l, v0.v[i], v1.v[i]);
     }
 }
 
-__global__ void vm_bwd_kernel(atdf_field_t f, const float* __restrict__ pmin, const float* __restrict__ pmax,
-                              int64_t num_nodes, const float* __restrict__ pos, const int64_t* __restrict__ node,
-                              int64_t S, const float* __restrict__ gout, atdf_field_grad_t gr, int32_t* err)
+template <int V, int N>
+__global__ void __launch_bounds__(256)
+    vm_fwd_kernel(atdf_field_t f, const float* __restrict__ pmin, const float* __restrict__ pmax, int64_t num_nodes,
+                  const float* __restrict__ pos, const int64_t* __restrict__ node, int64_t S, float* __restrict__ out,
+                  int32_t* err)
 {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int C = f.channels, Q = C / (V * N);
+    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t i = e / Q;
     if (i >= S) return;
-    const int C = f.channels;
-    const int F = f.mode ? 3 * C : C;
-    const int64_t nd = node[i];
-    if (nd < 0 || nd >= num_nodes) {
-        set_err(err, ATDF_DEVERR_INDEX);
-        return;
-    }
-    const int64_t slot = f.leaf_slot[nd];
-    if (slot < 0 || slot >= f.num_slots) return;
-    const float p[3] = {pos[3 * i], pos[3 * i + 1], pos[3 * i + 2]};
-    const SampleGeo g = sample_geo(p, pmin + 3 * nd, pmax + 3 * nd, f.roi_min, f.roi_max);
-    const float* go = gout + i * F;
-    for (int m = 0; m < 3; ++m) {
-        const int H = f.plane_h[m], W = f.plane_w[m], L = f.line_len[m];
-        const Corner2 k = corners2(g.pu[m], g.pv[m], H, W);
-        const Corner1 l = corners1(g.lu[m], L);
-        const int64_t pbase = slot * (int64_t)H * W * C;
-        const float* P = (const float*)f.plane[m] + pbase;
-        const float* V = (const float*)f.line[m];
-        float* GP = gr.plane[m] ? gr.plane[m] + pbase : nullptr;
-        float* GV = gr.line[m];
-        for (int c = 0; c < C; ++c) {
-            const float gf = f.mode ? go[m * C + c] : go[c];
-            const float mat = bilerp(k, P[(k.y0 * W + k.x0) * C + c], P[(k.y0 * W + k.x1) * C + c],
-                                     P[(k.y1 * W + k.x0) * C + c], P[(k.y1 * W + k.x1) * C + c]);
-            const float vec = lerp1(l, V[l.x0 * C + c], V[l.x1 * C + c]);
-            const float gm = __fmul_rn(gf, vec), gv = __fmul_rn(gf, mat);
-            if (GP) {
-                atomicAdd(&GP[(k.y0 * W + k.x0) * C + c], __fmul_rn(k.w_nw, gm));
-                atomicAdd(&GP[(k.y0 * W + k.x1) * C + c], __fmul_rn(k.w_ne, gm));
-                atomicAdd(&GP[(k.y1 * W + k.x0) * C + c], __fmul_rn(k.w_sw, gm));
-                atomicAdd(&GP[(k.y1 * W + k.x1) * C + c], __fmul_rn(k.w_se, gm));
-            }
-            if (GV) {
-                atomicAdd(&GV[l.x0 * C + c], __fmul_rn(l.w0, gv));
-                atomicAdd(&GV[l.x1 * C + c], __fmul_rn(l.w1, gv));
-            }
-        }
-    }
-}
-
-// ---------------------------------------------------------------------------
-// Decoder MLP, one thread per row (reference-compatible unfused path)
-// ---------------------------------------------------------------------------
-constexpr int kMlpMaxWidth = 256;
-
-__global__ void mlp_fwd_kernel(atdf_mlp_t m, const float* __restrict__ x, int64_t S, float* __restrict__ out)
-{
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= S) return;
-    float buf[2][kMlpMaxWidth];
-    const int in0 = m.dims[0];
-    for (int k = 0; k < in0; ++k) buf[0][k] = x[i * in0 + k];
-    int cur = 0;
-    for (int l = 0; l < m.num_layers; ++l) {
-        const int in = m.dims[l], on = m.dims[l + 1];
-        const bool last = l == m.num_layers - 1;
-        const float* Wl = m.weight[l];
-        for (int o = 0; o < on; ++o) {
-            float acc = 0.0f;
-            for (int k = 0; k < in; ++k) acc = fmaf(buf[cur][k], Wl[o * in + k], acc);
-            acc += m.bias[l][o];
-            buf[cur ^ 1][o] = act_fwd(last ? m.last_activation : m.hidden_activation, acc, m.softplus_beta);
-        }
-        cur ^= 1;
-    }
-    const int on = m.dims[m.num_layers];
-    for (int o = 0; o < on; ++o) out[i * on + o] = buf[cur][o];
-}
-
-constexpr int kMlpMaxPre = 1024;
-
-__global__ void mlp_bwd_kernel(atdf_mlp_t m, const float* __restrict__ x, int64_t S, const float* __restrict__ gout,
-                               float* __restrict__ gx, atdf_mlp_grad_t gr)
-{
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= S) return;
-    float pre[kMlpMaxPre];
-    float g[2][kMlpMaxWidth];
-    int po[ATDF_MAX_LAYERS + 1];
-    po[0] = 0;
-    for (int l = 0; l < m.num_layers; ++l) po[l + 1] = po[l] + m.dims[l + 1];
-    const int in0 = m.dims[0];
-    // forward keeping pre-activations
-    for (int l = 0; l < m.num_layers; ++l) {
-        const int in = m.dims[l], on = m.dims[l + 1];
-        const float* Wl = m.weight[l];
-        for (int o = 0; o < on; ++o) {
-            float acc = 0.0f;
-            for (int k = 0; k < in; ++k) {
-                const float xin = l == 0 ? x[i * in0 + k]
-                                         : act_fwd(m.hidden_activation, pre[po[l - 1] + k], m.softplus_beta);
-                acc = fmaf(xin, Wl[o * in + k], acc);
-            }
-            pre[po[l] + o] = acc + m.bias[l][o];
-        }
-    }
-    const int L = m.num_layers;
-    int cur = 0;
-    for (int o = 0; o < m.dims[L]; ++o) g[cur][o] = gout[i * m.dims[L] + o];
-    for (int l = L - 1; l >= 0; --l) {
-        const int in = m.dims[l], on = m.dims[l + 1];
-        const int a = l == L - 1 ? m.last_activation : m.hidden_activation;
-        for (int o = 0; o < on; ++o) g[cur][o] *= act_grad(a, pre[po[l] + o], m.softplus_beta);
-        const float* Wl = m.weight[l];
-        for (int o = 0; o < on; ++o) {
-            const float gp = g[cur][o];
-            if (gr.bias[l]) atomicAdd(&gr.bias[l][o], gp);
-            if (gr.weight[l] && gp != 0.0f) {
-                for (int k = 0; k < in; ++k) {
-                    const float xin = l == 0 ? x[i * in0 + k]
-                                             : act_fwd(m.hidden_activation, pre[po[l - 1] + k], m.softplus_beta);
-                    atomicAdd(&gr.weight[l][o * in + k], gp * xin);
+    const int c0 = (int)(e - i * Q) * V;  // channels c0 + n Q V .. + V - 1 of piece n
+    float* o = out + i * (f.mode ? 3 * C : C) + c0;
+    SampleGeo g;
+    const int64_t slot = vm_sample(f, pmin, pmax, num_nodes, pos, node, i, g, err);
+    Vec<V> acc[N];
+#pragma unroll
+    for (int n = 0; n < N; ++n)
+#pragma unroll
+        for (int j = 0; j < V; ++j) acc[n].v[j] = 0.0f;
+    if (slot >= 0) {
+#pragma unroll
+        for (int m = 0; m < 3; ++m) {
+            const int H = f.plane_h[m], W = f.plane_w[m];
+            const Corner2 k = corners2(g.pu[m], g.pv[m], H, W);
+            const Corner1 l = corners1(g.lu[m], f.line_len[m]);
+            const float* P = (const float*)f.plane[m] + slot * (int64_t)H * W * C;
+#pragma unroll
+            for (int n = 0; n < N; ++n) {
+                Vec<V> mat, vec;
+                vm_values<V>(k, l, P, (const float*)f.line[m], W, C, c0 + n * Q * V, mat, vec);
+#pragma unroll
+                for (int j = 0; j < V; ++j) {
+                    const float prod = __fmul_rn(mat.v[j], vec.v[j]);
+                    acc[n].v[j] = m == 0 || f.mode ? prod : __fadd_rn(acc[n].v[j], prod);
                 }
+                if (f.mode) store_vec<V>(o + m * C + n * Q * V, acc[n]);
             }
         }
-        for (int k = 0; k < in; ++k) {
-            float acc = 0.0f;
-            for (int o = 0; o < on; ++o) acc = fmaf(g[cur][o], Wl[o * in + k], acc);
-            g[cur ^ 1][k] = acc;
-        }
-        cur ^= 1;
+    } else if (f.mode) {
+        for (int m = 0; m < 3; ++m)
+            for (int n = 0; n < N; ++n) store_vec<V>(o + m * C + n * Q * V, acc[n]);
     }
-    if (gx)
-        for (int k = 0; k < in0; ++k) gx[i * in0 + k] = g[cur][k];
+    if (!f.mode)
+#pragma unroll
+        for (int n = 0; n < N; ++n) store_vec<V>(o + n * Q * V, acc[n]);
+}
+
+// The adjoint: plane gradients by (vector) reductions into global memory.
+// Line gradients collect every sample in a few hundred entries, so with
+// smem_lines each block sums its own copy in shared memory (the blocks stride
+// over the samples) and adds it once; more entries than fit go to global
+// memory directly. One piece of channels a thread: two put twice as many
+// samples in a warp, whose adds to the shared lines then collide more (98 us
+// against 169 us for 290 k samples of 8 channels; one thread a sample with
+// global line atomics took 1942 us).
+template <int V>
+__global__ void __launch_bounds__(256)
+    vm_bwd_kernel(atdf_field_t f, const float* __restrict__ pmin, const float* __restrict__ pmax, int64_t num_nodes,
+                  const float* __restrict__ pos, const int64_t* __restrict__ node, int64_t S,
+                  const float* __restrict__ gout, atdf_field_grad_t gr, bool smem_lines, int32_t* err)
+{
+    extern __shared__ __align__(16) float s_line[];
+    const int C = f.channels, Q = C / V;
+    const int off[4] = {0, f.line_len[0] * C, (f.line_len[0] + f.line_len[1]) * C,
+                        (f.line_len[0] + f.line_len[1] + f.line_len[2]) * C};
+    const int lane = threadIdx.x & 31;
+    const bool pow2_q = smem_lines && Q < 32 && (Q & (Q - 1)) == 0;
+    if (smem_lines) {
+        for (int i = threadIdx.x; i < off[3]; i += blockDim.x) s_line[i] = 0.0f;
+        __syncthreads();
+    }
+    // the loop bounds are the block's, so that all lanes of a warp reach the votes and shuffles
+    for (int64_t e0 = (int64_t)blockIdx.x * blockDim.x; e0 < S * Q; e0 += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t e = e0 + threadIdx.x, i = e / Q;
+        const int c0 = (int)(e - i * Q) * V;
+        SampleGeo g;
+        int64_t slot = -1;
+        if (e < S * Q) {
+            const int64_t nd = node[i];
+            if (nd < 0 || nd >= num_nodes)
+                set_err(err, ATDF_DEVERR_INDEX);
+            else
+                slot = vm_sample(f, pmin, pmax, num_nodes, pos, node, i, g, nullptr);
+        }
+        // The samples of a ray follow one another: where a whole warp falls
+        // between the same two entries of a line (the y line under a beam
+        // normal to y) its shared-memory adds would all collide.
+        bool same[3] = {false, false, false};
+        const bool whole = pow2_q && __all_sync(0xffffffffu, slot >= 0);
+        if (whole) {
+#pragma unroll
+            for (int m = 0; m < 3; ++m) {
+                const Corner1 l = corners1(g.lu[m], f.line_len[m]);
+                const int x0 = __shfl_sync(0xffffffffu, l.x0, 0), x1 = __shfl_sync(0xffffffffu, l.x1, 0);
+                same[m] = __all_sync(0xffffffffu, l.x0 == x0 && l.x1 == x1);
+            }
+        }
+        if (slot < 0) continue;
+        const float* go = gout + i * (f.mode ? 3 * C : C);
+#pragma unroll
+        for (int m = 0; m < 3; ++m) {
+            const int H = f.plane_h[m], W = f.plane_w[m];
+            const Corner2 k = corners2(g.pu[m], g.pv[m], H, W);
+            const Corner1 l = corners1(g.lu[m], f.line_len[m]);
+            const int64_t base = slot * (int64_t)H * W * C;
+            Vec<V> mat, vec;
+            vm_values<V>(k, l, (const float*)f.plane[m] + base, (const float*)f.line[m], W, C, c0, mat, vec);
+            const Vec<V> gf = load_vec<V>(go + (f.mode ? m * C : 0) + c0);
+            Vec<V> gm, gv;
+#pragma unroll
+            for (int j = 0; j < V; ++j) {
+                gm.v[j] = __fmul_rn(gf.v[j], vec.v[j]);
+                gv.v[j] = __fmul_rn(gf.v[j], mat.v[j]);
+            }
+            if (gr.plane[m]) {
+                float* GP = gr.plane[m] + base + c0;
+                add_vec<V>(GP + (k.y0 * W + k.x0) * C, k.w_nw, gm);
+                add_vec<V>(GP + (k.y0 * W + k.x1) * C, k.w_ne, gm);
+                add_vec<V>(GP + (k.y1 * W + k.x0) * C, k.w_sw, gm);
+                add_vec<V>(GP + (k.y1 * W + k.x1) * C, k.w_se, gm);
+            }
+            if (!gr.line[m]) continue;
+            if (smem_lines) {
+                float* dst = s_line + off[m] + c0;
+                if (same[m]) {  // one entry pair for the whole warp: its sums, added by one sample's lanes
+#pragma unroll
+                    for (int j = 0; j < V; ++j) {
+                        float a0 = __fmul_rn(l.w0, gv.v[j]), a1 = __fmul_rn(l.w1, gv.v[j]);
+                        for (int d = Q; d < 32; d <<= 1) {
+                            a0 += __shfl_xor_sync(0xffffffffu, a0, d);
+                            a1 += __shfl_xor_sync(0xffffffffu, a1, d);
+                        }
+                        if (lane < Q) {
+                            atomicAdd(&dst[l.x0 * C + j], a0);
+                            atomicAdd(&dst[l.x1 * C + j], a1);
+                        }
+                    }
+                } else {
+#pragma unroll
+                    for (int j = 0; j < V; ++j) {
+                        atomicAdd(&dst[l.x0 * C + j], __fmul_rn(l.w0, gv.v[j]));
+                        atomicAdd(&dst[l.x1 * C + j], __fmul_rn(l.w1, gv.v[j]));
+                    }
+                }
+            } else {
+                add_vec<V>(gr.line[m] + l.x0 * C + c0, l.w0, gv);
+                add_vec<V>(gr.line[m] + l.x1 * C + c0, l.w1, gv);
+            }
+        }
+    }
+    if (!smem_lines) return;
+    __syncthreads();
+    for (int m = 0; m < 3; ++m)
+        if (gr.line[m])
+            for (int i = threadIdx.x; i < f.line_len[m] * C; i += blockDim.x) {
+                const float v = s_line[off[m] + i];
+                if (v != 0.0f) atomicAdd(&gr.line[m][i], v);
+            }
 }
 
 // ---------------------------------------------------------------------------
@@ -468,6 +540,19 @@ static bool field_ok(const atdf_field_t* f)
     return true;
 }
 
+// Channels per thread: 8 or 4 by 16-byte accesses when the channel count is a
+// multiple and every pointer is aligned, else 1.
+static int vm_channels(const atdf_field_t* f, const float* features, const atdf_field_grad_t* g)
+{
+    uintptr_t bits = reinterpret_cast<uintptr_t>(features);
+    for (int m = 0; m < 3; ++m) {
+        bits |= reinterpret_cast<uintptr_t>(f->plane[m]) | reinterpret_cast<uintptr_t>(f->line[m]);
+        if (g) bits |= reinterpret_cast<uintptr_t>(g->plane[m]) | reinterpret_cast<uintptr_t>(g->line[m]);
+    }
+    if ((bits & 15) != 0 || f->channels % 4 != 0) return 1;
+    return f->channels % 8 == 0 ? 8 : 4;
+}
+
 int atdf_vm_features_forward(const atdf_field_t* field, const float* pmin, const float* pmax, int64_t num_nodes,
                              const float* position, const int64_t* node_id, int64_t S, float* out, int32_t* dev_error,
                              atdf_stream_t stream)
@@ -476,8 +561,10 @@ int atdf_vm_features_forward(const atdf_field_t* field, const float* pmin, const
         return ATDF_ERR_INVALID_ARGUMENT;
     if (field->dtype != ATDF_F32) return ATDF_ERR_UNSUPPORTED;
     if (S == 0) return ATDF_OK;
-    vm_fwd_kernel<<<blocks_for(S, 128), 128, 0, (cudaStream_t)stream>>>(*field, pmin, pmax, num_nodes, position,
-                                                                         node_id, S, out, dev_error);
+    const int per = vm_channels(field, out, nullptr);
+    const int64_t threads = S * (field->channels / per);
+    (per == 8 ? vm_fwd_kernel<4, 2> : per == 4 ? vm_fwd_kernel<4, 1> : vm_fwd_kernel<1, 1>)<<<blocks_for(threads), 256, 0, (cudaStream_t)stream>>>(
+        *field, pmin, pmax, num_nodes, position, node_id, S, out, dev_error);
     ATDF_LAUNCH_CHECK();
     return ATDF_OK;
 }
@@ -490,40 +577,25 @@ int atdf_vm_features_backward(const atdf_field_t* field, const float* pmin, cons
         return ATDF_ERR_INVALID_ARGUMENT;
     if (field->dtype != ATDF_F32) return ATDF_ERR_UNSUPPORTED;
     if (S == 0) return ATDF_OK;
-    vm_bwd_kernel<<<blocks_for(S, 128), 128, 0, (cudaStream_t)stream>>>(*field, pmin, pmax, num_nodes, position,
-                                                                         node_id, S, grad_features, *grad, dev_error);
-    ATDF_LAUNCH_CHECK();
-    return ATDF_OK;
-}
-
-static bool mlp_ok(const atdf_mlp_t* m)
-{
-    if (!m || m->num_layers <= 0 || m->num_layers > ATDF_MAX_LAYERS) return false;
-    int total = 0;
-    for (int l = 0; l <= m->num_layers; ++l) {
-        if (m->dims[l] <= 0 || m->dims[l] > kMlpMaxWidth) return false;
-        if (l > 0) total += m->dims[l];
+    const int chan = std::min(4, vm_channels(field, grad_features, grad));
+    const int64_t threads = S * (field->channels / chan);
+    // a copy of the lines per block while two blocks of 256 threads still fit an SM
+    const int64_t line_bytes =
+        ((int64_t)field->line_len[0] + field->line_len[1] + field->line_len[2]) * field->channels * 4;
+    const bool smem_lines = line_bytes <= 100 * 1024;
+    auto kernel = chan == 4 ? vm_bwd_kernel<4> : vm_bwd_kernel<1>;
+    const int smem = smem_lines ? (int)line_bytes : 0;
+    ATDF_CUDA_TRY(cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    unsigned blocks = blocks_for(threads);
+    if (smem_lines) {
+        int dev = 0, sms = 0, per = 0;
+        ATDF_CUDA_TRY(cudaGetDevice(&dev));
+        ATDF_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        ATDF_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, (const void*)kernel, 256, smem));
+        if (per > 0 && blocks > (unsigned)(sms * per)) blocks = (unsigned)(sms * per);
     }
-    for (int l = 0; l < m->num_layers; ++l)
-        if (!m->weight[l] || !m->bias[l]) return false;
-    return total <= kMlpMaxPre;
-}
-
-int atdf_mlp_forward(const atdf_mlp_t* mlp, const float* x, int64_t S, float* out, atdf_stream_t stream)
-{
-    if (!mlp_ok(mlp) || S < 0 || (S > 0 && (!x || !out))) return ATDF_ERR_INVALID_ARGUMENT;
-    if (S == 0) return ATDF_OK;
-    mlp_fwd_kernel<<<blocks_for(S, 128), 128, 0, (cudaStream_t)stream>>>(*mlp, x, S, out);
-    ATDF_LAUNCH_CHECK();
-    return ATDF_OK;
-}
-
-int atdf_mlp_backward(const atdf_mlp_t* mlp, const float* x, int64_t S, const float* grad_out, float* grad_x,
-                      const atdf_mlp_grad_t* grad, atdf_stream_t stream)
-{
-    if (!mlp_ok(mlp) || !grad || S < 0 || (S > 0 && (!x || !grad_out))) return ATDF_ERR_INVALID_ARGUMENT;
-    if (S == 0) return ATDF_OK;
-    mlp_bwd_kernel<<<blocks_for(S, 64), 64, 0, (cudaStream_t)stream>>>(*mlp, x, S, grad_out, grad_x, *grad);
+    kernel<<<blocks, 256, smem, (cudaStream_t)stream>>>(*field, pmin, pmax, num_nodes, position, node_id, S,
+                                                        grad_features, *grad, smem_lines, dev_error);
     ATDF_LAUNCH_CHECK();
     return ATDF_OK;
 }
