@@ -192,27 +192,41 @@ __global__ void ray_reduce_kernel(Ws w, int64_t R, float* image)
 }
 
 // ---------------------------------------------------------------------------
-// node-error scoring: one warp per segment, FP64 sums
+// node-error scoring: 16 lanes per segment, a lane per sample, FP64 sums. The
+// weights come from the neighbours' t, which the neighbouring lanes hold (a
+// warp per segment with three t per sample was bound by its instructions: 127
+// us for 319 k segments of 11 samples).
 // ---------------------------------------------------------------------------
-__global__ void node_error_kernel(Ws w, const float* __restrict__ prl, int cout, int64_t R, uint64_t seed,
-                                  double* ls, double* wsum, int64_t num_nodes, int32_t* err)
+__global__ void __launch_bounds__(256) node_error_kernel(Ws w, const float* __restrict__ prl, int cout, int64_t R,
+                                                         uint64_t seed, double* ls, double* wsum, int64_t num_nodes,
+                                                         int32_t* err)
 {
-    const int lane = threadIdx.x & 31;
+    constexpr int G = 16;
+    const int lane = threadIdx.x & (G - 1);
     const int64_t nseg = min(w.totals[0], w.cap);
-    for (int64_t sidx = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; sidx < nseg;
-         sidx += ((int64_t)gridDim.x * blockDim.x) >> 5) {
-        const int n = w.nsamp[sidx], node = w.node[sidx], r = w.ray[sidx];
-        const float tmin = w.tmin[sidx], tmax = w.tmax[sidx];
+    const int64_t groups = (int64_t)gridDim.x * blockDim.x / G;
+    // every lane of a warp makes the same number of rounds (full-warp shuffles)
+    for (int64_t s0 = 0; s0 < nseg; s0 += groups) {
+        const int64_t sidx = s0 + ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / G;
+        const bool have = sidx < nseg;
+        const int n = have ? w.nsamp[sidx] : 0, node = have ? w.node[sidx] : 0, r = have ? w.ray[sidx] : 0;
+        const float tmin = have ? w.tmin[sidx] : 0.0f, tmax = have ? w.tmax[sidx] : 0.0f;
+        const float step = n > 0 ? __fdiv_rn(__fsub_rn(tmax, tmin), (float)n) : 0.0f;
+        auto t_of = [&](int j) { return sample_t_step(tmin, step, j, sample_a(nullptr, 0, seed, r, node, j)); };
+        int most = n;  // rounds of the warp's longer segment
+        most = max(most, __shfl_xor_sync(0xffffffffu, most, G));
         double acc = 0.0;
-        for (int j = lane; j < n; j += 32) {
-            const float t = sample_t(tmin, tmax, n, j, sample_a(nullptr, 0, seed, r, node, j));
-            const float tp = j > 0 ? sample_t(tmin, tmax, n, j - 1, sample_a(nullptr, 0, seed, r, node, j - 1)) : 0.f;
-            const float tn = j < n - 1 ? sample_t(tmin, tmax, n, j + 1, sample_a(nullptr, 0, seed, r, node, j + 1))
-                                       : 0.f;
-            acc += (double)sample_w(tmin, tmax, n, j, tp, t, tn);
+        for (int j0 = 0; j0 < most; j0 += G) {
+            const int j = j0 + lane;
+            const float t = j < n ? t_of(j) : 0.0f;
+            float tp = __shfl_up_sync(0xffffffffu, t, 1, G), tn = __shfl_down_sync(0xffffffffu, t, 1, G);
+            if (lane == 0 && j > 0 && j < n) tp = t_of(j - 1);
+            if (lane == G - 1 && j < n - 1) tn = t_of(j + 1);
+            if (j < n) acc += (double)sample_w(tmin, tmax, n, j, tp, t, tn);
         }
-        for (int off = 16; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
-        if (lane == 0) {
+#pragma unroll
+        for (int off = G / 2; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
+        if (lane == 0 && have) {
             if (node < 0 || node >= num_nodes) {
                 set_err(err, ATDF_DEVERR_INDEX);
                 continue;

@@ -15,151 +15,7 @@
 
 namespace atdf {
 
-// ---------------------------------------------------------------------------
-// grid sample 2D / 1D (one thread per sample, channels in a loop)
-// ---------------------------------------------------------------------------
-__global__ void gs2_fwd_kernel(const float* __restrict__ grid, int64_t N, int64_t C, int H, int W, int64_t sN,
-                               int64_t sC, int64_t sH, int64_t sW, const int64_t* __restrict__ index,
-                               const float* __restrict__ uv, int64_t S, float* __restrict__ out, int32_t* err)
-{
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= S) return;
-    const int64_t n = index[i];
-    if (n < 0 || n >= N) {
-        set_err(err, ATDF_DEVERR_INDEX);
-        for (int64_t c = 0; c < C; ++c) out[i * C + c] = 0.0f;
-        return;
-    }
-    const Corner2 k = corners2(uv[2 * i], uv[2 * i + 1], H, W);
-    const float* g = grid + n * sN;
-    for (int64_t c = 0; c < C; ++c) {
-        const float* gc = g + c * sC;
-        out[i * C + c] = bilerp(k, gc[k.y0 * sH + k.x0 * sW], gc[k.y0 * sH + k.x1 * sW], gc[k.y1 * sH + k.x0 * sW],
-                                gc[k.y1 * sH + k.x1 * sW]);
-    }
-}
-
-__global__ void gs2_bwd_kernel(const float* __restrict__ grid, int64_t N, int64_t C, int H, int W, int64_t sN,
-                               int64_t sC, int64_t sH, int64_t sW, const int64_t* __restrict__ index,
-                               const float* __restrict__ uv, int64_t S, const float* __restrict__ gout,
-                               float* __restrict__ ggrid, float* __restrict__ guv, int32_t* err)
-{
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= S) return;
-    const int64_t n = index[i];
-    if (n < 0 || n >= N) {
-        set_err(err, ATDF_DEVERR_INDEX);
-        return;
-    }
-    const Corner2 k = corners2(uv[2 * i], uv[2 * i + 1], H, W);
-    const float* g = grid + n * sN;
-    float* gg = ggrid ? ggrid + n * C * H * W : nullptr;
-    float gix = 0.0f, giy = 0.0f;
-    const float ay1 = __fsub_rn(k.fy1, k.iy), ay0 = __fsub_rn(k.iy, k.fy0);
-    const float ax1 = __fsub_rn(k.fx1, k.ix), ax0 = __fsub_rn(k.ix, k.fx0);
-    for (int64_t c = 0; c < C; ++c) {
-        const float go = gout[i * C + c];
-        const float* gc = g + c * sC;
-        if (gg) {
-            float* ggc = gg + c * H * W;
-            atomicAdd(&ggc[k.y0 * W + k.x0], __fmul_rn(k.w_nw, go));
-            atomicAdd(&ggc[k.y0 * W + k.x1], __fmul_rn(k.w_ne, go));
-            atomicAdd(&ggc[k.y1 * W + k.x0], __fmul_rn(k.w_sw, go));
-            atomicAdd(&ggc[k.y1 * W + k.x1], __fmul_rn(k.w_se, go));
-        }
-        const float vnw = gc[k.y0 * sH + k.x0 * sW], vne = gc[k.y0 * sH + k.x1 * sW];
-        const float vsw = gc[k.y1 * sH + k.x0 * sW], vse = gc[k.y1 * sH + k.x1 * sW];
-        // IndirectGridSample2D.cu:354-367, one rounding per operation
-        gix = __fadd_rn(gix, __fmul_rn(__fmul_rn(__fmul_rn(-1.0f, vnw), ay1), go));
-        gix = __fadd_rn(gix, __fmul_rn(__fmul_rn(vne, ay1), go));
-        gix = __fadd_rn(gix, __fmul_rn(__fmul_rn(__fmul_rn(-1.0f, vsw), ay0), go));
-        gix = __fadd_rn(gix, __fmul_rn(__fmul_rn(vse, ay0), go));
-        giy = __fadd_rn(giy, __fmul_rn(__fmul_rn(__fmul_rn(-1.0f, vnw), ax1), go));
-        giy = __fadd_rn(giy, __fmul_rn(__fmul_rn(__fmul_rn(-1.0f, vne), ax0), go));
-        giy = __fadd_rn(giy, __fmul_rn(__fmul_rn(vsw, ax1), go));
-        giy = __fadd_rn(giy, __fmul_rn(__fmul_rn(vse, ax0), go));
-    }
-    if (guv) {
-        guv[2 * i] = __fadd_rn(guv[2 * i], __fdiv_rn(__fmul_rn(gix, (float)(W - 1)), 2.0f));
-        guv[2 * i + 1] = __fadd_rn(guv[2 * i + 1], __fdiv_rn(__fmul_rn(giy, (float)(H - 1)), 2.0f));
-    }
-}
-
-__global__ void gs1_fwd_kernel(const float* __restrict__ grid, int64_t N, int64_t C, int W, int64_t sN, int64_t sC,
-                               int64_t sW, const int64_t* __restrict__ index, const float* __restrict__ uv, int64_t S,
-                               float* __restrict__ out, int32_t* err)
-{
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= S) return;
-    const int64_t n = index[i];
-    if (n < 0 || n >= N) {
-        set_err(err, ATDF_DEVERR_INDEX);
-        for (int64_t c = 0; c < C; ++c) out[i * C + c] = 0.0f;
-        return;
-    }
-    const Corner1 k = corners1(uv[i], W);
-    const float* g = grid + n * sN;
-    for (int64_t c = 0; c < C; ++c) out[i * C + c] = lerp1(k, g[c * sC + k.x0 * sW], g[c * sC + k.x1 * sW]);
-}
-
-__global__ void gs1_bwd_kernel(const float* __restrict__ grid, int64_t N, int64_t C, int W, int64_t sN, int64_t sC,
-                               int64_t sW, const int64_t* __restrict__ index, const float* __restrict__ uv, int64_t S,
-                               const float* __restrict__ gout, float* __restrict__ ggrid, float* __restrict__ guv,
-                               int32_t* err)
-{
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= S) return;
-    const int64_t n = index[i];
-    if (n < 0 || n >= N) {
-        set_err(err, ATDF_DEVERR_INDEX);
-        return;
-    }
-    const Corner1 k = corners1(uv[i], W);
-    const float* g = grid + n * sN;
-    float* gg = ggrid ? ggrid + n * C * W : nullptr;
-    float gix = 0.0f;
-    const float a1 = __fsub_rn(k.fx1, k.ix), a0 = __fsub_rn(k.ix, k.fx0);
-    for (int64_t c = 0; c < C; ++c) {
-        const float go = gout[i * C + c];
-        if (gg) {
-            atomicAdd(&gg[c * W + k.x0], __fmul_rn(k.w0, go));
-            atomicAdd(&gg[c * W + k.x1], __fmul_rn(k.w1, go));
-        }
-        const float v0 = g[c * sC + k.x0 * sW], v1 = g[c * sC + k.x1 * sW];
-        gix = __fadd_rn(gix, __fmul_rn(__fmul_rn(__fmul_rn(-1.0f, v0), a1), go));
-        gix = __fadd_rn(gix, __fmul_rn(__fmul_rn(v1, a0), go));
-    }
-    if (guv) guv[i] = __fadd_rn(guv[i], __fdiv_rn(__fmul_rn(gix, (float)(W - 1)), 2.0f));
-}
-
-__global__ void gradcorr_bwd_kernel(const float* __restrict__ dir, const int64_t* __restrict__ ray, int64_t R,
-                                    const float* __restrict__ gin, int64_t S, float* __restrict__ gout, int32_t* err)
-{
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= S) return;
-    const int64_t r = ray[i];
-    if (r < 0 || r >= R) {
-        set_err(err, ATDF_DEVERR_INDEX);
-        return;
-    }
-    const float d0 = dir[3 * r], d1 = dir[3 * r + 1], d2 = dir[3 * r + 2];
-    const float g0 = gin[3 * i], g1 = gin[3 * i + 1], g2 = gin[3 * i + 2];
-    // grad - grad.dot(direction) * direction, one rounding per operation
-    // (the dot product summed left to right), so the result is reproducible
-    const float dot = __fadd_rn(__fadd_rn(__fmul_rn(g0, d0), __fmul_rn(g1, d1)), __fmul_rn(g2, d2));
-    gout[3 * i] = __fsub_rn(g0, __fmul_rn(dot, d0));
-    gout[3 * i + 1] = __fsub_rn(g1, __fmul_rn(dot, d1));
-    gout[3 * i + 2] = __fsub_rn(g2, __fmul_rn(dot, d2));
-}
-
-// ---------------------------------------------------------------------------
-// VM feature field, FP32, channels-last. A thread takes N pieces of V channels
-// of one sample (V = 4 with 16-byte accesses when the channel count and the
-// pointers allow it, else 1; N = 2 for channel counts that are multiples of 8,
-// which halves the threads that repeat a sample's geometry). Neighbouring
-// threads read and write neighbouring pieces: one thread per sample walking
-// its channels left every access of a warp in a cache line of its own.
-// ---------------------------------------------------------------------------
+// V floats by one access.
 template <int V>
 struct Vec {
     float v[V];
@@ -203,6 +59,244 @@ __device__ __forceinline__ void add_vec(float* p, float w, const Vec<V>& r)
         atomicAdd(p, __fmul_rn(w, r.v[0]));
 }
 
+// ---------------------------------------------------------------------------
+// grid sample 2D / 1D (one thread per sample, channels in a loop)
+// ---------------------------------------------------------------------------
+__global__ void gs2_fwd_kernel(const float* __restrict__ grid, int64_t N, int64_t C, int H, int W, int64_t sN,
+                               int64_t sC, int64_t sH, int64_t sW, const int64_t* __restrict__ index,
+                               const float* __restrict__ uv, int64_t S, float* __restrict__ out, int32_t* err)
+{
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= S) return;
+    const int64_t n = index[i];
+    if (n < 0 || n >= N) {
+        set_err(err, ATDF_DEVERR_INDEX);
+        for (int64_t c = 0; c < C; ++c) out[i * C + c] = 0.0f;
+        return;
+    }
+    const Corner2 k = corners2(uv[2 * i], uv[2 * i + 1], H, W);
+    const float* g = grid + n * sN;
+    for (int64_t c = 0; c < C; ++c) {
+        const float* gc = g + c * sC;
+        out[i * C + c] = bilerp(k, gc[k.y0 * sH + k.x0 * sW], gc[k.y0 * sH + k.x1 * sW], gc[k.y1 * sH + k.x0 * sW],
+                                gc[k.y1 * sH + k.x1 * sW]);
+    }
+}
+
+// One channel's terms of the coordinate gradient, one rounding per operation
+// (IndirectGridSample2D.cu:354-367).
+__device__ __forceinline__ void coord_grad2(float vnw, float vne, float vsw, float vse, float ax0, float ax1, float ay0,
+                                            float ay1, float go, float& gix, float& giy)
+{
+    gix = __fadd_rn(gix, __fmul_rn(__fmul_rn(__fmul_rn(-1.0f, vnw), ay1), go));
+    gix = __fadd_rn(gix, __fmul_rn(__fmul_rn(vne, ay1), go));
+    gix = __fadd_rn(gix, __fmul_rn(__fmul_rn(__fmul_rn(-1.0f, vsw), ay0), go));
+    gix = __fadd_rn(gix, __fmul_rn(__fmul_rn(vse, ay0), go));
+    giy = __fadd_rn(giy, __fmul_rn(__fmul_rn(__fmul_rn(-1.0f, vnw), ax1), go));
+    giy = __fadd_rn(giy, __fmul_rn(__fmul_rn(__fmul_rn(-1.0f, vne), ax0), go));
+    giy = __fadd_rn(giy, __fmul_rn(__fmul_rn(vsw, ax1), go));
+    giy = __fadd_rn(giy, __fmul_rn(__fmul_rn(vse, ax0), go));
+}
+
+__global__ void gs2_bwd_kernel(const float* __restrict__ grid, int64_t N, int64_t C, int H, int W, int64_t sN,
+                               int64_t sC, int64_t sH, int64_t sW, const int64_t* __restrict__ index,
+                               const float* __restrict__ uv, int64_t S, const float* __restrict__ gout,
+                               float* __restrict__ ggrid, float* __restrict__ guv, int32_t* err)
+{
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= S) return;
+    const int64_t n = index[i];
+    if (n < 0 || n >= N) {
+        set_err(err, ATDF_DEVERR_INDEX);
+        return;
+    }
+    const Corner2 k = corners2(uv[2 * i], uv[2 * i + 1], H, W);
+    const float* g = grid + n * sN;
+    float* gg = ggrid ? ggrid + n * C * H * W : nullptr;
+    float gix = 0.0f, giy = 0.0f;
+    const float ay1 = __fsub_rn(k.fy1, k.iy), ay0 = __fsub_rn(k.iy, k.fy0);
+    const float ax1 = __fsub_rn(k.fx1, k.ix), ax0 = __fsub_rn(k.ix, k.fx0);
+    for (int64_t c = 0; c < C; ++c) {
+        const float go = gout[i * C + c];
+        const float* gc = g + c * sC;
+        if (gg) {
+            float* ggc = gg + c * H * W;
+            atomicAdd(&ggc[k.y0 * W + k.x0], __fmul_rn(k.w_nw, go));
+            atomicAdd(&ggc[k.y0 * W + k.x1], __fmul_rn(k.w_ne, go));
+            atomicAdd(&ggc[k.y1 * W + k.x0], __fmul_rn(k.w_sw, go));
+            atomicAdd(&ggc[k.y1 * W + k.x1], __fmul_rn(k.w_se, go));
+        }
+        const float vnw = gc[k.y0 * sH + k.x0 * sW], vne = gc[k.y0 * sH + k.x1 * sW];
+        const float vsw = gc[k.y1 * sH + k.x0 * sW], vse = gc[k.y1 * sH + k.x1 * sW];
+        coord_grad2(vnw, vne, vsw, vse, ax0, ax1, ay0, ay1, go, gix, giy);
+    }
+    if (guv) {
+        guv[2 * i] = __fadd_rn(guv[2 * i], __fdiv_rn(__fmul_rn(gix, (float)(W - 1)), 2.0f));
+        guv[2 * i + 1] = __fadd_rn(guv[2 * i + 1], __fdiv_rn(__fmul_rn(giy, (float)(H - 1)), 2.0f));
+    }
+}
+
+// Channels-last grids [N][H][W][C] with C a multiple of 4 and 16-byte aligned
+// rows. Forward: a thread per sample and 4 channels.
+__global__ void __launch_bounds__(256)
+    gs2_fwd_cl_kernel(const float* __restrict__ grid, int64_t N, int C, int H, int W,
+                      const int64_t* __restrict__ index, const float* __restrict__ uv, int64_t S,
+                      float* __restrict__ out, int32_t* err)
+{
+    const int Q = C / 4;
+    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, i = e / Q;
+    if (i >= S) return;
+    const int c0 = (int)(e - i * Q) * 4;
+    const int64_t n = index[i];
+    Vec<4> r;
+    if (n < 0 || n >= N) {
+        set_err(err, ATDF_DEVERR_INDEX);
+        for (int j = 0; j < 4; ++j) r.v[j] = 0.0f;
+    } else {
+        const Corner2 k = corners2(uv[2 * i], uv[2 * i + 1], H, W);
+        const float* g = grid + n * (int64_t)H * W * C + c0;
+        const Vec<4> nw = load_vec<4>(g + (int64_t)(k.y0 * W + k.x0) * C), ne = load_vec<4>(g + (int64_t)(k.y0 * W + k.x1) * C),
+                     sw = load_vec<4>(g + (int64_t)(k.y1 * W + k.x0) * C), se = load_vec<4>(g + (int64_t)(k.y1 * W + k.x1) * C);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) r.v[j] = bilerp(k, nw.v[j], ne.v[j], sw.v[j], se.v[j]);
+    }
+    store_vec<4>(out + e * 4, r);
+}
+
+// Adjoint into a channels-last gradient by 16-byte reductions. A thread per
+// sample: the coordinate gradient is one chain of roundings over the channels
+// in order (IndirectGridSample2D.cu:354-367).
+__global__ void __launch_bounds__(256)
+    gs2_bwd_cl_kernel(const float* __restrict__ grid, int64_t N, int C, int H, int W,
+                      const int64_t* __restrict__ index, const float* __restrict__ uv, int64_t S,
+                      const float* __restrict__ gout, float* __restrict__ ggrid, float* __restrict__ guv, int32_t* err)
+{
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= S) return;
+    const int64_t n = index[i];
+    if (n < 0 || n >= N) {
+        set_err(err, ATDF_DEVERR_INDEX);
+        return;
+    }
+    const Corner2 k = corners2(uv[2 * i], uv[2 * i + 1], H, W);
+    const int64_t base = n * (int64_t)H * W * C;
+    const int64_t o[4] = {base + (int64_t)(k.y0 * W + k.x0) * C, base + (int64_t)(k.y0 * W + k.x1) * C,
+                          base + (int64_t)(k.y1 * W + k.x0) * C, base + (int64_t)(k.y1 * W + k.x1) * C};
+    float gix = 0.0f, giy = 0.0f;
+    const float ay1 = __fsub_rn(k.fy1, k.iy), ay0 = __fsub_rn(k.iy, k.fy0);
+    const float ax1 = __fsub_rn(k.fx1, k.ix), ax0 = __fsub_rn(k.ix, k.fx0);
+    for (int c = 0; c < C; c += 4) {
+        const Vec<4> go = load_vec<4>(gout + i * C + c);
+        add_vec<4>(ggrid + o[0] + c, k.w_nw, go);
+        add_vec<4>(ggrid + o[1] + c, k.w_ne, go);
+        add_vec<4>(ggrid + o[2] + c, k.w_sw, go);
+        add_vec<4>(ggrid + o[3] + c, k.w_se, go);
+        const Vec<4> nw = load_vec<4>(grid + o[0] + c), ne = load_vec<4>(grid + o[1] + c),
+                     sw = load_vec<4>(grid + o[2] + c), se = load_vec<4>(grid + o[3] + c);
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            coord_grad2(nw.v[j], ne.v[j], sw.v[j], se.v[j], ax0, ax1, ay0, ay1, go.v[j], gix, giy);
+    }
+    guv[2 * i] = __fadd_rn(guv[2 * i], __fdiv_rn(__fmul_rn(gix, (float)(W - 1)), 2.0f));
+    guv[2 * i + 1] = __fadd_rn(guv[2 * i + 1], __fdiv_rn(__fmul_rn(giy, (float)(H - 1)), 2.0f));
+}
+
+// V channels at a time: 16-byte stores when the channel count allows (V = 4).
+template <int V>
+__global__ void gs1_fwd_kernel(const float* __restrict__ grid, int64_t N, int64_t C, int W, int64_t sN, int64_t sC,
+                               int64_t sW, const int64_t* __restrict__ index, const float* __restrict__ uv, int64_t S,
+                               float* __restrict__ out, int32_t* err)
+{
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= S) return;
+    const int64_t n = index[i];
+    const bool ok = n >= 0 && n < N;
+    if (!ok) set_err(err, ATDF_DEVERR_INDEX);
+    const Corner1 k = corners1(uv[i], W);
+    const float* g = grid + (ok ? n * sN : 0);
+    for (int64_t c = 0; c < C; c += V) {
+        Vec<V> r;
+#pragma unroll
+        for (int j = 0; j < V; ++j)
+            r.v[j] = ok ? lerp1(k, g[(c + j) * sC + k.x0 * sW], g[(c + j) * sC + k.x1 * sW]) : 0.0f;
+        store_vec<V>(out + i * C + c, r);
+    }
+}
+
+// smem_sum: the grid's gradient fits in shared memory. Every sample adds to
+// one of few entries, so each block sums its own copy there and adds it once;
+// larger grids take global atomics.
+__global__ void __launch_bounds__(256)
+    gs1_bwd_kernel(const float* __restrict__ grid, int64_t N, int64_t C, int W, int64_t sN, int64_t sC, int64_t sW,
+                   const int64_t* __restrict__ index, const float* __restrict__ uv, int64_t S,
+                   const float* __restrict__ gout, float* __restrict__ ggrid, float* __restrict__ guv, bool smem_sum,
+                   int32_t* err)
+{
+    extern __shared__ float s_sum[];
+    const int64_t total = N * C * W;
+    if (smem_sum) {
+        for (int64_t j = threadIdx.x; j < total; j += blockDim.x) s_sum[j] = 0.0f;
+        __syncthreads();
+    }
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < S; i += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t n = index[i];
+        if (n < 0 || n >= N) {
+            set_err(err, ATDF_DEVERR_INDEX);
+            continue;
+        }
+        const Corner1 k = corners1(uv[i], W);
+        const float* g = grid + n * sN;
+        float* gg = smem_sum ? s_sum + n * C * W : ggrid ? ggrid + n * C * W : nullptr;
+        float gix = 0.0f;
+        const float a1 = __fsub_rn(k.fx1, k.ix), a0 = __fsub_rn(k.ix, k.fx0);
+        for (int64_t c = 0; c < C; ++c) {
+            const float go = gout[i * C + c];
+            if (gg) {
+                atomicAdd(&gg[c * W + k.x0], __fmul_rn(k.w0, go));
+                atomicAdd(&gg[c * W + k.x1], __fmul_rn(k.w1, go));
+            }
+            const float v0 = g[c * sC + k.x0 * sW], v1 = g[c * sC + k.x1 * sW];
+            gix = __fadd_rn(gix, __fmul_rn(__fmul_rn(__fmul_rn(-1.0f, v0), a1), go));
+            gix = __fadd_rn(gix, __fmul_rn(__fmul_rn(v1, a0), go));
+        }
+        if (guv) guv[i] = __fadd_rn(guv[i], __fdiv_rn(__fmul_rn(gix, (float)(W - 1)), 2.0f));
+    }
+    if (!smem_sum) return;
+    __syncthreads();
+    for (int64_t j = threadIdx.x; j < total; j += blockDim.x) {
+        const float v = s_sum[j];
+        if (v != 0.0f) atomicAdd(&ggrid[j], v);
+    }
+}
+
+__global__ void gradcorr_bwd_kernel(const float* __restrict__ dir, const int64_t* __restrict__ ray, int64_t R,
+                                    const float* __restrict__ gin, int64_t S, float* __restrict__ gout, int32_t* err)
+{
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= S) return;
+    const int64_t r = ray[i];
+    if (r < 0 || r >= R) {
+        set_err(err, ATDF_DEVERR_INDEX);
+        return;
+    }
+    const float d0 = dir[3 * r], d1 = dir[3 * r + 1], d2 = dir[3 * r + 2];
+    const float g0 = gin[3 * i], g1 = gin[3 * i + 1], g2 = gin[3 * i + 2];
+    // grad - grad.dot(direction) * direction, one rounding per operation
+    // (the dot product summed left to right), so the result is reproducible
+    const float dot = __fadd_rn(__fadd_rn(__fmul_rn(g0, d0), __fmul_rn(g1, d1)), __fmul_rn(g2, d2));
+    gout[3 * i] = __fsub_rn(g0, __fmul_rn(dot, d0));
+    gout[3 * i + 1] = __fsub_rn(g1, __fmul_rn(dot, d1));
+    gout[3 * i + 2] = __fsub_rn(g2, __fmul_rn(dot, d2));
+}
+
+// ---------------------------------------------------------------------------
+// VM feature field, FP32, channels-last. A thread takes N pieces of V channels
+// of one sample (V = 4 with 16-byte accesses when the channel count and the
+// pointers allow it, else 1; N = 2 for channel counts that are multiples of 8,
+// which halves the threads that repeat a sample's geometry). Neighbouring
+// threads read and write neighbouring pieces: one thread per sample walking
+// its channels left every access of a warp in a cache line of its own.
+// ---------------------------------------------------------------------------
 // Slot and coordinates of sample i; slot -1 (zero features) for a bad index
 // (which sets the error bit) and outside the ROI.
 __device__ __forceinline__ int64_t vm_sample(const atdf_field_t& f, const float* __restrict__ pmin,
@@ -466,6 +560,13 @@ static inline unsigned blocks_for(int64_t n, int t = 256) { return (unsigned)div
 
 extern "C" {
 
+// Strides of a dense channels-last grid that 16-byte accesses can take.
+static bool channels_last4(const float* grid, int64_t C, int64_t H, int64_t W, const int64_t* s)
+{
+    return C % 4 == 0 && (reinterpret_cast<uintptr_t>(grid) & 15) == 0 && s[1] == 1 && s[3] == C && s[2] == C * W &&
+           s[0] == C * W * H && C <= INT32_MAX / 4;
+}
+
 int atdf_grid_sample2d_forward(const float* grid, int64_t N, int64_t C, int64_t H, int64_t W,
                                const int64_t* s, const int64_t* index, const float* uv, int64_t S, float* out,
                                int32_t* dev_error, atdf_stream_t stream)
@@ -473,8 +574,12 @@ int atdf_grid_sample2d_forward(const float* grid, int64_t N, int64_t C, int64_t 
     if (!grid || !s || N <= 0 || C <= 0 || H <= 0 || W <= 0 || S < 0 || (S > 0 && (!index || !uv || !out)))
         return ATDF_ERR_INVALID_ARGUMENT;
     if (S == 0) return ATDF_OK;
-    gs2_fwd_kernel<<<blocks_for(S), 256, 0, (cudaStream_t)stream>>>(grid, N, C, (int)H, (int)W, s[0], s[1], s[2],
-                                                                    s[3], index, uv, S, out, dev_error);
+    if (channels_last4(grid, C, H, W, s) && (reinterpret_cast<uintptr_t>(out) & 15) == 0)
+        gs2_fwd_cl_kernel<<<blocks_for(S * (C / 4)), 256, 0, (cudaStream_t)stream>>>(grid, N, (int)C, (int)H, (int)W,
+                                                                                     index, uv, S, out, dev_error);
+    else
+        gs2_fwd_kernel<<<blocks_for(S), 256, 0, (cudaStream_t)stream>>>(grid, N, C, (int)H, (int)W, s[0], s[1], s[2],
+                                                                        s[3], index, uv, S, out, dev_error);
     ATDF_LAUNCH_CHECK();
     return ATDF_OK;
 }
@@ -493,6 +598,24 @@ int atdf_grid_sample2d_backward(const float* grid, int64_t N, int64_t C, int64_t
     return ATDF_OK;
 }
 
+int atdf_grid_sample2d_backward_channels_last(const float* grid, int64_t N, int64_t C, int64_t H, int64_t W,
+                                              const int64_t* index, const float* uv, int64_t S, const float* grad_out,
+                                              float* grad_grid, float* grad_uv, int32_t* dev_error,
+                                              atdf_stream_t stream)
+{
+    if (!grid || !grad_grid || !grad_uv || N <= 0 || C <= 0 || H <= 0 || W <= 0 || S < 0 ||
+        (S > 0 && (!index || !uv || !grad_out)))
+        return ATDF_ERR_INVALID_ARGUMENT;
+    if (C % 4 != 0 || ((reinterpret_cast<uintptr_t>(grid) | reinterpret_cast<uintptr_t>(grad_grid) |
+                        reinterpret_cast<uintptr_t>(grad_out)) & 15) != 0)
+        return ATDF_ERR_UNSUPPORTED;
+    if (S == 0) return ATDF_OK;
+    gs2_bwd_cl_kernel<<<blocks_for(S), 256, 0, (cudaStream_t)stream>>>(grid, N, (int)C, (int)H, (int)W, index, uv, S,
+                                                                       grad_out, grad_grid, grad_uv, dev_error);
+    ATDF_LAUNCH_CHECK();
+    return ATDF_OK;
+}
+
 int atdf_grid_sample1d_forward(const float* grid, int64_t N, int64_t C, int64_t W, const int64_t* s,
                                const int64_t* index, const float* uv, int64_t S, float* out, int32_t* dev_error,
                                atdf_stream_t stream)
@@ -500,8 +623,9 @@ int atdf_grid_sample1d_forward(const float* grid, int64_t N, int64_t C, int64_t 
     if (!grid || !s || N <= 0 || C <= 0 || W <= 0 || S < 0 || (S > 0 && (!index || !uv || !out)))
         return ATDF_ERR_INVALID_ARGUMENT;
     if (S == 0) return ATDF_OK;
-    gs1_fwd_kernel<<<blocks_for(S), 256, 0, (cudaStream_t)stream>>>(grid, N, C, (int)W, s[0], s[1], s[2], index, uv,
-                                                                    S, out, dev_error);
+    const bool vec = C % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
+    (vec ? gs1_fwd_kernel<4> : gs1_fwd_kernel<1>)<<<blocks_for(S), 256, 0, (cudaStream_t)stream>>>(
+        grid, N, C, (int)W, s[0], s[1], s[2], index, uv, S, out, dev_error);
     ATDF_LAUNCH_CHECK();
     return ATDF_OK;
 }
@@ -513,8 +637,21 @@ int atdf_grid_sample1d_backward(const float* grid, int64_t N, int64_t C, int64_t
     if (!grid || !s || N <= 0 || C <= 0 || W <= 0 || S < 0 || (S > 0 && (!index || !uv || !grad_out)))
         return ATDF_ERR_INVALID_ARGUMENT;
     if (S == 0) return ATDF_OK;
-    gs1_bwd_kernel<<<blocks_for(S), 256, 0, (cudaStream_t)stream>>>(grid, N, C, (int)W, s[0], s[1], s[2], index, uv,
-                                                                    S, grad_out, grad_grid, grad_uv, dev_error);
+    // a block's copy of the gradient: up to 64 KB, so that three blocks share an
+    // SM, and fewer entries than samples to sum
+    const bool smem_sum = grad_grid && N * C * W * 4 <= 64 * 1024 && N * W <= S;
+    unsigned blocks = blocks_for(S);
+    if (smem_sum) {
+        int dev = 0, sms = 0, per = 0;
+        const int smem = (int)(N * C * W * 4);
+        ATDF_CUDA_TRY(cudaFuncSetAttribute((const void*)gs1_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        ATDF_CUDA_TRY(cudaGetDevice(&dev));
+        ATDF_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        ATDF_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, (const void*)gs1_bwd_kernel, 256, smem));
+        if (per > 0 && blocks > (unsigned)(sms * per)) blocks = (unsigned)(sms * per);
+    }
+    gs1_bwd_kernel<<<blocks, 256, smem_sum ? (size_t)(N * C * W * 4) : 0, (cudaStream_t)stream>>>(
+        grid, N, C, (int)W, s[0], s[1], s[2], index, uv, S, grad_out, grad_grid, grad_uv, smem_sum, dev_error);
     ATDF_LAUNCH_CHECK();
     return ATDF_OK;
 }

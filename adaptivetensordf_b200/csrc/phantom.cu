@@ -45,39 +45,51 @@ __global__ void siddon_kernel(SiddonGrid g, const float* __restrict__ origin, co
         out[r] = 0.0;
         return;
     }
-    // voxel containing the point just inside the entry face
+    // voxel containing the point just inside the entry face, and per axis the
+    // parameter of the next voxel face crossed there. A face's parameter is
+    // recomputed from the voxel index, so rounding does not accumulate, but
+    // only on the axis that moved, and with the direction's reciprocal: the
+    // walk is bound by its FP64 chain (one face a step; with three FP64
+    // divides a step it took 0.76 ms for 262144 rays through 256^3 voxels).
     int idx[3], step[3];
+    double tf[3], inv[3];
     const double tin = t0 + 1e-9 * (t1 - t0);
+#pragma unroll
     for (int a = 0; a < 3; ++a) {
         const double u = (o[a] + d[a] * tin - g.bmin[a]) / g.h[a];
         int i = (int)floor(u);
         idx[a] = i < 0 ? 0 : (i >= g.n[a] ? g.n[a] - 1 : i);
         step[a] = d[a] > 0 ? 1 : -1;
+        inv[a] = d[a] != 0.0 ? 1.0 / d[a] : 0.0;
+        tf[a] = d[a] != 0.0 ? (g.bmin[a] + (double)(idx[a] + (step[a] > 0 ? 1 : 0)) * g.h[a] - o[a]) * inv[a] : INFINITY;
     }
     double acc = 0.0, t = t0;
     const int max_steps = g.n[0] + g.n[1] + g.n[2] + 3;
     for (int it = 0; it < max_steps && t < t1; ++it) {
-        // parameter of the next voxel face crossed on each axis, recomputed
-        // from the voxel index so that rounding does not accumulate
+        // the nearest face before the exit (ties: the lower axis)
         double tn = t1;
         int axis = -1;
-        for (int a = 0; a < 3; ++a) {
-            if (d[a] == 0.0) continue;
-            const double face = g.bmin[a] + (double)(idx[a] + (step[a] > 0 ? 1 : 0)) * g.h[a];
-            const double ta = (face - o[a]) / d[a];
-            if (ta < tn) {
-                tn = ta;
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+            if (tf[a] < tn) {
+                tn = tf[a];
                 axis = a;
             }
-        }
         if (tn > t) {
             const int64_t v = ((int64_t)idx[2] * g.n[1] + idx[1]) * g.n[0] + idx[0];
-            acc += (tn - t) * (double)g.vol[v];
+            acc += (tn - t) * (double)__ldg(&g.vol[v]);
             t = tn;
         }
         if (axis < 0) break;
-        idx[axis] += step[axis];
-        if (idx[axis] < 0 || idx[axis] >= g.n[axis]) break;
+        bool left = false;
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+            if (axis == a) {
+                idx[a] += step[a];
+                left = idx[a] < 0 || idx[a] >= g.n[a];
+                tf[a] = (g.bmin[a] + (double)(idx[a] + (step[a] > 0 ? 1 : 0)) * g.h[a] - o[a]) * inv[a];
+            }
+        if (left) break;
     }
     out[r] = acc;
 }

@@ -43,6 +43,35 @@ int activation_id(const std::string& a)
 // IndirectGridSample2D / 1D (IndirectGridSample2D.cu:408-492,
 // IndirectGridSample1D.cu:153-220)
 // ---------------------------------------------------------------------------
+// The 2D operator's channels-last kernels read and add a texel's channels with
+// 16-byte accesses. Grids of another layout are copied for them when there are
+// enough samples to pay for it: a copy moves every texel once each way, a
+// sample gathers four texels whose channels lie in separate sectors otherwise
+// (1 M samples on 1.2 M texels of 16 channels: forward 252 -> 75 us, adjoint
+// 771 -> 175 us with the copies; below one sample per 4 texels the copy costs
+// more than it saves).
+static bool samples_in_channels_last(const Tensor& grid, int64_t samples)
+{
+    const int64_t texels = grid.size(0) * grid.size(2) * grid.size(3);
+    return grid.size(1) % 4 == 0 && grid.numel() > 0 &&
+           (grid.is_contiguous(torch::MemoryFormat::ChannelsLast) || 4 * samples >= texels);
+}
+
+static Tensor aligned16(const Tensor& t)
+{
+    return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0 ? t : t.clone();
+}
+
+// Dense NHWC storage, 16-byte aligned.
+static Tensor channels_last_copy(const Tensor& grid)
+{
+    const int64_t C = grid.size(1), H = grid.size(2), W = grid.size(3);
+    const bool dense = grid.stride(1) == 1 && grid.stride(3) == C && grid.stride(2) == C * W &&
+                       grid.stride(0) == C * W * H;
+    if (dense) return aligned16(grid);
+    return grid.permute({0, 2, 3, 1}).contiguous().permute({0, 3, 1, 2});
+}
+
 class GridSample2DFn : public torch::autograd::Function<GridSample2DFn> {
    public:
     static Tensor forward(AutogradContext* ctx, Tensor grid, Tensor index, Tensor uv)
@@ -56,10 +85,12 @@ class GridSample2DFn : public torch::autograd::Function<GridSample2DFn> {
         auto idx = index.to(torch::kLong).contiguous();
         auto u = uv.contiguous();
         const int64_t S = idx.size(0), C = grid.size(1);
-        auto out = torch::zeros({S, C}, grid.options().memory_format(torch::MemoryFormat::Contiguous));
-        int64_t st[4] = {grid.stride(0), grid.stride(1), grid.stride(2), grid.stride(3)};
+        auto out = torch::empty({S, C}, grid.options().memory_format(torch::MemoryFormat::Contiguous));
+        auto grid_read = grid;
+        if (samples_in_channels_last(grid, S)) grid_read = channels_last_copy(grid);
+        int64_t st[4] = {grid_read.stride(0), grid_read.stride(1), grid_read.stride(2), grid_read.stride(3)};
         auto err = err_word(grid.device());
-        check_status(atdf_grid_sample2d_forward(grid.data_ptr<float>(), grid.size(0), C, grid.size(2), grid.size(3), st,
+        check_status(atdf_grid_sample2d_forward(grid_read.data_ptr<float>(), grid.size(0), C, grid.size(2), grid.size(3), st,
                                                 idx.data_ptr<int64_t>(), u.data_ptr<float>(), S, out.data_ptr<float>(),
                                                 err.data_ptr<int32_t>(), stream_arg()),
                      "IndirectGridSample2D");
@@ -75,10 +106,22 @@ class GridSample2DFn : public torch::autograd::Function<GridSample2DFn> {
         auto s = ctx->get_saved_variables();
         auto grid = s[0], idx = s[1], u = s[2];
         auto g = go[0].contiguous();
-        auto ggrid = torch::zeros(grid.sizes(), grid.options().memory_format(torch::MemoryFormat::Contiguous));
         auto guv = torch::zeros_like(u);
-        int64_t st[4] = {grid.stride(0), grid.stride(1), grid.stride(2), grid.stride(3)};
         auto err = ctx->saved_data["err"].toTensor();
+        if (samples_in_channels_last(grid, idx.size(0)) && idx.size(0) > 0) {
+            auto grid_read = channels_last_copy(grid);
+            auto ggrid = torch::zeros_like(grid_read);
+            g = aligned16(g);
+            check_status(atdf_grid_sample2d_backward_channels_last(
+                             grid_read.data_ptr<float>(), grid.size(0), grid.size(1), grid.size(2), grid.size(3),
+                             idx.data_ptr<int64_t>(), u.data_ptr<float>(), idx.size(0), g.data_ptr<float>(),
+                             ggrid.data_ptr<float>(), guv.data_ptr<float>(), err.data_ptr<int32_t>(), stream_arg()),
+                         "IndirectGridSample2D backward");
+            check_dev_error(err, "IndirectGridSample2D backward");
+            return {ggrid.contiguous(), Tensor(), guv};
+        }
+        auto ggrid = torch::zeros(grid.sizes(), grid.options().memory_format(torch::MemoryFormat::Contiguous));
+        int64_t st[4] = {grid.stride(0), grid.stride(1), grid.stride(2), grid.stride(3)};
         check_status(atdf_grid_sample2d_backward(grid.data_ptr<float>(), grid.size(0), grid.size(1), grid.size(2),
                                                  grid.size(3), st, idx.data_ptr<int64_t>(), u.data_ptr<float>(),
                                                  idx.size(0), g.data_ptr<float>(), ggrid.data_ptr<float>(),
@@ -102,7 +145,7 @@ class GridSample1DFn : public torch::autograd::Function<GridSample1DFn> {
         auto idx = index.to(torch::kLong).contiguous();
         auto u = uv.contiguous();
         const int64_t S = idx.size(0), C = grid.size(1);
-        auto out = torch::zeros({S, C}, grid.options().memory_format(torch::MemoryFormat::Contiguous));
+        auto out = torch::empty({S, C}, grid.options().memory_format(torch::MemoryFormat::Contiguous));
         int64_t st[3] = {grid.stride(0), grid.stride(1), grid.stride(2)};
         auto err = err_word(grid.device());
         check_status(atdf_grid_sample1d_forward(grid.data_ptr<float>(), grid.size(0), C, grid.size(2), st,

@@ -204,6 +204,13 @@ int atdf_grid_sample2d_backward(const float* grid, int64_t N, int64_t C, int64_t
                                 const int64_t* grid_stride, const int64_t* index, const float* uv,
                                 int64_t num_samples, const float* grad_out, float* grad_grid, float* grad_uv,
                                 int32_t* dev_error, atdf_stream_t stream);
+/* The adjoint for a channels-last grid ([N][H][W][C], C a multiple of 4, all
+ * three arrays 16-byte aligned, else ATDF_ERR_UNSUPPORTED): accumulates into a
+ * grad_grid of the same layout and into grad_uv. */
+int atdf_grid_sample2d_backward_channels_last(const float* grid, int64_t N, int64_t C, int64_t H, int64_t W,
+                                              const int64_t* index, const float* uv, int64_t num_samples,
+                                              const float* grad_out, float* grad_grid, float* grad_uv,
+                                              int32_t* dev_error, atdf_stream_t stream);
 int atdf_grid_sample1d_forward(const float* grid, int64_t N, int64_t C, int64_t W, const int64_t* grid_stride,
                                const int64_t* index, const float* uv, int64_t num_samples, float* out,
                                int32_t* dev_error, atdf_stream_t stream);

@@ -103,3 +103,71 @@ def test_field_long_lines(oracle):
     gr = oracle.project_backward(fd, md, td, so, R, np.ones((1, R)), np.float32)
     for m in range(3):
         assert rel_err(geo.lines[m].grad.cpu().numpy(), gr["lines"][m]) < REL_TOL, f"line {m}"
+
+
+@pytest.mark.parametrize("shape,S", [((5, 8, 17, 17), 1), ((5, 8, 17, 17), 300), ((5, 8, 17, 17), 361),
+                                     ((5, 8, 17, 17), 4000), ((3, 4, 6, 9), 777), ((2, 7, 5, 8), 500),
+                                     ((9, 24, 3, 2), 65)])
+@pytest.mark.parametrize("layout", ["contiguous", "channels_last", "sliced"])
+def test_grid_sample_layouts(oracle, shape, S, layout):
+    """The 2D operator's channels-last kernels and the strided ones (channel
+    counts of 4 or not, samples around one per 4 texels, other strides): the
+    forward and the coordinate gradient bit for bit."""
+    import adaptivetensordf_b200 as ab
+
+    rng = np.random.default_rng(S)
+    g = rng.normal(size=shape).astype(np.float32)
+    idx = rng.integers(0, shape[0], S)
+    uv = rng.uniform(-1.2, 1.2, (S, 2)).astype(np.float32)
+    go = rng.normal(size=(S, shape[1])).astype(np.float32)
+    gt = torch.from_numpy(g).cuda()
+    if layout == "channels_last":
+        gt = gt.contiguous(memory_format=torch.channels_last)
+    elif layout == "sliced":
+        gt = torch.cat([gt, gt], 3)[..., :shape[3]]
+    gt = gt.requires_grad_(True)
+    ut = torch.from_numpy(uv).cuda().requires_grad_(True)
+    out = ab.IndirectGridSample2D(gt, torch.from_numpy(idx).cuda(), ut)
+    assert np.array_equal(out.detach().cpu().numpy(), oracle.grid_sample2d(g, idx, uv, np.float32))
+    gg, gu = torch.autograd.grad(out, [gt, ut], torch.from_numpy(go).cuda())
+    assert gg.shape == gt.shape and gg.is_contiguous()
+    assert rel_err(gg.cpu().numpy(), oracle.grid_sample2d_bwd(g, idx, uv, go, np.float64)[0]) < REL_TOL
+    assert np.array_equal(gu.cpu().numpy(), oracle.grid_sample2d_bwd(g, idx, uv, go, np.float32)[1])
+
+
+@pytest.mark.parametrize("shape,S", [((1, 16, 256, 1), 5000), ((2, 7, 33, 1), 65), ((2, 7, 33, 1), 66),
+                                     ((40, 8, 64, 1), 3000), ((3, 4, 1, 1), 100)])
+def test_grid_sample_lines(oracle, shape, S):
+    """The 1D operator's gradient summed in shared memory (few entries) and in
+    global memory (more than 64 KB, or more entries than samples)."""
+    import adaptivetensordf_b200 as ab
+
+    rng = np.random.default_rng(S)
+    g = rng.normal(size=shape).astype(np.float32)
+    idx = rng.integers(0, shape[0], S)
+    u = rng.uniform(-1.1, 1.1, (S, 1)).astype(np.float32)
+    go = rng.normal(size=(S, shape[1])).astype(np.float32)
+    gt, ut = torch.from_numpy(g).cuda().requires_grad_(True), torch.from_numpy(u).cuda().requires_grad_(True)
+    out = ab.IndirectGridSample1D(gt, torch.from_numpy(idx).cuda(), ut)
+    assert np.array_equal(out.detach().cpu().numpy(), oracle.grid_sample1d(g, idx, u, np.float32))
+    out.backward(torch.from_numpy(go).cuda())
+    assert rel_err(gt.grad.cpu().numpy(), oracle.grid_sample1d_bwd(g, idx, u, go, np.float64)[0]) < REL_TOL
+    assert np.array_equal(ut.grad.cpu().numpy(), oracle.grid_sample1d_bwd(g, idx, u, go, np.float32)[1])
+
+
+@pytest.mark.parametrize("M,seed", [(1, 0), (27, 0), (28, 9), (56, 9), (90, 3)])
+def test_node_error_segment_lengths(oracle, M, seed):
+    """Segments of up to 1, 16, 17, 33 and more samples (16 lanes a segment)."""
+    import adaptivetensordf_b200 as ab
+
+    R = 333
+    tree, geo, o, d = gpu_scene(2, 8, 9, (32, 9, 32), [32], R, seed=M)
+    td, _, _ = oracle_views(tree, geo)
+    y = np.random.default_rng(0).uniform(0, 2, (1, R)).astype(np.float32)
+    rays = ab.RayList(torch.from_numpy(o).cuda(), torch.from_numpy(d).cuda())
+    img, ls, ws = geo.ProjectNodeError(tree, rays, M, seed, torch.from_numpy(y).cuda())
+    segs = oracle.ray_segments(td, o, d, M)
+    so = oracle.emit_samples(segs, o, d, oracle.jitter_for_segments(seed, segs) if seed else None)
+    ls_o, ws_o = oracle.accumulate_loss_per_node(so, (img.cpu().numpy() - y) ** 2, len(td["node_depth"]))
+    assert rel_err(ws.cpu().numpy(), ws_o) < 1e-12
+    assert rel_err(ls.cpu().numpy(), ls_o) < 1e-9
