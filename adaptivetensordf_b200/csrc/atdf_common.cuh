@@ -311,9 +311,92 @@ __device__ __forceinline__ uint32_t float_key(float f)
     return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
 
+// Exclusive scan of n values with one 1024-thread block: each thread owns a
+// contiguous chunk, loads it 8 values at a time (the loads of a group are in
+// flight together; chunks of up to 16 stay in registers for the write-back),
+// then a warp-shuffle scan of the chunk sums and one of the 32 warp totals.
+template <typename T>
+__device__ __forceinline__ void block_scan_exclusive(T* data, int64_t n, T* total, T* warp_sums)
+{
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int64_t per = div_up(n, 1024);
+    const int64_t b = min(n, (int64_t)tid * per), e = min(n, b + per);
+    constexpr int KEEP = 17;  // 16384 rays + 1 offsets per 1024 threads
+    T keep[KEEP];
+    T s = 0;
+    if (per <= KEEP) {
+#pragma unroll
+        for (int k = 0; k < KEEP; ++k) keep[k] = b + k < e ? data[b + k] : T(0);
+#pragma unroll
+        for (int k = 0; k < KEEP; ++k) s += keep[k];
+    } else {
+        for (int64_t i = b; i < e; i += 8) {
+            T v[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) v[k] = i + k < e ? data[i + k] : T(0);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) s += v[k];
+        }
+    }
+    T incl = s;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const T x = __shfl_up_sync(0xffffffffu, incl, off);
+        if (lane >= off) incl += x;
+    }
+    if (lane == 31) warp_sums[warp] = incl;
+    __syncthreads();
+    if (warp == 0) {
+        const T ws = warp_sums[lane];
+        T wi = ws;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const T x = __shfl_up_sync(0xffffffffu, wi, off);
+            if (lane >= off) wi += x;
+        }
+        warp_sums[lane] = wi - ws;  // exclusive warp offsets
+        if (lane == 31 && total) *total = wi;
+    }
+    __syncthreads();
+    T run = warp_sums[warp] + incl - s;
+    if (per <= KEEP) {
+#pragma unroll
+        for (int k = 0; k < KEEP; ++k)
+            if (b + k < e) {
+                data[b + k] = run;
+                run += keep[k];
+            }
+    } else {
+        for (int64_t i = b; i < e; i += 8) {
+            T v[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) v[k] = i + k < e ? data[i + k] : T(0);
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+                if (i + k < e) {
+                    data[i + k] = run;
+                    run += v[k];
+                }
+        }
+    }
+    __syncthreads();  // warp_sums is reused by a second scan in the same block
+}
+
 // Single-block exclusive scan of n int64 values in place; writes the total to
 // *total (if non-null). Launched with 1024 threads.
 __global__ void scan_exclusive_i64_kernel(int64_t* data, int64_t n, int64_t* total);
-__global__ void scan_exclusive_i32_kernel(int32_t* data, int64_t n, int32_t* total);
+
+// Scratch of the ray/leaf segment pass in the fused path's workspace (all
+// nullable): every ray's sorted hits (kept_per entries each) and the segment
+// and sample sums of each block's rays.
+struct SegScratch {
+    uint32_t* kept_lo;
+    uint32_t* kept_hi;
+    int64_t kept_per;
+    longlong2* block_sums;
+};
+
+int launch_ray_segments(const atdf_tree_t& tree, const float* origin, const float* dir, int64_t R, int M,
+                        const atdf_segments_t& segs, int32_t* err, cudaStream_t st, const SegScratch* scratch);
 
 }  // namespace atdf

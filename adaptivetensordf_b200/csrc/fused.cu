@@ -25,109 +25,105 @@
 
 namespace atdf {
 
-int launch_ray_segments(const atdf_tree_t& tree, const float* origin, const float* dir, int64_t R, int M,
-                        const atdf_segments_t& segs, int32_t* err, cudaStream_t st, uint32_t* kept_lo = nullptr,
-                        uint32_t* kept_hi = nullptr, int64_t kept_per = 0);
-
-// The workspace's bucket and segment-partial arrays (R * per entries, idle
-// until the segments exist) hold the segment pass's kept hits.
+// The segment pass's scratch: the kept hits in the workspace's bucket and
+// segment-partial arrays (R * per entries, idle until the segments exist), the
+// block sums (2 R bytes) in the item queue's (at least 6 R).
 static int launch_ray_segments_ws(const atdf_tree_t& tree, const float* origin, const float* dir, int64_t R, int M,
                                   const Ws& w, int32_t* err, cudaStream_t st)
 {
-    const int64_t per = R > 0 ? w.cap / R : 0;
-    return launch_ray_segments(tree, origin, dir, R, M, ws_segments(w), err, st, reinterpret_cast<uint32_t*>(w.bucket),
-                               reinterpret_cast<uint32_t*>(w.seg_partial), per);
+    SegScratch sc;
+    sc.kept_lo = reinterpret_cast<uint32_t*>(w.bucket);
+    sc.kept_hi = reinterpret_cast<uint32_t*>(w.seg_partial);
+    sc.kept_per = R > 0 ? w.cap / R : 0;
+    sc.block_sums = reinterpret_cast<longlong2*>(w.item_queue);
+    return launch_ray_segments(tree, origin, dir, R, M, ws_segments(w), err, st, &sc);
 }
 
 // ---------------------------------------------------------------------------
 // bucketing by plane slot
 // ---------------------------------------------------------------------------
-// A segment whose node id or plane slot is out of range sets the index bit
-// and joins the out-of-ROI bucket (zero features, no gradient).
+// Counts the segments of each slot; a segment keeps its rank there (in the
+// segment partials, idle until the forward). A segment whose node id or plane
+// slot is out of range sets the index bit and joins the out-of-ROI bucket
+// (zero features, no gradient).
 __global__ void bucket_count_kernel(Ws w, atdf_field_t f, int64_t num_nodes, int32_t* err)
 {
     const int64_t nseg = min(w.totals[0], w.cap);
+    int32_t* rank = reinterpret_cast<int32_t*>(w.seg_partial);
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nseg; i += (int64_t)gridDim.x * blockDim.x) {
         const int32_t nd = w.node[i];
         if (nd < 0 || nd >= num_nodes || f.leaf_slot[nd] >= f.num_slots) set_err(err, ATDF_DEVERR_INDEX);
-        atomicAdd(&w.slot_offset[seg_slot(f, num_nodes, nd)], 1);
+        rank[i] = atomicAdd(&w.slot_offset[seg_slot(f, num_nodes, nd)], 1);
     }
 }
 
 __global__ void bucket_scatter_kernel(Ws w, atdf_field_t f, int64_t num_nodes)
 {
     const int64_t nseg = min(w.totals[0], w.cap);
+    const int32_t* rank = reinterpret_cast<const int32_t*>(w.seg_partial);
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nseg; i += (int64_t)gridDim.x * blockDim.x) {
         const int64_t s = seg_slot(f, num_nodes, w.node[i]);
-        const int pos = w.slot_offset[s] + atomicAdd(&w.slot_cursor[s], 1);
-        w.bucket[pos] = (int32_t)i;
+        w.bucket[w.slot_offset[s] + rank[i]] = (int32_t)i;
     }
 }
 
-// Order of the slot queue: slots by descending segment count, so that the
-// largest slots start first and the kernels' tail holds the smallest ones
-// (longest-processing-time-first scheduling of the slot-sticky work). A
-// counting sort on min(segments / 2, 255) in one block; it writes into
-// slot_cursor, whose bucketing role has ended.
-__global__ void slot_order_kernel(Ws w)
-{
-    __shared__ int hist[256];
-    const int n = (int)w.nslot + 1;
-    for (int i = threadIdx.x; i < 256; i += blockDim.x) hist[i] = 0;
-    __syncthreads();
-    for (int s = threadIdx.x; s < n; s += blockDim.x)
-        atomicAdd(&hist[255 - min((w.slot_offset[s + 1] - w.slot_offset[s]) >> 1, 255)], 1);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int run = 0;
-        for (int i = 0; i < 256; ++i) {
-            const int c = hist[i];
-            hist[i] = run;
-            run += c;
-        }
-    }
-    __syncthreads();
-    for (int s = threadIdx.x; s < n; s += blockDim.x) {
-        const int pos = atomicAdd(&hist[255 - min((w.slot_offset[s + 1] - w.slot_offset[s]) >> 1, 255)], 1);
-        w.slot_cursor[pos] = s;
-    }
-}
-
-// Items per slot: equal shares of at most kSegItem segments. items > 0 (the
-// kernels that take items one by one): also small enough that the call makes
-// about that many items, but not below kMinItem segments each.
-__global__ void item_count_kernel(Ws w, int items)
-{
-    int per = kSegItem;
-    if (items > 0) per = (int)max((int64_t)kMinItem, min((int64_t)kSegItem, min(w.totals[0], w.cap) / items));
-    for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s <= w.nslot + 1;
-         s += (int64_t)gridDim.x * blockDim.x) {
-        if (s == w.nslot + 1) {
-            w.item_offset[s] = 0;
-        } else {
-            const int cnt = w.slot_offset[s + 1] - w.slot_offset[s];
-            w.item_offset[s] = (cnt + per - 1) / per;
-        }
-    }
-}
-
-// The item queue of the forwards: for each slot in the slot queue's order
-// (slot_cursor) its items (slot, 0 .. n - 1), at the exclusive prefix of the
-// item counts in that order; counters[4] = the number of items. One block.
-__global__ void item_queue_kernel(Ws w)
+// From the slots' segment counts, in one block and launch (each step is a few
+// microseconds of latency on a few thousand slots; as five kernels they took
+// 40 us a call):
+//  * slot offsets (exclusive scan) and items per slot: equal shares of at most
+//    kSegItem segments. items > 0 (the FP32 kernels): also small enough that
+//    the call makes about that many items, but not below kMinItem segments;
+//  * the slot queue's order (slot_order): slots by descending segment count,
+//    so that the largest start first and the kernels' tail holds the smallest
+//    (longest-processing-time-first), a counting sort on min(count / 2, 255);
+//  * the item queue: each slot's items in the slot queue's order;
+//    counters[4] = the number of items.
+__global__ void __launch_bounds__(1024) plan_kernel(Ws w, int items)
 {
     __shared__ int warp_sum[32];
+    __shared__ int hist[256];
     __shared__ int s_base;
-    const int n = (int)w.nslot + 1;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    if (threadIdx.x == 0) s_base = 0;
+    const int n = (int)w.nslot + 1;  // plane slots and the out-of-ROI bucket
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    int per = kSegItem;
+    if (items > 0) per = (int)max((int64_t)kMinItem, min((int64_t)kSegItem, min(w.totals[0], w.cap) / items));
+    for (int i = tid; i < 256; i += 1024) hist[i] = 0;
+    if (tid == 0) s_base = 0;
     __syncthreads();
-    for (int c0 = 0; c0 < n; c0 += blockDim.x) {
-        const int q = c0 + threadIdx.x;
+    for (int s = tid; s < n; s += 1024) {
+        const int cnt = w.slot_offset[s];
+        w.item_offset[s] = (cnt + per - 1) / per;
+        atomicAdd(&hist[255 - min(cnt >> 1, 255)], 1);
+    }
+    if (tid == 0) w.slot_offset[n] = w.item_offset[n] = 0;
+    __syncthreads();
+    if (wid == 0) {  // exclusive scan of the 256 bins, 8 a lane
+        int v[8], sum = 0;
+        for (int k = 0; k < 8; ++k) {
+            v[k] = hist[8 * lane + k];
+            sum += v[k];
+        }
+        int incl = sum;
+        for (int off = 1; off < 32; off <<= 1) {
+            const int x = __shfl_up_sync(0xffffffffu, incl, off);
+            if (lane >= off) incl += x;
+        }
+        int run = incl - sum;
+        for (int k = 0; k < 8; ++k) {
+            hist[8 * lane + k] = run;
+            run += v[k];
+        }
+    }
+    __syncthreads();
+    for (int s = tid; s < n; s += 1024) w.slot_order[atomicAdd(&hist[255 - min(w.slot_offset[s] >> 1, 255)], 1)] = s;
+    __syncthreads();
+    // the items in the order of the queue, before the scan of their counts
+    for (int c0 = 0; c0 < n; c0 += 1024) {
+        const int q = c0 + tid;
         int sl = -1, ni = 0;
         if (q < n) {
-            sl = w.slot_cursor[q];
-            ni = w.item_offset[sl + 1] - w.item_offset[sl];
+            sl = w.slot_order[q];
+            ni = w.item_offset[sl];
         }
         int incl = ni;
         for (int off = 1; off < 32; off <<= 1) {
@@ -137,21 +133,23 @@ __global__ void item_queue_kernel(Ws w)
         if (lane == 31) warp_sum[wid] = incl;
         __syncthreads();
         if (wid == 0) {
-            int v = lane < nw ? warp_sum[lane] : 0;
+            int v = warp_sum[lane];
             for (int off = 1; off < 32; off <<= 1) {
                 const int x = __shfl_up_sync(0xffffffffu, v, off);
                 if (lane >= off) v += x;
             }
-            if (lane < nw) warp_sum[lane] = v;  // inclusive over warps
+            warp_sum[lane] = v;  // inclusive over warps
         }
         __syncthreads();
         const int pos = s_base + (wid > 0 ? warp_sum[wid - 1] : 0) + incl - ni;
         for (int i = 0; i < ni; ++i) w.item_queue[pos + i] = make_int2(sl, i);
         __syncthreads();
-        if (threadIdx.x == 0) s_base += warp_sum[nw - 1];
+        if (tid == 0) s_base += warp_sum[31];
         __syncthreads();
     }
-    if (threadIdx.x == 0) w.counters[4] = s_base;
+    if (tid == 0) w.counters[4] = s_base;
+    block_scan_exclusive<int32_t>(w.slot_offset, n + 1, nullptr, warp_sum);
+    block_scan_exclusive<int32_t>(w.item_offset, n + 1, nullptr, warp_sum);
 }
 
 // Zeroes the plane gradients of the slots that no segment touches; the
@@ -404,22 +402,13 @@ static int project_forward(const atdf_tree_t* tree, const atdf_field_t* field, c
         if (st != ATDF_OK) return st;
     }
     if (bins) ATDF_CUDA_TRY(cudaMemsetAsync(bins, 0, (size_t)w.cap * kBins * sizeof(float), s));
-    ATDF_CUDA_TRY(cudaMemsetAsync(w.slot_offset, 0, (w.nslot + 2) * 4, s));
-    ATDF_CUDA_TRY(cudaMemsetAsync(w.slot_cursor, 0, (w.nslot + 1) * 4, s));
-    ATDF_CUDA_TRY(cudaMemsetAsync(w.counters, 0, 8 * 4, s));
+    // counters and slot counts lie side by side
+    ATDF_CUDA_TRY(cudaMemsetAsync(w.counters, 0, 256 + (w.nslot + 2) * 4, s));
     bucket_count_kernel<<<592, 256, 0, s>>>(w, *field, tree->num_nodes, dev_error);
     ATDF_LAUNCH_CHECK();
-    scan_exclusive_i32_kernel<<<1, 1024, 0, s>>>(w.slot_offset, w.nslot + 2, nullptr);
+    plan_kernel<<<1, 1024, 0, s>>>(w, var ? kSimtItems : 0);
     ATDF_LAUNCH_CHECK();
     bucket_scatter_kernel<<<592, 256, 0, s>>>(w, *field, tree->num_nodes);
-    ATDF_LAUNCH_CHECK();
-    item_count_kernel<<<(unsigned)div_up(w.nslot + 2, 256), 256, 0, s>>>(w, var ? kSimtItems : 0);
-    ATDF_LAUNCH_CHECK();
-    slot_order_kernel<<<1, 1024, 0, s>>>(w);
-    ATDF_LAUNCH_CHECK();
-    scan_exclusive_i32_kernel<<<1, 1024, 0, s>>>(w.item_offset, w.nslot + 2, nullptr);
-    ATDF_LAUNCH_CHECK();
-    item_queue_kernel<<<1, 1024, 0, s>>>(w);
     ATDF_LAUNCH_CHECK();
     st = var ? launch_persistent(var->fwd, var->smem(false), p, s) : launch_tc_forward(p, s);
     if (st != ATDF_OK) return st;

@@ -31,10 +31,10 @@ struct Ws {
     int32_t* first;
     float* seg_partial;
     int32_t* bucket;
-    int32_t* slot_offset;  // [nslot + 2]
-    int32_t* slot_cursor;  // [nslot + 1]: bucket cursors, then the queue's slot order
-    int32_t* item_offset;  // [nslot + 2]
     int32_t* counters;     // [8]: the queues' positions (0, 1), the item queue's length (4)
+    int32_t* slot_offset;  // [nslot + 2], 256 bytes after the counters
+    int32_t* slot_order;   // [nslot + 1]: the slot queue
+    int32_t* item_offset;  // [nslot + 2]
     int2* item_queue;      // (slot, item of the slot) in the slot queue's order
     int64_t cap;
     int64_t nslot;
@@ -71,10 +71,10 @@ static size_t ws_layout(int64_t R, int max_depth, int64_t nslot, char* base, Ws*
     x.first = (int32_t*)carve(p, cap * 4);
     x.seg_partial = (float*)carve(p, cap * 4);
     x.bucket = (int32_t*)carve(p, cap * 4);
-    x.slot_offset = (int32_t*)carve(p, (nslot + 2) * 4);
-    x.slot_cursor = (int32_t*)carve(p, (nslot + 1) * 4);
-    x.item_offset = (int32_t*)carve(p, (nslot + 2) * 4);
     x.counters = (int32_t*)carve(p, 8 * 4);
+    x.slot_offset = (int32_t*)carve(p, (nslot + 2) * 4);
+    x.slot_order = (int32_t*)carve(p, (nslot + 1) * 4);
+    x.item_offset = (int32_t*)carve(p, (nslot + 2) * 4);
     x.item_queue = (int2*)carve(p, (nslot + 3 + cap / kMinItem) * 8);
     x.cap = cap;
     x.nslot = nslot;
@@ -333,7 +333,7 @@ __device__ __forceinline__ ItemInfo next_item(const FusedParams& p, int queue, f
                 while (true) {
                     const int q = atomicAdd(&w.counters[queue], 1);
                     if (q >= nslots) break;
-                    const int sl = w.slot_cursor[q];  // largest slots first (slot_order_kernel)
+                    const int sl = w.slot_order[q];  // largest slots first (plan_kernel)
                     const int i0 = w.item_offset[sl], i1 = w.item_offset[sl + 1];
                     if (i1 > i0) {
                         s_ctl[4] = sl;

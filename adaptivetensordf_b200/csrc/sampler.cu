@@ -17,77 +17,6 @@
 
 namespace atdf {
 
-// Exclusive scan of n values with one 1024-thread block: each thread owns a
-// contiguous chunk, loads it 8 values at a time (the loads of a group are in
-// flight together; chunks of up to 16 stay in registers for the write-back),
-// then a warp-shuffle scan of the chunk sums and one of the 32 warp totals.
-template <typename T>
-__device__ __forceinline__ void block_scan_exclusive(T* data, int64_t n, T* total, T* warp_sums)
-{
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int64_t per = div_up(n, 1024);
-    const int64_t b = min(n, (int64_t)tid * per), e = min(n, b + per);
-    constexpr int KEEP = 17;  // 16384 rays + 1 offsets per 1024 threads
-    T keep[KEEP];
-    T s = 0;
-    if (per <= KEEP) {
-#pragma unroll
-        for (int k = 0; k < KEEP; ++k) keep[k] = b + k < e ? data[b + k] : T(0);
-#pragma unroll
-        for (int k = 0; k < KEEP; ++k) s += keep[k];
-    } else {
-        for (int64_t i = b; i < e; i += 8) {
-            T v[8];
-#pragma unroll
-            for (int k = 0; k < 8; ++k) v[k] = i + k < e ? data[i + k] : T(0);
-#pragma unroll
-            for (int k = 0; k < 8; ++k) s += v[k];
-        }
-    }
-    T incl = s;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-        const T x = __shfl_up_sync(0xffffffffu, incl, off);
-        if (lane >= off) incl += x;
-    }
-    if (lane == 31) warp_sums[warp] = incl;
-    __syncthreads();
-    if (warp == 0) {
-        const T ws = warp_sums[lane];
-        T wi = ws;
-#pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            const T x = __shfl_up_sync(0xffffffffu, wi, off);
-            if (lane >= off) wi += x;
-        }
-        warp_sums[lane] = wi - ws;  // exclusive warp offsets
-        if (lane == 31 && total) *total = wi;
-    }
-    __syncthreads();
-    T run = warp_sums[warp] + incl - s;
-    if (per <= KEEP) {
-#pragma unroll
-        for (int k = 0; k < KEEP; ++k)
-            if (b + k < e) {
-                data[b + k] = run;
-                run += keep[k];
-            }
-    } else {
-        for (int64_t i = b; i < e; i += 8) {
-            T v[8];
-#pragma unroll
-            for (int k = 0; k < 8; ++k) v[k] = i + k < e ? data[i + k] : T(0);
-#pragma unroll
-            for (int k = 0; k < 8; ++k)
-                if (i + k < e) {
-                    data[i + k] = run;
-                    run += v[k];
-                }
-        }
-    }
-    __syncthreads();  // warp_sums is reused by a second scan in the same block
-}
-
 __global__ void scan_exclusive_i64_kernel(int64_t* data, int64_t n, int64_t* total)
 {
     __shared__ int64_t ws[32];
@@ -99,12 +28,6 @@ __global__ void scan2_exclusive_i64_kernel(int64_t* a, int64_t* b, int64_t n)
 {
     __shared__ int64_t ws[32];
     block_scan_exclusive<int64_t>(blockIdx.x == 0 ? a : b, n, nullptr, ws);
-}
-
-__global__ void scan_exclusive_i32_kernel(int32_t* data, int64_t n, int32_t* total)
-{
-    __shared__ int32_t ws[32];
-    block_scan_exclusive<int32_t>(data, n, total, ws);
 }
 
 // bit 0: active leaf; bit 1: some descendant is an active leaf. Bits only
@@ -157,13 +80,16 @@ enum SegMode {
 template <int MODE>
 __global__ void __launch_bounds__(kSegWarps * 32)
     ray_segments_kernel(atdf_tree_t tree, const float* __restrict__ origin, const float* __restrict__ dir, int64_t R,
-                        int M, atdf_segments_t segs, int32_t* err, uint32_t* kept_lo, uint32_t* kept_hi,
-                        int64_t kept_per)
+                        int M, atdf_segments_t segs, int32_t* err, SegScratch sc)
 {
     constexpr bool WRITE = MODE == kSegWrite || MODE == kSegWriteKept;
     constexpr bool TRAVERSE = MODE != kSegWriteKept;
     __shared__ uint64_t keys[kSegWarps][ATDF_MAX_HITS];
     __shared__ int32_t front[kSegWarps][2][ATDF_MAX_HITS];
+    __shared__ int64_t s_sum[2][kSegWarps];  // per warp: segments and samples (of its ray, or before its block)
+    uint32_t* const kept_lo = sc.kept_lo;
+    uint32_t* const kept_hi = sc.kept_hi;
+    const int64_t kept_per = sc.kept_per;
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     const int64_t r = (int64_t)blockIdx.x * kSegWarps + warp;
@@ -171,13 +97,15 @@ __global__ void __launch_bounds__(kSegWarps * 32)
         segs.ray_seg_offset[R] = 0;
         segs.ray_sample_offset[R] = 0;
     }
-    if (r >= R) return;
+    const bool active = r < R;  // warps past the last ray stay for the block's sums
 
-    float o[3], d[3];
+    float o[3] = {0.0f, 0.0f, 0.0f}, d[3] = {0.0f, 0.0f, 0.0f};
+    if (active) {
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        o[k] = origin[3 * r + k];
-        d[k] = dir[3 * r + k];
+        for (int k = 0; k < 3; ++k) {
+            o[k] = origin[3 * r + k];
+            d[k] = dir[3 * r + k];
+        }
     }
     const float* pmin = tree.node_position_min;
     const float* pmax = tree.node_position_max;
@@ -188,8 +116,63 @@ __global__ void __launch_bounds__(kSegWarps * 32)
     int64_t nsamp = 0;
     bool overflow = false;
 
+    int64_t seg0 = 0;
+    if constexpr (MODE == kSegWriteKept) {
+        if (sc.block_sums) {
+            // offsets of the block's rays: the sums of the blocks before it,
+            // then its own rays' counts (which the counting pass left in the
+            // offset arrays). Every block adds up its predecessors itself, so
+            // no scan kernel and no wait sits between the two passes.
+            int64_t a = 0, b = 0;
+            for (int j = threadIdx.x; j < (int)blockIdx.x; j += kSegWarps * 32) {
+                const longlong2 v = sc.block_sums[j];
+                a += v.x;
+                b += v.y;
+            }
+            for (int off = 16; off > 0; off >>= 1) {
+                a += __shfl_xor_sync(0xffffffffu, a, off);
+                b += __shfl_xor_sync(0xffffffffu, b, off);
+            }
+            if (lane == 0) {
+                s_sum[0][warp] = a;
+                s_sum[1][warp] = b;
+            }
+            // the counts of the block's rays, before any of them is overwritten
+            int64_t n = 0, m = 0;
+            const int64_t rr = (int64_t)blockIdx.x * kSegWarps + lane;
+            if (lane < kSegWarps && rr < R) {
+                n = segs.ray_seg_offset[rr];
+                m = segs.ray_sample_offset[rr];
+            }
+            __syncthreads();
+            int64_t before_n = 0, before_m = 0;
+            for (int k = 0; k < kSegWarps; ++k) {
+                before_n += s_sum[0][k];
+                before_m += s_sum[1][k];
+            }
+            for (int k = 0; k < warp; ++k) {
+                before_n += __shfl_sync(0xffffffffu, n, k);
+                before_m += __shfl_sync(0xffffffffu, m, k);
+            }
+            nhit = (int)__shfl_sync(0xffffffffu, n, warp);
+            const int64_t ray_samples = __shfl_sync(0xffffffffu, m, warp);
+            seg0 = before_n;
+            if (active && lane == 0) {
+                segs.ray_seg_offset[r] = before_n;
+                segs.ray_sample_offset[r] = before_m;
+                if (r == R - 1) {
+                    segs.ray_seg_offset[R] = segs.totals[0] = before_n + nhit;
+                    segs.ray_sample_offset[R] = segs.totals[1] = before_m + ray_samples;
+                }
+            }
+        } else if (active) {
+            seg0 = segs.ray_seg_offset[r];
+            nhit = (int)(segs.ray_seg_offset[r + 1] - seg0);
+        }
+    }
+
     if constexpr (!TRAVERSE) {  // the hits kept by the counting pass, already sorted
-        nhit = (int)(segs.ray_seg_offset[r + 1] - segs.ray_seg_offset[r]);
+        if (!active) return;
         const int kmax = (int)(kept_per < ATDF_MAX_HITS ? kept_per : ATDF_MAX_HITS);
         nhit = max(0, min(nhit, kmax));
         for (int i = lane; i < nhit; i += 32)
@@ -202,7 +185,7 @@ __global__ void __launch_bounds__(kSegWarps * 32)
     {
         uint8_t f = tree.node_flags[0];
         float tmin, tmax;
-        bool hit = (f & 3) ? intersect_box(pmin, pmax, o, d, tmin, tmax) : false;
+        bool hit = active && (f & 3) ? intersect_box(pmin, pmax, o, d, tmin, tmax) : false;
         if (f & 1) {
             if (hit && !((double)__fsub_rn(tmax, tmin) < 1e-5)) {
                 nhit = 1;
@@ -277,13 +260,32 @@ __global__ void __launch_bounds__(kSegWarps * 32)
 
     if constexpr (!WRITE) {
         if (lane == 0) {
-            segs.ray_seg_offset[r] = nhit;
-            segs.ray_sample_offset[r] = nsamp;
-            atomicMax((unsigned long long*)&segs.totals[2], (unsigned long long)nsamp);
-            atomicMax((unsigned long long*)&segs.totals[3], (unsigned long long)nhit);
+            if (active) {
+                segs.ray_seg_offset[r] = nhit;
+                segs.ray_sample_offset[r] = nsamp;
+            }
+            s_sum[0][warp] = nhit;
+            s_sum[1][warp] = nsamp;
+        }
+        // the block's sums, and one atomic a block for the maxima (one a ray
+        // on the same two words cost as much as the traversal)
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            longlong2 sum = make_longlong2(0, 0);
+            int64_t most_n = 0, most_m = 0;
+            for (int k = 0; k < kSegWarps; ++k) {
+                sum.x += s_sum[0][k];
+                sum.y += s_sum[1][k];
+                most_n = max(most_n, s_sum[0][k]);
+                most_m = max(most_m, s_sum[1][k]);
+            }
+            if (sc.block_sums) sc.block_sums[blockIdx.x] = sum;
+            atomicMax((unsigned long long*)&segs.totals[2], (unsigned long long)most_m);
+            atomicMax((unsigned long long*)&segs.totals[3], (unsigned long long)most_n);
         }
         if constexpr (MODE == kSegCount) return;
     }
+    if (!active) return;
 
     if constexpr (TRAVERSE) {
         // sort the hits by (tmin, node): bitonic sort of the padded key array
@@ -321,19 +323,15 @@ __global__ void __launch_bounds__(kSegWarps * 32)
         return;
     }
 
-    const int64_t seg0 = segs.ray_seg_offset[r];
+    if constexpr (MODE == kSegWrite) seg0 = segs.ray_seg_offset[r];
     if (seg0 + nhit > segs.capacity) {
         if (lane == 0) set_err(err, ATDF_DEVERR_SEG_CAPACITY);
         return;
     }
-    // each lane owns up to 8 consecutive sorted hits
-    constexpr int PER = ATDF_MAX_HITS / 32;
-    int nloc[PER];
-    int lsum = 0;
-#pragma unroll
-    for (int q = 0; q < PER; ++q) {
-        const int i = lane * PER + q;
-        nloc[q] = 0;
+    int run = 0;
+    for (int i0 = 0; i0 < nhit; i0 += 32) {
+        const int i = i0 + lane;
+        int n = 0;
         if (i < nhit) {
             int node = (int)(key[i] & 0xffffffffu);
             if (node < 0 || node >= tree.num_nodes) {  // kept hits of a ray that overflowed its slots
@@ -342,27 +340,21 @@ __global__ void __launch_bounds__(kSegWarps * 32)
             }
             float tmin, tmax;
             intersect_box(pmin + 3 * (int64_t)node, pmax + 3 * (int64_t)node, o, d, tmin, tmax);
-            nloc[q] = seg_num_samples(pmin + 3 * (int64_t)node, pmax + 3 * (int64_t)node, tmin, tmax, M);
+            n = seg_num_samples(pmin + 3 * (int64_t)node, pmax + 3 * (int64_t)node, tmin, tmax, M);
             const int64_t s = seg0 + i;
             segs.node[s] = node;
             segs.tmin[s] = tmin;
             segs.tmax[s] = tmax;
-            segs.nsamp[s] = nloc[q];
+            segs.nsamp[s] = n;
             segs.ray[s] = (int32_t)r;
         }
-        lsum += nloc[q];
-    }
-    int incl = lsum;
-    for (int off = 1; off < 32; off <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, incl, off);
-        if (lane >= off) incl += v;
-    }
-    int run = incl - lsum;
-#pragma unroll
-    for (int q = 0; q < PER; ++q) {
-        const int i = lane * PER + q;
-        if (i < nhit) segs.first[seg0 + i] = run;
-        run += nloc[q];
+        int incl = n;
+        for (int off = 1; off < 32; off <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, incl, off);
+            if (lane >= off) incl += v;
+        }
+        if (i < nhit) segs.first[seg0 + i] = run + incl - n;
+        run += __shfl_sync(0xffffffffu, incl, 31);
     }
 }
 
@@ -472,43 +464,42 @@ __global__ void node_id_kernel(atdf_tree_t tree, const int64_t* __restrict__ act
     }
 }
 
-// Launch helpers shared with the fused path. kept_lo / kept_hi (nullable):
-// scratch of R * kept_per entries each where the counting pass keeps every
-// ray's sorted hits, so that the writing pass does not traverse the tree again.
+// The two passes over the rays. With scratch (the fused path) the counting
+// pass keeps every ray's sorted hits, so that the writing pass does not
+// traverse the tree again, and up to kScanBlocks blocks need no scan between
+// the passes.
+constexpr int64_t kScanBlocks = 4096;
+
 int launch_ray_segments(const atdf_tree_t& tree, const float* origin, const float* dir, int64_t R, int M,
-                        const atdf_segments_t& segs, int32_t* err, cudaStream_t st, uint32_t* kept_lo = nullptr,
-                        uint32_t* kept_hi = nullptr, int64_t kept_per = 0)
+                        const atdf_segments_t& segs, int32_t* err, cudaStream_t st, const SegScratch* scratch)
 {
     ATDF_CUDA_TRY(cudaMemsetAsync(segs.totals, 0, 4 * sizeof(int64_t), st));
     const int64_t blocks = div_up(R, kSegWarps);
-    const bool keep = kept_lo && kept_hi && kept_per > 0;
-    if (R > 0) {
-        if (keep)
-            ray_segments_kernel<kSegCountKeep><<<(unsigned)blocks, kSegWarps * 32, 0, st>>>(
-                tree, origin, dir, R, M, segs, err, kept_lo, kept_hi, kept_per);
-        else
-            ray_segments_kernel<kSegCount><<<(unsigned)blocks, kSegWarps * 32, 0, st>>>(tree, origin, dir, R, M, segs,
-                                                                                       err, nullptr, nullptr, 0);
-        ATDF_LAUNCH_CHECK();
-    } else {
+    SegScratch sc = {};
+    if (scratch) sc = *scratch;
+    const bool keep = sc.kept_lo && sc.kept_hi && sc.kept_per > 0;
+    if (!keep || blocks > kScanBlocks) sc.block_sums = nullptr;
+    if (R == 0) {
         ATDF_CUDA_TRY(cudaMemsetAsync(segs.ray_seg_offset, 0, sizeof(int64_t), st));
         ATDF_CUDA_TRY(cudaMemsetAsync(segs.ray_sample_offset, 0, sizeof(int64_t), st));
+        return ATDF_OK;
     }
-    scan2_exclusive_i64_kernel<<<2, 1024, 0, st>>>(segs.ray_seg_offset, segs.ray_sample_offset, R + 1);
+    (keep ? ray_segments_kernel<kSegCountKeep> : ray_segments_kernel<kSegCount>)<<<(unsigned)blocks, kSegWarps * 32, 0,
+                                                                                  st>>>(tree, origin, dir, R, M, segs,
+                                                                                        err, sc);
     ATDF_LAUNCH_CHECK();
-    ATDF_CUDA_TRY(cudaMemcpyAsync(&segs.totals[0], &segs.ray_seg_offset[R], sizeof(int64_t),
-                                  cudaMemcpyDeviceToDevice, st));
-    ATDF_CUDA_TRY(cudaMemcpyAsync(&segs.totals[1], &segs.ray_sample_offset[R], sizeof(int64_t),
-                                  cudaMemcpyDeviceToDevice, st));
-    if (R > 0) {
-        if (keep)
-            ray_segments_kernel<kSegWriteKept><<<(unsigned)blocks, kSegWarps * 32, 0, st>>>(
-                tree, origin, dir, R, M, segs, err, kept_lo, kept_hi, kept_per);
-        else
-            ray_segments_kernel<kSegWrite><<<(unsigned)blocks, kSegWarps * 32, 0, st>>>(tree, origin, dir, R, M, segs,
-                                                                                       err, nullptr, nullptr, 0);
+    if (!sc.block_sums) {
+        scan2_exclusive_i64_kernel<<<2, 1024, 0, st>>>(segs.ray_seg_offset, segs.ray_sample_offset, R + 1);
         ATDF_LAUNCH_CHECK();
+        ATDF_CUDA_TRY(cudaMemcpyAsync(&segs.totals[0], &segs.ray_seg_offset[R], sizeof(int64_t),
+                                      cudaMemcpyDeviceToDevice, st));
+        ATDF_CUDA_TRY(cudaMemcpyAsync(&segs.totals[1], &segs.ray_sample_offset[R], sizeof(int64_t),
+                                      cudaMemcpyDeviceToDevice, st));
     }
+    (keep ? ray_segments_kernel<kSegWriteKept> : ray_segments_kernel<kSegWrite>)<<<(unsigned)blocks, kSegWarps * 32, 0,
+                                                                                  st>>>(tree, origin, dir, R, M, segs,
+                                                                                        err, sc);
+    ATDF_LAUNCH_CHECK();
     return ATDF_OK;
 }
 
@@ -558,7 +549,7 @@ int atdf_ray_segments(const atdf_tree_t* tree, const float* ray_origin, const fl
         return ATDF_ERR_INVALID_ARGUMENT;
     if (num_rays >= (int64_t)1 << 31) return ATDF_ERR_UNSUPPORTED;
     return launch_ray_segments(*tree, ray_origin, ray_direction, num_rays, max_samples_per_node, *segs, dev_error,
-                               (cudaStream_t)stream);
+                               (cudaStream_t)stream, nullptr);
 }
 
 int atdf_emit_samples(const atdf_segments_t* segs, int64_t num_rays, const float* ray_origin,
