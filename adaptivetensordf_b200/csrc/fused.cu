@@ -20,6 +20,8 @@
 //  The backward kernels recompute each sample (no stored activations).
 
 #include <algorithm>
+#include <mutex>
+#include <vector>
 
 #include "fused_simt.cuh"
 
@@ -357,18 +359,51 @@ static int prepare(const atdf_tree_t* tree, const atdf_field_t* field, const atd
     return ATDF_OK;
 }
 
+// What the device's limits say about a kernel: blocks per SM and the shared
+// memory carve-out (percent) they need, the rest of the L1 holding texels. Asked
+// once per kernel and device; the answers depend on nothing else.
+struct LaunchShape {
+    const void* fn;
+    int dev, sms, per, carveout;
+};
+
+static int launch_shape(const void* fn, int smem, LaunchShape& out)
+{
+    static std::mutex lock;
+    static std::vector<LaunchShape> known;
+    int dev = 0;
+    ATDF_CUDA_TRY(cudaGetDevice(&dev));
+    {
+        std::lock_guard<std::mutex> g(lock);
+        for (const LaunchShape& k : known)
+            if (k.fn == fn && k.dev == dev) {
+                out = k;
+                return ATDF_OK;
+            }
+    }
+    int per_sm = 0;
+    out.fn = fn;
+    out.dev = dev;
+    ATDF_CUDA_TRY(cudaDeviceGetAttribute(&out.sms, cudaDevAttrMultiProcessorCount, dev));
+    ATDF_CUDA_TRY(cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
+    ATDF_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                       (int)cudaSharedmemCarveoutMaxShared));
+    ATDF_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&out.per, fn, simt::kThreads, smem));
+    if (out.per < 1) return ATDF_ERR_UNSUPPORTED;
+    out.carveout = std::min(100, (int)((int64_t)out.per * (smem + 1536) * 100 / per_sm) + 1);  // 1 KB a block is the system's
+    std::lock_guard<std::mutex> g(lock);
+    known.push_back(out);
+    return ATDF_OK;
+}
+
 static int launch_persistent(KernelFn fn, int smem, const FusedParams& p, cudaStream_t st)
 {
     if (smem > max_smem_optin()) return ATDF_ERR_UNSUPPORTED;
     ATDF_CUDA_TRY(cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    ATDF_CUDA_TRY(cudaFuncSetAttribute((const void*)fn, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                       (int)cudaSharedmemCarveoutMaxShared));
-    int dev = 0, sms = 0, per = 0;
-    ATDF_CUDA_TRY(cudaGetDevice(&dev));
-    ATDF_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    ATDF_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, (const void*)fn, simt::kThreads, smem));
-    if (per < 1) return ATDF_ERR_UNSUPPORTED;
-    fn<<<sms * per, simt::kThreads, smem, st>>>(p);
+    LaunchShape k;
+    if (const int e = launch_shape((const void*)fn, smem, k)) return e;
+    ATDF_CUDA_TRY(cudaFuncSetAttribute((const void*)fn, cudaFuncAttributePreferredSharedMemoryCarveout, k.carveout));
+    fn<<<k.sms * k.per, simt::kThreads, smem, st>>>(p);
     ATDF_LAUNCH_CHECK();
     return ATDF_OK;
 }
@@ -469,10 +504,21 @@ static int project_backward(const atdf_tree_t* tree, const atdf_field_t* field, 
                                                                                                 *field);
         ATDF_LAUNCH_CHECK();
     }
+    // the decoder's gradients, neighbouring arrays (one flat vector) at once
+    float* from = grad_mlp->weight[0];
+    float* to = from;
     for (int l = 0; l < mlp->num_layers; ++l) {
-        ATDF_CUDA_TRY(cudaMemsetAsync(grad_mlp->weight[l], 0, (size_t)mlp->dims[l] * mlp->dims[l + 1] * 4, s));
-        ATDF_CUDA_TRY(cudaMemsetAsync(grad_mlp->bias[l], 0, (size_t)mlp->dims[l + 1] * 4, s));
+        float* part[2] = {grad_mlp->weight[l], grad_mlp->bias[l]};
+        const size_t n[2] = {(size_t)mlp->dims[l] * mlp->dims[l + 1], (size_t)mlp->dims[l + 1]};
+        for (int k = 0; k < 2; ++k) {
+            if (part[k] != to) {
+                ATDF_CUDA_TRY(cudaMemsetAsync(from, 0, (to - from) * sizeof(float), s));
+                from = to = part[k];
+            }
+            to += n[k];
+        }
     }
+    ATDF_CUDA_TRY(cudaMemsetAsync(from, 0, (to - from) * sizeof(float), s));
     ATDF_CUDA_TRY(cudaMemsetAsync(p.ws.counters + 1, 0, 4, s));
     if (!var) return launch_tc_backward(p, s);
     if (p.line_rep > 0) ATDF_CUDA_TRY(cudaMemsetAsync(p.ws.seg_partial, 0, (size_t)p.line_rep * n * 4, s));

@@ -32,6 +32,7 @@ namespace simt {
 
 constexpr int kThreads = 128;
 constexpr int kGeo = 128;  // samples of one geometry pass
+constexpr int kMapCap = 2048;  // samples of an item covered by the sample -> segment map (2 KB of the L1)
 
 template <int C, int MODE, int H, int NH>
 struct Cfg {
@@ -74,7 +75,7 @@ struct Smem {
     static constexpr int zp = si + kGeo;                              // [CW][kGeo]
     static constexpr int dz = zp + K::CW * kGeo;                      // [T]
     static constexpr int seg = dz + K::T;
-    static constexpr int total = seg + kSegTabFloats;
+    static constexpr int total = seg + kSegTabFloats - (kSegMapCap - kMapCap) / 4;
 };
 
 // A sample's coordinates in shared memory, and back.
@@ -291,7 +292,7 @@ __global__ void __launch_bounds__(kThreads, 3) forward_kernel(FusedParams p)
     const float beta = p.mlp.softplus_beta;
     const int hact = p.mlp.hidden_activation, lact = p.mlp.last_activation;
     while (true) {
-        const ItemInfo it = next_item(p, 0, nullptr, tab, nullptr, s_ctl, false, kSegMapCap, true);
+        const ItemInfo it = next_item(p, 0, nullptr, tab, nullptr, s_ctl, false, kMapCap, true);
         if (it.slot < 0) break;
         const bool real = it.slot < p.ws.nslot;
         for (int t0 = 0; t0 < it.total; t0 += kGeo) {
@@ -370,7 +371,7 @@ __device__ __forceinline__ void red4(float* dst, float w, const float (&v)[4])
 }
 
 template <int C, int MODE, int H, int NH>
-__global__ void __launch_bounds__(kThreads, 2) backward_kernel(FusedParams p)
+__global__ void __launch_bounds__(kThreads, NH == 1 ? 3 : 2) backward_kernel(FusedParams p)
 {
     using K = Cfg<C, MODE, H, NH>;
     using S = Smem<C, MODE, H, NH, true>;
@@ -406,7 +407,7 @@ __global__ void __launch_bounds__(kThreads, 2) backward_kernel(FusedParams p)
     const int rx = (lane >> 2) + 8 * (warp & 1), cx = (lane & 3) + 4 * (warp >> 1);  // dX: rows rx + 16 i, columns cx + 8 j
 
     while (true) {
-        const ItemInfo it = next_item(p, 1, nullptr, tab, nullptr, s_ctl, true, kSegMapCap, true);
+        const ItemInfo it = next_item(p, 1, nullptr, tab, nullptr, s_ctl, true, kMapCap, true);
         if (it.slot < 0) break;
         const bool real = it.slot < p.ws.nslot;
         for (int t0 = 0; t0 < it.total; t0 += kGeo) {
@@ -571,16 +572,24 @@ __global__ void __launch_bounds__(kThreads, 2) backward_kernel(FusedParams p)
                 atomicAdd(&p.gmlp.weight[1][(o1 + 2 * i) * H + k1 + j], lo);
                 atomicAdd(&p.gmlp.weight[1][(o1 + 2 * i + 1) * H + k1 + j], hi);
             }
-    if (sg0 < K::SG)
+    // dW0's sample groups first add up in shared memory (x is free now): one
+    // global atomic per weight and block, since all blocks meet on the same
+    // few addresses here
+    for (int gg = 0; gg < K::SG; ++gg) {
+        if (sg0 == gg)
 #pragma unroll
-        for (int i = 0; i < 2; ++i)
+            for (int i = 0; i < 2; ++i)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                float lo, hi;
-                unpack2(gw0[i][j], lo, hi);
-                atomicAdd(&p.gmlp.weight[0][(o0 + 2 * i) * F + c0w + j], lo);
-                atomicAdd(&p.gmlp.weight[0][(o0 + 2 * i + 1) * F + c0w + j], hi);
-            }
+                for (int j = 0; j < 4; ++j) {
+                    float lo, hi;
+                    unpack2(gw0[i][j], lo, hi);
+                    float* q = sm + S::x + (o0 + 2 * i) * F + c0w + j;
+                    q[0] = gg == 0 ? lo : q[0] + lo;
+                    q[F] = gg == 0 ? hi : q[F] + hi;
+                }
+        __syncthreads();
+    }
+    for (int i = tid; i < H * F; i += kThreads) atomicAdd(&p.gmlp.weight[0][i], sm[S::x + i]);
 #pragma unroll
     for (int j = 0; j < 4; ++j)
 #pragma unroll

@@ -7,6 +7,8 @@
 #include <ATen/cuda/CUDAContext.h>
 #include <cuda_runtime_api.h>
 
+#include <array>
+
 #include "atdf_host.h"
 
 using torch::Tensor;
@@ -321,15 +323,58 @@ static std::vector<int64_t> layer_dims(const Decoder& dec)
     return dims;
 }
 
-static Tensor flat_params(const Decoder& dec)
+// The decoder's parameters as autograd inputs: weight and bias of each layer,
+// and a detached stand-in past the last (a custom function takes a fixed
+// number of defined tensors).
+// The function itself copies them into one flat vector for the kernels, so no
+// autograd node per parameter (reshape, concatenation and their adjoints)
+// stands between them and the projection.
+using DecoderInputs = std::array<Tensor, 2 * ATDF_MAX_LAYERS>;
+
+static DecoderInputs decoder_inputs(const Decoder& dec)
+{
+    layer_dims(dec);  // checks the number of layers
+    DecoderInputs t;
+    t.fill(dec.bias[0].detach());
+    for (size_t l = 0; l < dec.weight.size(); ++l) {
+        t[2 * l] = dec.weight[l];
+        t[2 * l + 1] = dec.bias[l];
+    }
+    return t;
+}
+
+static Tensor flat_params(const DecoderInputs& t, size_t layers)
 {
     std::vector<Tensor> parts;
-    for (size_t l = 0; l < dec.weight.size(); ++l) {
-        parts.push_back(dec.weight[l].reshape({-1}));
-        parts.push_back(dec.bias[l].reshape({-1}));
-    }
+    for (size_t i = 0; i < 2 * layers; ++i) parts.push_back(t[i].detach().reshape({-1}));
     return torch::cat(parts).contiguous();
 }
+
+// The gradients of the decoder's inputs as views of the flat gradient.
+static void append_decoder_grads(const std::vector<int64_t>& dims, const Tensor& gflat, tensor_list& out)
+{
+    int64_t off = 0;
+    for (size_t l = 0; l < ATDF_MAX_LAYERS; ++l) {
+        if (l + 1 >= dims.size()) {
+            out.push_back(Tensor());
+            out.push_back(Tensor());
+            continue;
+        }
+        const int64_t nw = dims[l] * dims[l + 1], nb = dims[l + 1];
+        out.push_back(gflat.slice(0, off, off + nw).view({dims[l + 1], dims[l]}));
+        off += nw;
+        out.push_back(gflat.slice(0, off, off + nb));
+        off += nb;
+    }
+}
+
+#define ATDF_DECODER_PARAMS                                                                                  \
+    Tensor w0, Tensor b0, Tensor w1, Tensor b1, Tensor w2, Tensor b2, Tensor w3, Tensor b3, Tensor w4, Tensor b4, \
+        Tensor w5, Tensor b5, Tensor w6, Tensor b6, Tensor w7, Tensor b7
+#define ATDF_DECODER_NAMES w0, b0, w1, b1, w2, b2, w3, b3, w4, b4, w5, b5, w6, b6, w7, b7
+#define ATDF_DECODER_UNPACK(t) \
+    t[0], t[1], t[2], t[3], t[4], t[5], t[6], t[7], t[8], t[9], t[10], t[11], t[12], t[13], t[14], t[15]
+static_assert(ATDF_MAX_LAYERS == 8, "the parameter lists above hold 8 layers");
 
 // MLP view whose weights point into the flat vector.
 static atdf_mlp_t mlp_view(const std::vector<int64_t>& dims, const float* flat, int act, int last, float beta)
@@ -373,10 +418,12 @@ atdf_mlp_t Decoder::view() const
 
 class MlpFn : public torch::autograd::Function<MlpFn> {
    public:
-    static Tensor forward(AutogradContext* ctx, Tensor x, Tensor flat, std::vector<int64_t> dims, int64_t act,
+    static Tensor forward(AutogradContext* ctx, Tensor x, ATDF_DECODER_PARAMS, std::vector<int64_t> dims, int64_t act,
                           int64_t last, double beta)
     {
         ATDF_CHECK_CUDA(x);
+        auto flat = flat_params({ATDF_DECODER_NAMES}, dims.size() - 1);
+        ATDF_CHECK_CUDA(flat);
         auto xc = x.reshape({-1, dims[0]}).contiguous();
         auto m = mlp_view(dims, flat.data_ptr<float>(), (int)act, (int)last, (float)beta);
         auto out = torch::empty({xc.size(0), dims.back()}, xc.options());
@@ -406,14 +453,18 @@ class MlpFn : public torch::autograd::Function<MlpFn> {
         check_status(atdf_mlp_backward(&m, xc.data_ptr<float>(), xc.size(0), g.data_ptr<float>(), gx.data_ptr<float>(),
                                        &gv, stream_arg()),
                      "DecodeFeatures backward");
-        return {gx.reshape(ctx->saved_data["xshape"].toIntVector()), gflat, Tensor(), Tensor(), Tensor(), Tensor()};
+        tensor_list grads{gx.reshape(ctx->saved_data["xshape"].toIntVector())};
+        append_decoder_grads(dims, gflat, grads);
+        for (int i = 0; i < 4; ++i) grads.push_back(Tensor());
+        return grads;
     }
 };
 
 Tensor DecodeFeatures(const Decoder& dec, Tensor features)
 {
     auto dims = layer_dims(dec);
-    return MlpFn::apply(features, flat_params(dec), dims, activation_id(dec.activation),
+    auto t = decoder_inputs(dec);
+    return MlpFn::apply(features, ATDF_DECODER_UNPACK(t), dims, activation_id(dec.activation),
                         activation_id(dec.last_activation), dec.softplus_beta);
 }
 
@@ -654,9 +705,11 @@ struct ProjectArgs {
 class ProjectFn : public torch::autograd::Function<ProjectFn> {
    public:
     static Tensor forward(AutogradContext* ctx, Tensor origin, Tensor dir, Tensor p0, Tensor p1, Tensor p2, Tensor l0,
-                          Tensor l1, Tensor l2, Tensor flat, int64_t args_ptr)
+                          Tensor l1, Tensor l2, ATDF_DECODER_PARAMS, int64_t args_ptr)
     {
         auto* a = reinterpret_cast<ProjectArgs*>(args_ptr);
+        auto flat = flat_params({ATDF_DECODER_NAMES}, a->geo->decoder.weight.size());
+        ATDF_CHECK_CUDA(flat);
         std::vector<Tensor> P{p0, p1, p2}, L{l0, l1, l2};
         auto f = fused_field_view(*a->geo, P, L);
         auto dims = layer_dims(a->geo->decoder);
@@ -747,7 +800,10 @@ class ProjectFn : public torch::autograd::Function<ProjectFn> {
                                                stream_arg()),
                          "ProjectRays backward");
         }
-        return {Tensor(), Tensor(), gp[0], gp[1], gp[2], gl[0], gl[1], gl[2], gflat, Tensor()};
+        tensor_list grads{Tensor(), Tensor(), gp[0], gp[1], gp[2], gl[0], gl[1], gl[2]};
+        append_decoder_grads(dims, gflat, grads);
+        grads.push_back(Tensor());
+        return grads;
     }
 };
 
@@ -786,7 +842,8 @@ static Tensor project_apply(GeometryTensorQO& geo, ProjectArgs& args, const RayL
         P.push_back(channels_last(geo.planes[m]));
         L.push_back(channels_last(geo.lines[m]));
     }
-    return ProjectFn::apply(rays.origin, rays.direction, P[0], P[1], P[2], L[0], L[1], L[2], flat_params(geo.decoder),
+    auto t = decoder_inputs(geo.decoder);
+    return ProjectFn::apply(rays.origin, rays.direction, P[0], P[1], P[2], L[0], L[1], L[2], ATDF_DECODER_UNPACK(t),
                             reinterpret_cast<int64_t>(&args));
 }
 
@@ -811,7 +868,7 @@ std::tuple<Tensor, Tensor, Tensor> GeometryTensorQO::ProjectNodeError(HyperTreeB
     }
     auto f = fused_field_view(*this, P, L);
     auto dims = layer_dims(decoder);
-    auto flat = flat_params(decoder);
+    auto flat = flat_params(decoder_inputs(decoder), decoder.weight.size());
     auto m = mlp_view(dims, flat.data_ptr<float>(), activation_id(decoder.activation),
                       activation_id(decoder.last_activation), (float)decoder.softplus_beta);
     auto t = tree.view();
