@@ -32,7 +32,7 @@ namespace simt {
 
 constexpr int kThreads = 128;
 constexpr int kGeo = 128;  // samples of one geometry pass
-constexpr int kMapCap = 2048;  // samples of an item covered by the sample -> segment map (2 KB of the L1)
+constexpr int kMapCap = 2048;  // samples of an item covered by the sample -> segment map (2 KB), where there is room
 
 template <int C, int MODE, int H, int NH>
 struct Cfg {
@@ -70,12 +70,17 @@ struct Smem {
     static constexpr int x = bl + 4;                                  // [T][XP]
     static constexpr int h = x + K::T * K::XP;                        // [T][HP]: H0, then dA0
     static constexpr int d = h + (NH == 2 || BWD ? K::T * K::HP : 0);  // [T][HP]: dA1
-    static constexpr int geo = d + (NH == 2 && BWD ? K::T * K::HP : 0);  // [7][kGeo]
-    static constexpr int si = geo + 7 * kGeo;                         // [kGeo]
-    static constexpr int zp = si + kGeo;                              // [CW][kGeo]
-    static constexpr int dz = zp + K::CW * kGeo;                      // [T]
-    static constexpr int seg = dz + K::T;
-    static constexpr int total = seg + kSegTabFloats - (kSegMapCap - kMapCap) / 4;
+    static constexpr int geo = d + (NH == 2 && BWD ? K::T * K::HP : 0);  // [6][kGeo], forward also t
+    static constexpr int si = geo + (BWD ? 6 : 7) * kGeo;             // [kGeo]
+    static constexpr int zrow = BWD ? K::T : kGeo;
+    static constexpr int zp = si + kGeo;                              // [CW][zrow]
+    static constexpr int dz = zp + K::CW * zrow;                      // [T]
+    static constexpr int stash = dz + K::T;                           // adjoint: [GI][3][V][kThreads] float4
+    static constexpr int seg = stash + (BWD ? K::GI * 3 * K::V * kThreads * 4 : 0);
+    static constexpr int map_cap = BWD && NH == 2 ? 0 : kMapCap;
+    static constexpr int total = seg + kSegTabFloats - (kSegMapCap - map_cap) / 4;
+    // two blocks an SM (1 KB of each is the system's)
+    static_assert(2 * (total * 4 + 1024) <= 228 * 1024 - 1024, "shared memory");
 };
 
 // A sample's coordinates in shared memory, and back.
@@ -130,17 +135,21 @@ __device__ __forceinline__ Tap tap(const FusedParams& p, const SampleGeo& g, int
     return t;
 }
 
-// The plane's bilinear and the line's linear values of the 4 channels at c0;
-// P: the slot's plane.
-__device__ __forceinline__ void tap_values(const Tap& t, const float* P, const float* V, int c0, float (&mat)[4],
-                                           float (&vec)[4])
+// The plane's bilinear values (P: the slot's plane) and the line's linear
+// values of the 4 channels at c0.
+__device__ __forceinline__ void tap_matrix(const Tap& t, const float* P, int c0, float (&mat)[4])
 {
     const float4 nw = ldg4(P + t.o[0] + c0), ne = ldg4(P + t.o[1] + c0), sw = ldg4(P + t.o[2] + c0),
-                 se = ldg4(P + t.o[3] + c0), v0 = ldg4(V + t.l0 + c0), v1 = ldg4(V + t.l1 + c0);
+                 se = ldg4(P + t.o[3] + c0);
     mat[0] = bilerp(t.k, nw.x, ne.x, sw.x, se.x);
     mat[1] = bilerp(t.k, nw.y, ne.y, sw.y, se.y);
     mat[2] = bilerp(t.k, nw.z, ne.z, sw.z, se.z);
     mat[3] = bilerp(t.k, nw.w, ne.w, sw.w, se.w);
+}
+
+__device__ __forceinline__ void tap_vector(const Tap& t, const float* V, int c0, float (&vec)[4])
+{
+    const float4 v0 = ldg4(V + t.l0 + c0), v1 = ldg4(V + t.l1 + c0);
     vec[0] = lerp1(t.l, v0.x, v1.x);
     vec[1] = lerp1(t.l, v0.y, v1.y);
     vec[2] = lerp1(t.l, v0.z, v1.z);
@@ -155,9 +164,12 @@ __device__ __forceinline__ int64_t plane_base(const FusedParams& p, int64_t slot
 
 // Features of the tile's samples [s0, s0 + T) of the geometry pass into x
 // (zeros for samples past the item's end and outside the region of interest).
-template <int C, int MODE, int H, int NH>
+// stash (adjoint): the planes' bilinear values, for the line gradients of the
+// same thread's samples; gathering them a second time cost as much as the
+// features.
+template <int C, int MODE, int H, int NH, bool STASH>
 __device__ __forceinline__ void gather_tile(const FusedParams& p, int64_t slot, bool real, const float* geo, int s0,
-                                            int left, float* x)
+                                            int left, float* x, float* stash)
 {
     using K = Cfg<C, MODE, H, NH>;
     constexpr int V = K::V;
@@ -179,7 +191,11 @@ __device__ __forceinline__ void gather_tile(const FusedParams& p, int64_t slot, 
 #pragma unroll
                 for (int v = 0; v < V; ++v) {
                     float mat[4], vec[4];
-                    tap_values(t, P, (const float*)p.field.line[m], c0 + 4 * K::Q * v, mat, vec);
+                    tap_matrix(t, P, c0 + 4 * K::Q * v, mat);
+                    tap_vector(t, (const float*)p.field.line[m], c0 + 4 * K::Q * v, vec);
+                    if (STASH)
+                        *reinterpret_cast<float4*>(stash + (((it * 3 + m) * V + v) * kThreads + threadIdx.x) * 4) =
+                            make_float4(mat[0], mat[1], mat[2], mat[3]);
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
                         const float x = __fmul_rn(mat[i], vec[i]);
@@ -233,15 +249,8 @@ __device__ __forceinline__ void tile_place(int& rg, int& cg, int& cw)
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     cw = warp % K::CW;
-    rg = (lane >> 2) + 8 * (warp / K::CW);
-    cg = (lane & 3) + 4 * cw;
-}
-
-// Sum over the 4 lanes that share a row group's rows.
-__device__ __forceinline__ float sum_quad(float v)
-{
-    v += __shfl_xor_sync(0xffffffffu, v, 1);
-    return v + __shfl_xor_sync(0xffffffffu, v, 2);
+    rg = lane_row(lane) + 8 * (warp / K::CW);
+    cg = lane_col(lane) + 4 * cw;
 }
 
 // Geometry of the item's samples [t0, t0 + kGeo), one per thread. dI: keep
@@ -255,7 +264,7 @@ __device__ __forceinline__ void geometry_pass(const FusedParams& p, const SegTab
         const SampleGeo g = sample_geo_fast(p, tab, st.node, st.pos);
         store_geo(geo, s, g, dI ? __fmul_rn(tab.acc[st.si], st.w) : st.w);
         si[s] = st.si;
-        geo[6 * kGeo + s] = st.t;
+        if (!dI) geo[6 * kGeo + s] = st.t;
     } else {
         geo[5 * kGeo + s] = 0.0f;
         si[s] = -1;
@@ -292,14 +301,14 @@ __global__ void __launch_bounds__(kThreads, 3) forward_kernel(FusedParams p)
     const float beta = p.mlp.softplus_beta;
     const int hact = p.mlp.hidden_activation, lact = p.mlp.last_activation;
     while (true) {
-        const ItemInfo it = next_item(p, 0, nullptr, tab, nullptr, s_ctl, false, kMapCap, true);
+        const ItemInfo it = next_item(p, 0, nullptr, tab, nullptr, s_ctl, false, S::map_cap, true);
         if (it.slot < 0) break;
         const bool real = it.slot < p.ws.nslot;
         for (int t0 = 0; t0 < it.total; t0 += kGeo) {
             geometry_pass(p, tab, it, t0, false, geo, si);
             __syncthreads();
             for (int s0 = 0; s0 < kGeo && t0 + s0 < it.total; s0 += K::T) {
-                gather_tile<C, MODE, H, NH>(p, it.slot, real, geo, s0, it.total - t0 - s0, sm + S::x);
+                gather_tile<C, MODE, H, NH, false>(p, it.slot, real, geo, s0, it.total - t0 - s0, sm + S::x, nullptr);
                 __syncthreads();
                 uint64_t acc[8][4];
                 layer0<C, MODE, H, NH, false>(sm, rg, cg, acc);
@@ -328,15 +337,15 @@ __global__ void __launch_bounds__(kThreads, 3) forward_kernel(FusedParams p)
                 }
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
-                    z[i] = sum_quad(z[i]);
-                    if ((tid & 3) == 0) sm[S::zp + cw * kGeo + s0 + rg + i * K::RG] = z[i];
+                    z[i] = sum_cols(z[i]);
+                    if ((tid & 6) == 0) sm[S::zp + cw * S::zrow + s0 + rg + i * K::RG] = z[i];
                 }
             }
             __syncthreads();
             {
                 float zz = sm[S::bl];
 #pragma unroll
-                for (int w = 0; w < K::CW; ++w) zz += sm[S::zp + w * kGeo + tid];
+                for (int w = 0; w < K::CW; ++w) zz += sm[S::zp + w * S::zrow + tid];
                 const int sg = si[tid];
                 if (__any_sync(0xffffffffu, sg >= 0)) {
                     const float v = __fmul_rn(act_fwd(lact, zz, beta), geo[5 * kGeo + tid]);
@@ -399,15 +408,15 @@ __global__ void __launch_bounds__(kThreads, NH == 1 ? 3 : 2) backward_kernel(Fus
     uint64_t gw1[4][4], gw0[2][4];
     zero2<4, 4>(gw1);
     zero2<2, 4>(gw0);
-    const int o1 = 8 * (lane >> 2), k1 = 4 * ((lane & 3) + 4 * warp);
+    const int o1 = 8 * lane_row(lane), k1 = 4 * (lane_col(lane) + 4 * warp);
     const int u0 = tid % K::W0T, sg0 = tid / K::W0T;
     const int o0 = 4 * (u0 / (F / 4)), c0w = 4 * (u0 % (F / 4));
     float gb0[4] = {0.f, 0.f, 0.f, 0.f}, gb1[4] = {0.f, 0.f, 0.f, 0.f}, gwl[4] = {0.f, 0.f, 0.f, 0.f};
     double gbl = 0.0;  // one scalar summed over every sample: FP64 against cancellation
-    const int rx = (lane >> 2) + 8 * (warp & 1), cx = (lane & 3) + 4 * (warp >> 1);  // dX: rows rx + 16 i, columns cx + 8 j
+    const int rx = lane_row(lane) + 8 * (warp & 1), cx = lane_col(lane) + 4 * (warp >> 1);  // dX: rows rx + 16 i, columns cx + 8 j
 
     while (true) {
-        const ItemInfo it = next_item(p, 1, nullptr, tab, nullptr, s_ctl, true, kMapCap, true);
+        const ItemInfo it = next_item(p, 1, nullptr, tab, nullptr, s_ctl, true, S::map_cap, true);
         if (it.slot < 0) break;
         const bool real = it.slot < p.ws.nslot;
         for (int t0 = 0; t0 < it.total; t0 += kGeo) {
@@ -415,7 +424,7 @@ __global__ void __launch_bounds__(kThreads, NH == 1 ? 3 : 2) backward_kernel(Fus
             __syncthreads();
             for (int s0 = 0; s0 < kGeo && t0 + s0 < it.total; s0 += T) {
                 const int left = it.total - t0 - s0;
-                gather_tile<C, MODE, H, NH>(p, it.slot, real, geo, s0, left, sm + S::x);
+                gather_tile<C, MODE, H, NH, true>(p, it.slot, real, geo, s0, left, sm + S::x, sm + S::stash);
                 __syncthreads();
                 // ---- forward recompute: h and g, the last hidden layer's
                 // activation and derivative; g0 the first one's derivative
@@ -451,14 +460,14 @@ __global__ void __launch_bounds__(kThreads, NH == 1 ? 3 : 2) backward_kernel(Fus
                     float z = 0.0f;
 #pragma unroll
                     for (int j = 0; j < 4; ++j) z = fmaf(h[i][j], sm[S::wl + cg + j * K::CG], z);
-                    z = sum_quad(z);
-                    if ((tid & 3) == 0) sm[S::zp + cw * kGeo + rg + i * K::RG] = z;
+                    z = sum_cols(z);
+                    if ((tid & 6) == 0) sm[S::zp + cw * S::zrow + rg + i * K::RG] = z;
                 }
                 __syncthreads();
                 if (tid < T) {
                     float z = sm[S::bl];
 #pragma unroll
-                    for (int w = 0; w < K::CW; ++w) z += sm[S::zp + w * kGeo + tid];
+                    for (int w = 0; w < K::CW; ++w) z += sm[S::zp + w * S::zrow + tid];
                     const float dz = geo[5 * kGeo + s0 + tid] * act_grad(lact, z, beta);
                     sm[S::dz + tid] = dz;
                     gbl += (double)dz;
@@ -531,14 +540,15 @@ __global__ void __launch_bounds__(kThreads, NH == 1 ? 3 : 2) backward_kernel(Fus
 #pragma unroll
                         for (int v = 0; v < K::V; ++v) {
                             const int c = c0 + 4 * K::Q * v;
-                            float mat[4], vec[4];
-                            tap_values(t, (const float*)p.field.plane[m] + base, (const float*)p.field.line[m], c, mat,
-                                       vec);
+                            float vec[4];
+                            tap_vector(t, (const float*)p.field.line[m], c, vec);
+                            const float4 mat = *reinterpret_cast<const float4*>(
+                                sm + S::stash + (((e0 * 3 + m) * K::V + v) * kThreads + tid) * 4);
                             const float4 gf = *reinterpret_cast<const float4*>(sm + S::x + s * K::XP + (MODE ? m * C : 0) + c);
                             const float gm[4] = {__fmul_rn(gf.x, vec[0]), __fmul_rn(gf.y, vec[1]),
                                                  __fmul_rn(gf.z, vec[2]), __fmul_rn(gf.w, vec[3])};
-                            const float gv[4] = {__fmul_rn(gf.x, mat[0]), __fmul_rn(gf.y, mat[1]),
-                                                 __fmul_rn(gf.z, mat[2]), __fmul_rn(gf.w, mat[3])};
+                            const float gv[4] = {__fmul_rn(gf.x, mat.x), __fmul_rn(gf.y, mat.y),
+                                                 __fmul_rn(gf.z, mat.z), __fmul_rn(gf.w, mat.w)};
                             red4(GP + t.o[0] + c, t.k.w_nw, gm);
                             red4(GP + t.o[1] + c, t.k.w_ne, gm);
                             red4(GP + t.o[2] + c, t.k.w_sw, gm);
@@ -591,14 +601,12 @@ __global__ void __launch_bounds__(kThreads, NH == 1 ? 3 : 2) backward_kernel(Fus
     }
     for (int i = tid; i < H * F; i += kThreads) atomicAdd(&p.gmlp.weight[0][i], sm[S::x + i]);
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-#pragma unroll
-        for (int off = 4; off < 32; off <<= 1) {
-            gwl[j] += __shfl_xor_sync(0xffffffffu, gwl[j], off);
-            gb0[j] += __shfl_xor_sync(0xffffffffu, gb0[j], off);
-            gb1[j] += __shfl_xor_sync(0xffffffffu, gb1[j], off);
-        }
-    if (lane < 4)
+    for (int j = 0; j < 4; ++j) {
+        gwl[j] = sum_rows(gwl[j]);
+        gb0[j] = sum_rows(gb0[j]);
+        gb1[j] = sum_rows(gb1[j]);
+    }
+    if (lane_row(lane) == 0)
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const int c = cg + j * K::CG;

@@ -178,7 +178,7 @@ __device__ __forceinline__ void tile_layer(const float* A, int ap, const float* 
         }
         return;
     }
-    const int rg = (lane >> 2) + 8 * (warp >> 2), cg = (lane & 3) + 4 * (warp & 3);
+    const int rg = lane_row(lane) + 8 * (warp >> 2), cg = lane_col(lane) + 4 * (warp & 3);
     const float* a = A + rg * ap;
     for (int c0 = 0; c0 < n; c0 += 64) {
         const float* b = B + (c0 + cg) * bp;

@@ -6,16 +6,17 @@
 // as two packed pairs (fma.rn.f32x2): a pair accumulates the even and the odd
 // terms, added at the end. Each lane is a plain FP32 fma.
 //
-// Lanes of a warp: lane / 4 picks the rows (A), lane % 4 the columns (B). On
-// sm_100a a warp's 16-byte shared load takes 2 cycles when neighbouring lanes
-// read the same address (A) and 4 otherwise (B; measured 2.06 and 3.9 cycles
-// an SM), so an 8 x 4 tile of outputs per thread costs 8 * 2 + 4 * 4 = 32
-// load cycles per 4 steps of the contraction against 32 cycles of its 128
-// FMAs per lane at 128 a cycle: both pipes are near balance, and a smaller
-// tile would be bound by the loads. Rows and columns of a thread are
-// interleaved (row i * groups + group), and the pitches are 4 mod 32 floats
-// (or 12, 20, 28) apart, so the distinct addresses of a load fall into
-// distinct banks.
+// Lanes of a warp: bits 0, 3, 4 of the lane pick the rows (A), bits 1, 2 the
+// columns (B): lane_row, lane_col. On sm_100a a warp's 16-byte shared load
+// takes 2.1 cycles when either neighbouring lanes or every other lane of each
+// 8 read the same address, and 3.9 otherwise; with this mapping both operands'
+// loads are of the cheap kind (lane / 4 and lane % 4 left B's at 3.9). An
+// 8 x 4 tile of outputs per thread costs 12 * 2.1 = 25 load cycles per 4 steps
+// of the contraction against 32 cycles of its 128 FMAs per lane at 128 a
+// cycle; a smaller tile would be bound by the loads. Rows and columns of a
+// thread are interleaved (row i * groups + group), and the pitches are 4 mod
+// 32 floats (or 12, 20, 28) apart, so the distinct addresses of a load fall
+// into distinct banks.
 #pragma once
 
 #include <stdint.h>
@@ -23,6 +24,24 @@
 #include "atdf_common.cuh"
 
 namespace atdf {
+
+__device__ __forceinline__ int lane_row(int lane) { return (lane & 1) | ((lane >> 3) << 1); }  // 0..7
+__device__ __forceinline__ int lane_col(int lane) { return (lane >> 1) & 3; }                     // 0..3
+
+// Sum over the 4 lanes that share a row.
+__device__ __forceinline__ float sum_cols(float v)
+{
+    v += __shfl_xor_sync(0xffffffffu, v, 2);
+    return v + __shfl_xor_sync(0xffffffffu, v, 4);
+}
+
+// Sum over the 8 lanes that share a column.
+__device__ __forceinline__ float sum_rows(float v)
+{
+    v += __shfl_xor_sync(0xffffffffu, v, 1);
+    v += __shfl_xor_sync(0xffffffffu, v, 8);
+    return v + __shfl_xor_sync(0xffffffffu, v, 16);
+}
 
 __device__ __forceinline__ uint64_t ffma2(uint64_t a, uint64_t b, uint64_t c)
 {
