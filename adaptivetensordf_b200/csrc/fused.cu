@@ -168,12 +168,15 @@ __global__ void zero_untouched_slots_kernel(Ws w, atdf_field_grad_t g, atdf_fiel
     }
 }
 
-// Sum of the line gradients' copies, in FP64 (one rounding at the end).
-__global__ void line_reduce_kernel(const float* __restrict__ rep, int n_rep, int n, int n0, int n1, float* g0,
-                                   float* g1, float* g2)
+// End of the FP32 adjoint: the sum of the line gradients' copies (n_rep > 0)
+// and the last bias' gradient, both in FP64 with one rounding at the end. The
+// last bias is one sum over every sample whose terms largely cancel.
+__global__ void adjoint_end_kernel(const float* __restrict__ rep, int n_rep, int n, int n0, int n1, float* g0,
+                                   float* g1, float* g2, const double* __restrict__ last_sum, float* last_bias)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+    if (i == 0) *last_bias = (float)*last_sum;
+    if (n_rep == 0 || i >= n) return;
     double acc = 0.0;
     for (int r = 0; r < n_rep; ++r) acc += (double)rep[(int64_t)r * n + i];
     (i < n0 ? g0[i] : i < n0 + n1 ? g1[i - n0] : g2[i - n0 - n1]) = (float)acc;
@@ -522,11 +525,12 @@ static int project_backward(const atdf_tree_t* tree, const atdf_field_t* field, 
     ATDF_CUDA_TRY(cudaMemsetAsync(p.ws.counters + 1, 0, 4, s));
     if (!var) return launch_tc_backward(p, s);
     if (p.line_rep > 0) ATDF_CUDA_TRY(cudaMemsetAsync(p.ws.seg_partial, 0, (size_t)p.line_rep * n * 4, s));
+    ATDF_CUDA_TRY(cudaMemsetAsync(p.ws.last_sum, 0, sizeof(double), s));
     st = launch_persistent(var->bwd, var->smem(true), p, s);
-    if (st != ATDF_OK || p.line_rep == 0) return st;
-    line_reduce_kernel<<<(unsigned)div_up(n, 128), 128, 0, s>>>(p.ws.seg_partial, p.line_rep, (int)n, ll[0], ll[1],
-                                                                grad_field->line[0], grad_field->line[1],
-                                                                grad_field->line[2]);
+    if (st != ATDF_OK) return st;
+    adjoint_end_kernel<<<p.line_rep > 0 ? (unsigned)div_up(n, 128) : 1, 128, 0, s>>>(
+        p.ws.seg_partial, p.line_rep, (int)n, ll[0], ll[1], grad_field->line[0], grad_field->line[1],
+        grad_field->line[2], p.ws.last_sum, grad_mlp->bias[mlp->num_layers - 1]);
     ATDF_LAUNCH_CHECK();
     return ATDF_OK;
 }

@@ -32,6 +32,7 @@ struct Ws {
     float* seg_partial;
     int32_t* bucket;
     int32_t* counters;     // [8]: the queues' positions (0, 1), the item queue's length (4)
+    double* last_sum;      // 64 bytes after the counters: the FP32 adjoint's last bias gradient
     int32_t* slot_offset;  // [nslot + 2], 256 bytes after the counters
     int32_t* slot_order;   // [nslot + 1]: the slot queue
     int32_t* item_offset;  // [nslot + 2]
@@ -71,7 +72,8 @@ static size_t ws_layout(int64_t R, int max_depth, int64_t nslot, char* base, Ws*
     x.first = (int32_t*)carve(p, cap * 4);
     x.seg_partial = (float*)carve(p, cap * 4);
     x.bucket = (int32_t*)carve(p, cap * 4);
-    x.counters = (int32_t*)carve(p, 8 * 4);
+    x.counters = (int32_t*)carve(p, 256);
+    x.last_sum = (double*)((char*)x.counters + 64);
     x.slot_offset = (int32_t*)carve(p, (nslot + 2) * 4);
     x.slot_order = (int32_t*)carve(p, (nslot + 1) * 4);
     x.item_offset = (int32_t*)carve(p, (nslot + 2) * 4);

@@ -615,7 +615,7 @@ __global__ void __launch_bounds__(kThreads, NH == 1 ? 3 : 2) backward_kernel(Fus
             if (NH == 2) atomicAdd(&p.gmlp.bias[1][c], gb1[j]);
         }
     for (int off = 16; off > 0; off >>= 1) gbl += __shfl_down_sync(0xffffffffu, gbl, off);
-    if (lane == 0) atomicAdd(&p.gmlp.bias[NH][0], (float)gbl);
+    if (lane == 0) atomicAdd(p.ws.last_sum, gbl);
 }
 
 }  // namespace simt
