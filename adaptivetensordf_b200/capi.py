@@ -173,6 +173,7 @@ def _declare(L):
                                                U64, P, P, P]),
         "atdf_siddon_project": (I32, [P, I32, I32, I32, ct.POINTER(ct.c_double), ct.POINTER(ct.c_double), P, P,
                                       I64, P, P]),
+        "atdf_field_density": (I32, [ct.POINTER(Field), ct.POINTER(Mlp), P, P, I64, P, P, I64, P, P, P]),
         "atdf_project_forward_segmented": (I32, [ct.POINTER(Tree), ct.POINTER(Field), ct.POINTER(Mlp), P, P, I64, U64,
                                                  P, P, SZ, P, P]),
         "atdf_project_forward_binned": (I32, [ct.POINTER(Tree), ct.POINTER(Field), ct.POINTER(Mlp), P, P, I64, I32,

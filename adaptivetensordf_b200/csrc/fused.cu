@@ -248,9 +248,12 @@ __global__ void __launch_bounds__(256) node_error_kernel(Ws w, const float* __re
 // ---------------------------------------------------------------------------
 using KernelFn = void (*)(FusedParams);
 
+using PointsFn = void (*)(FusedParams, simt::PointArgs);
+
 struct Variant {
     int C, mode, H, NH;
     KernelFn fwd, bwd;
+    PointsFn points;
     int (*smem)(bool);
 };
 
@@ -273,7 +276,8 @@ static int plane_limit(int C, int F, int H, int NH, bool bwd)
 }
 
 #define ATDF_VARIANT(C, M, H, NH) \
-    {C, M, H, NH, simt::forward_kernel<C, M, H, NH>, simt::backward_kernel<C, M, H, NH>, smem_bytes<C, M, H, NH>}
+    {C, M, H, NH, simt::forward_kernel<C, M, H, NH>, simt::backward_kernel<C, M, H, NH>, \
+     simt::points_kernel<C, M, H, NH>, smem_bytes<C, M, H, NH>}
 
 static const Variant kVariants[] = {
     ATDF_VARIANT(8, 0, 32, 1),  ATDF_VARIANT(8, 0, 64, 1),  ATDF_VARIANT(8, 0, 64, 2),
@@ -540,6 +544,42 @@ static int project_backward(const atdf_tree_t* tree, const atdf_field_t* field, 
 using namespace atdf;
 
 extern "C" {
+
+int atdf_field_density(const atdf_field_t* field, const atdf_mlp_t* mlp, const float* pmin, const float* pmax,
+                       int64_t num_nodes, const float* position, const int64_t* node_id, int64_t num_points, float* out,
+                       int32_t* dev_error, atdf_stream_t stream)
+{
+    if (!field || !mlp || !pmin || !pmax || num_points < 0 || (num_points > 0 && (!position || !node_id || !out)) ||
+        !field->leaf_slot)
+        return ATDF_ERR_INVALID_ARGUMENT;
+    const Variant* var = field->dtype == ATDF_F32 ? find_variant(field, mlp) : nullptr;
+    if (!var || field->num_slots > INT32_MAX) return ATDF_ERR_UNSUPPORTED;
+    for (int l = 0; l < mlp->num_layers; ++l)
+        if (!mlp->weight[l] || !mlp->bias[l]) return ATDF_ERR_INVALID_ARGUMENT;
+    for (int m = 0; m < 3; ++m)
+        if (!field->plane[m] || !field->line[m] || ((uintptr_t)field->plane[m] & 15) || ((uintptr_t)field->line[m] & 15))
+            return ATDF_ERR_UNSUPPORTED;
+    if (num_points == 0) return ATDF_OK;
+    FusedParams p = {};
+    p.field = *field;
+    p.mlp = *mlp;
+    p.tree.node_position_min = pmin;
+    p.tree.node_position_max = pmax;
+    p.tree.num_nodes = num_nodes;
+    p.err = dev_error;
+    const int smem = var->smem(false);
+    if (smem > max_smem_optin()) return ATDF_ERR_UNSUPPORTED;
+    ATDF_CUDA_TRY(cudaFuncSetAttribute((const void*)var->points, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    LaunchShape k;
+    if (const int e = launch_shape((const void*)var->points, smem, k)) return e;
+    ATDF_CUDA_TRY(
+        cudaFuncSetAttribute((const void*)var->points, cudaFuncAttributePreferredSharedMemoryCarveout, k.carveout));
+    const int64_t tiles = div_up(num_points, simt::kGeo);
+    var->points<<<(unsigned)std::min<int64_t>(tiles, (int64_t)k.sms * k.per), simt::kThreads, smem,
+                  (cudaStream_t)stream>>>(p, simt::PointArgs{position, node_id, num_points, out});
+    ATDF_LAUNCH_CHECK();
+    return ATDF_OK;
+}
 
 int atdf_project_workspace_size(int64_t num_rays, int32_t max_depth, int32_t ns, int64_t num_slots,
                                 int32_t out_channels, size_t* bytes)

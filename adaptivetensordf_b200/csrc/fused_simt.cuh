@@ -166,10 +166,10 @@ __device__ __forceinline__ int64_t plane_base(const FusedParams& p, int64_t slot
 // (zeros for samples past the item's end and outside the region of interest).
 // stash (adjoint): the planes' bilinear values, for the line gradients of the
 // same thread's samples; gathering them a second time cost as much as the
-// features.
+// features. slots (points): each sample's slot, -1 for zero features.
 template <int C, int MODE, int H, int NH, bool STASH>
 __device__ __forceinline__ void gather_tile(const FusedParams& p, int64_t slot, bool real, const float* geo, int s0,
-                                            int left, float* x, float* stash)
+                                            int left, float* x, float* stash, const int* slots = nullptr)
 {
     using K = Cfg<C, MODE, H, NH>;
     constexpr int V = K::V;
@@ -182,6 +182,10 @@ __device__ __forceinline__ void gather_tile(const FusedParams& p, int64_t slot, 
         for (int v = 0; v < V; ++v)
 #pragma unroll
             for (int i = 0; i < (MODE ? 12 : 4); ++i) f[v][i] = 0.0f;
+        if (slots && s < left) {
+            slot = slots[s0 + s];
+            real = slot >= 0;
+        }
         if (real && s < left) {
             const SampleGeo g = load_geo(geo, s0 + s);
 #pragma unroll
@@ -282,6 +286,46 @@ __device__ __forceinline__ void layer0(const float* sm, int rg, int cg, uint64_t
     gemm_k<8, 4, K::F>(acc, sm + S::x + rg * K::XP, K::RG * K::XP, sm + S::w0 + cg * K::XP, K::CG * K::XP);
 }
 
+// The decoder's hidden layers and the last layer's partial sums (per column
+// group, into zp) of the tile whose features are in x.
+template <int C, int MODE, int H, int NH>
+__device__ __forceinline__ void decode_tile(float* sm, int rg, int cg, int cw, int s0, int hact, float beta)
+{
+    using K = Cfg<C, MODE, H, NH>;
+    using S = Smem<C, MODE, H, NH, false>;
+    const int tid = threadIdx.x;
+                    uint64_t acc[8][4];
+                    layer0<C, MODE, H, NH, false>(sm, rg, cg, acc);
+                    if (NH == 2) {
+    #pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            const float b = sm[S::b0 + cg + j * K::CG];
+    #pragma unroll
+                            for (int i = 0; i < 8; ++i)
+                                sm[S::h + (rg + i * K::RG) * K::HP + cg + j * K::CG] =
+                                    act_hidden(hact, sum2(acc[i][j]) + b, beta);
+                        }
+                        __syncthreads();
+                        zero2<8, 4>(acc);
+                        gemm_k<8, 4, H>(acc, sm + S::h + rg * K::HP, K::RG * K::HP, sm + S::w1 + cg * K::HP,
+                                        K::CG * K::HP);
+                    }
+                    // the last layer's sums over the thread's columns
+                    float z[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    #pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const int c = cg + j * K::CG;
+                        const float b = sm[(NH == 2 ? S::b1 : S::b0) + c], wl = sm[S::wl + c];
+    #pragma unroll
+                        for (int i = 0; i < 8; ++i) z[i] = fmaf(act_hidden(hact, sum2(acc[i][j]) + b, beta), wl, z[i]);
+                    }
+    #pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        z[i] = sum_cols(z[i]);
+                        if ((tid & 6) == 0) sm[S::zp + cw * S::zrow + s0 + rg + i * K::RG] = z[i];
+                    }
+}
+
 template <int C, int MODE, int H, int NH>
 __global__ void __launch_bounds__(kThreads, 3) forward_kernel(FusedParams p)
 {
@@ -310,36 +354,7 @@ __global__ void __launch_bounds__(kThreads, 3) forward_kernel(FusedParams p)
             for (int s0 = 0; s0 < kGeo && t0 + s0 < it.total; s0 += K::T) {
                 gather_tile<C, MODE, H, NH, false>(p, it.slot, real, geo, s0, it.total - t0 - s0, sm + S::x, nullptr);
                 __syncthreads();
-                uint64_t acc[8][4];
-                layer0<C, MODE, H, NH, false>(sm, rg, cg, acc);
-                if (NH == 2) {
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        const float b = sm[S::b0 + cg + j * K::CG];
-#pragma unroll
-                        for (int i = 0; i < 8; ++i)
-                            sm[S::h + (rg + i * K::RG) * K::HP + cg + j * K::CG] =
-                                act_hidden(hact, sum2(acc[i][j]) + b, beta);
-                    }
-                    __syncthreads();
-                    zero2<8, 4>(acc);
-                    gemm_k<8, 4, H>(acc, sm + S::h + rg * K::HP, K::RG * K::HP, sm + S::w1 + cg * K::HP,
-                                    K::CG * K::HP);
-                }
-                // the last layer's sums over the thread's columns
-                float z[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const int c = cg + j * K::CG;
-                    const float b = sm[(NH == 2 ? S::b1 : S::b0) + c], wl = sm[S::wl + c];
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) z[i] = fmaf(act_hidden(hact, sum2(acc[i][j]) + b, beta), wl, z[i]);
-                }
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    z[i] = sum_cols(z[i]);
-                    if ((tid & 6) == 0) sm[S::zp + cw * S::zrow + s0 + rg + i * K::RG] = z[i];
-                }
+                decode_tile<C, MODE, H, NH>(sm, rg, cg, cw, s0, hact, beta);
             }
             __syncthreads();
             {
@@ -616,6 +631,67 @@ __global__ void __launch_bounds__(kThreads, NH == 1 ? 3 : 2) backward_kernel(Fus
         }
     for (int off = 16; off > 0; off >>= 1) gbl += __shfl_down_sync(0xffffffffu, gbl, off);
     if (lane == 0) atomicAdd(p.ws.last_sum, gbl);
+}
+
+// Density at points with known leaves (field and decoder in one pass, no
+// gradients): the forward's tiles with the geometry of points instead of the
+// samples of segments. Bound by the decoder like the forward.
+struct PointArgs {
+    const float* pos;     // [S, 3]
+    const int64_t* node;  // [S]
+    int64_t S;
+    float* out;  // [S]
+};
+
+template <int C, int MODE, int H, int NH>
+__global__ void __launch_bounds__(kThreads, 3) points_kernel(FusedParams p, PointArgs a)
+{
+    using K = Cfg<C, MODE, H, NH>;
+    using S = Smem<C, MODE, H, NH, false>;
+    extern __shared__ __align__(16) float sm[];
+    const int tid = threadIdx.x;
+    int rg, cg, cw;
+    tile_place<K>(rg, cg, cw);
+    load_weights<C, MODE, H, NH, false>(p, sm);
+    float* geo = sm + S::geo;
+    int* slots = reinterpret_cast<int*>(sm + S::si);
+    const float beta = p.mlp.softplus_beta;
+    const int hact = p.mlp.hidden_activation, lact = p.mlp.last_activation;
+    for (int64_t t0 = (int64_t)blockIdx.x * kGeo; t0 < a.S; t0 += (int64_t)gridDim.x * kGeo) {
+        const int left = (int)min((int64_t)kGeo, a.S - t0);
+        __syncthreads();
+        int slot = -1;
+        if (tid < left) {
+            const int64_t i = t0 + tid, nd = a.node[i];
+            if (nd < 0 || nd >= p.tree.num_nodes) {
+                set_err(p.err, ATDF_DEVERR_INDEX);
+            } else {
+                const int64_t s = p.field.leaf_slot[nd];
+                if (s >= p.field.num_slots) set_err(p.err, ATDF_DEVERR_INDEX);
+                if (s >= 0 && s < p.field.num_slots) {
+                    slot = (int)s;
+                    const float pos[3] = {a.pos[3 * i], a.pos[3 * i + 1], a.pos[3 * i + 2]};
+                    store_geo(geo, tid, sample_geo(pos, p.tree.node_position_min + 3 * nd,
+                                                   p.tree.node_position_max + 3 * nd, p.field.roi_min,
+                                                   p.field.roi_max), 0.0f);
+                }
+            }
+        }
+        slots[tid] = slot;
+        __syncthreads();
+        for (int s0 = 0; s0 < left; s0 += K::T) {
+            gather_tile<C, MODE, H, NH, false>(p, 0, false, geo, s0, left - s0, sm + S::x, nullptr, slots);
+            __syncthreads();
+            decode_tile<C, MODE, H, NH>(sm, rg, cg, cw, s0, hact, beta);
+        }
+        __syncthreads();
+        if (tid < left) {
+            float z = sm[S::bl];
+#pragma unroll
+            for (int w = 0; w < K::CW; ++w) z += sm[S::zp + w * S::zrow + tid];
+            a.out[t0 + tid] = act_fwd(lact, z, beta);
+        }
+    }
 }
 
 }  // namespace simt

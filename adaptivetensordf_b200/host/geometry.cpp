@@ -662,9 +662,53 @@ Tensor GeometryTensorQO::SampleVolumeIndirect_feature(HyperTreeBase& tree, Tenso
                               L[2], reinterpret_cast<int64_t>(this), reinterpret_cast<int64_t>(&tree));
 }
 
+// SampleVolumeIndirect through atdf_field_density; undefined where that kernel
+// does not take the decoder or the layout.
+static Tensor density_no_grad(GeometryTensorQO& geo, HyperTreeBase& tree, const Tensor& global_coordinate,
+                              const Tensor& node_id)
+{
+    torch::NoGradGuard ng;
+    ATDF_CHECK_CUDA(global_coordinate);
+    std::vector<Tensor> P, L;
+    for (int m = 0; m < 3; ++m) {
+        P.push_back(channels_last(geo.planes[m]));
+        L.push_back(channels_last(geo.lines[m]));
+    }
+    auto f = field_view(geo, P, L);
+    auto dims = layer_dims(geo.decoder);
+    if (dims.back() != 1) return Tensor();
+    auto flat = flat_params(decoder_inputs(geo.decoder), geo.decoder.weight.size());
+    ATDF_CHECK_CUDA(flat);
+    auto m = mlp_view(dims, flat.data_ptr<float>(), activation_id(geo.decoder.activation),
+                      activation_id(geo.decoder.last_activation), (float)geo.decoder.softplus_beta);
+    auto pc = global_coordinate.reshape({-1, 3}).contiguous();
+    auto nc = node_id.reshape({-1}).to(torch::kLong).contiguous();
+    auto out = torch::empty({nc.size(0), 1}, pc.options());
+    auto err = err_word(pc.device());
+    const int st = atdf_field_density(&f, &m, tree.node_position_min.data_ptr<float>(),
+                                      tree.node_position_max.data_ptr<float>(), tree.NumNodes(), pc.data_ptr<float>(),
+                                      nc.data_ptr<int64_t>(), nc.size(0), out.data_ptr<float>(),
+                                      err.data_ptr<int32_t>(), stream_arg());
+    if (st == ATDF_ERR_UNSUPPORTED) return Tensor();
+    check_status(st, "SampleVolumeIndirect");
+    check_dev_error(err, "SampleVolumeIndirect_feature");
+    return out;
+}
+
 Tensor GeometryTensorQO::SampleVolumeIndirect(HyperTreeBase& tree, Tensor global_coordinate, Tensor node_id)
 {
     if (global_coordinate.numel() == 0) return global_coordinate;
+    // without gradients (evaluation) one kernel does both, where it takes the shapes
+    bool grad = false;
+    if (torch::GradMode::is_enabled()) {
+        grad = global_coordinate.requires_grad();
+        for (const auto* v : {&planes, &lines, &decoder.weight, &decoder.bias})
+            for (const auto& t : *v) grad = grad || t.requires_grad();
+    }
+    if (!grad) {
+        Tensor out = density_no_grad(*this, tree, global_coordinate, node_id);
+        if (out.defined()) return out;
+    }
     auto feat = SampleVolumeIndirect_feature(tree, global_coordinate, node_id);
     return DecodeFeatures(decoder, feat).contiguous();
 }

@@ -171,3 +171,30 @@ def test_node_error_segment_lengths(oracle, M, seed):
     ls_o, ws_o = oracle.accumulate_loss_per_node(so, (img.cpu().numpy() - y) ** 2, len(td["node_depth"]))
     assert rel_err(ws.cpu().numpy(), ws_o) < 1e-12
     assert rel_err(ls.cpu().numpy(), ls_o) < 1e-9
+
+
+@pytest.mark.parametrize("C,hidden,op", [(8, [32], "add"), (16, [64, 64], "add"), (8, [64, 64], "cat"), (16, [64], "add"),
+                                         (24, [64, 64], "add")])
+@pytest.mark.parametrize("n", [1, 127, 128, 129, 3000])
+def test_density_without_gradients(oracle, C, hidden, op, n):
+    """The one-kernel density (no gradients wanted) against the FP64 oracle:
+    points counts around its tiles, leaves outside the ROI, a decoder it does
+    not take (24 channels), and a node id out of range."""
+    tree, geo, _, _ = gpu_scene(2, C, 9, (32, 9, 32), hidden, 1, seed=n, tensor_op=op)
+    slot = geo.leaf_slot.clone()
+    slot[tree.active_node_ids[::5]] = -1
+    geo.leaf_slot = slot
+    td, fd, md = oracle_views(tree, geo)
+    pts = np.random.default_rng(n).uniform(-1, 1, (n, 3)).astype(np.float32)
+    node, _ = tree.NodeIdForPositionGPU(torch.from_numpy(pts).cuda())
+    with torch.no_grad():
+        got = geo.SampleVolumeIndirect(tree, torch.from_numpy(pts).cuda(), node)
+    assert got.shape == (n, 1) and not got.requires_grad
+    # each point as one sample of weight 1 on a ray of its own
+    so = {"global_coordinate": pts, "node_id": node.cpu().numpy(), "weight": np.ones(n, np.float32),
+          "ray_index": np.arange(n)}
+    ref = oracle.project_forward(fd, md, td, so, n, np.float64).reshape(n, 1)
+    assert rel_err(got.cpu().numpy(), ref) < REL_TOL
+    node[0] = tree.NumNodes()
+    with torch.no_grad(), pytest.raises(RuntimeError, match="index out of range"):
+        geo.SampleVolumeIndirect(tree, torch.from_numpy(pts).cuda(), node)
