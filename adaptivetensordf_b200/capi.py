@@ -152,6 +152,8 @@ def _declare(L):
         "atdf_grid_sample2d_forward": (I32, [P, I64, I64, I64, I64, P, P, P, I64, P, P, P]),
         "atdf_grid_sample2d_backward": (I32, [P, I64, I64, I64, I64, P, P, P, I64, P, P, P, P, P]),
         "atdf_grid_sample2d_backward_channels_last": (I32, [P, I64, I64, I64, I64, P, P, I64, P, P, P, P, P]),
+        "atdf_grid_layout": (I32, [P, I64, I64, I64, I32, P, P]),
+        "atdf_grid_sample1d_backward_copies": (I32, [P, I64, I64, I64, P, P, P, I64, P, P, P, P, I32, P, P]),
         "atdf_grid_sample1d_forward": (I32, [P, I64, I64, I64, P, P, P, I64, P, P, P]),
         "atdf_grid_sample1d_backward": (I32, [P, I64, I64, I64, P, P, P, I64, P, P, P, P, P]),
         "atdf_gradient_correction_backward": (I32, [P, P, I64, P, I64, P, P, P]),

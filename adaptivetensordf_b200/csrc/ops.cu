@@ -83,19 +83,19 @@ __global__ void gs2_fwd_kernel(const float* __restrict__ grid, int64_t N, int64_
     }
 }
 
-// One channel's terms of the coordinate gradient, one rounding per operation
-// (IndirectGridSample2D.cu:354-367).
-__device__ __forceinline__ void coord_grad2(float vnw, float vne, float vsw, float vse, float ax0, float ax1, float ay0,
-                                            float ay1, float go, float& gix, float& giy)
+// One channel's four terms each of the coordinate gradient's x and y chains, one
+// rounding per operation (IndirectGridSample2D.cu:354-367).
+__device__ __forceinline__ void coord_terms2(float vnw, float vne, float vsw, float vse, float ax0, float ax1, float ay0,
+                                             float ay1, float go, float* tx, float* ty)
 {
-    gix = __fadd_rn(gix, __fmul_rn(__fmul_rn(__fmul_rn(-1.0f, vnw), ay1), go));
-    gix = __fadd_rn(gix, __fmul_rn(__fmul_rn(vne, ay1), go));
-    gix = __fadd_rn(gix, __fmul_rn(__fmul_rn(__fmul_rn(-1.0f, vsw), ay0), go));
-    gix = __fadd_rn(gix, __fmul_rn(__fmul_rn(vse, ay0), go));
-    giy = __fadd_rn(giy, __fmul_rn(__fmul_rn(__fmul_rn(-1.0f, vnw), ax1), go));
-    giy = __fadd_rn(giy, __fmul_rn(__fmul_rn(__fmul_rn(-1.0f, vne), ax0), go));
-    giy = __fadd_rn(giy, __fmul_rn(__fmul_rn(vsw, ax1), go));
-    giy = __fadd_rn(giy, __fmul_rn(__fmul_rn(vse, ax0), go));
+    tx[0] = __fmul_rn(__fmul_rn(__fmul_rn(-1.0f, vnw), ay1), go);
+    tx[1] = __fmul_rn(__fmul_rn(vne, ay1), go);
+    tx[2] = __fmul_rn(__fmul_rn(__fmul_rn(-1.0f, vsw), ay0), go);
+    tx[3] = __fmul_rn(__fmul_rn(vse, ay0), go);
+    ty[0] = __fmul_rn(__fmul_rn(__fmul_rn(-1.0f, vnw), ax1), go);
+    ty[1] = __fmul_rn(__fmul_rn(__fmul_rn(-1.0f, vne), ax0), go);
+    ty[2] = __fmul_rn(__fmul_rn(vsw, ax1), go);
+    ty[3] = __fmul_rn(__fmul_rn(vse, ax0), go);
 }
 
 __global__ void gs2_bwd_kernel(const float* __restrict__ grid, int64_t N, int64_t C, int H, int W, int64_t sN,
@@ -128,7 +128,12 @@ __global__ void gs2_bwd_kernel(const float* __restrict__ grid, int64_t N, int64_
         }
         const float vnw = gc[k.y0 * sH + k.x0 * sW], vne = gc[k.y0 * sH + k.x1 * sW];
         const float vsw = gc[k.y1 * sH + k.x0 * sW], vse = gc[k.y1 * sH + k.x1 * sW];
-        coord_grad2(vnw, vne, vsw, vse, ax0, ax1, ay0, ay1, go, gix, giy);
+        float tx[4], ty[4];
+        coord_terms2(vnw, vne, vsw, vse, ax0, ax1, ay0, ay1, go, tx, ty);
+        for (int j = 0; j < 4; ++j) {
+            gix = __fadd_rn(gix, tx[j]);
+            giy = __fadd_rn(giy, ty[j]);
+        }
     }
     if (guv) {
         guv[2 * i] = __fadd_rn(guv[2 * i], __fdiv_rn(__fmul_rn(gix, (float)(W - 1)), 2.0f));
@@ -163,42 +168,110 @@ __global__ void __launch_bounds__(256)
     store_vec<4>(out + e * 4, r);
 }
 
-// Adjoint into a channels-last gradient by 16-byte reductions. A thread per
-// sample: the coordinate gradient is one chain of roundings over the channels
-// in order (IndirectGridSample2D.cu:354-367).
+// Adjoint into a channels-last gradient by 16-byte reductions. Q threads per
+// sample (a power of two, 4 CQ channels each; Q = 1 for the channel counts
+// that do not split so). The coordinate gradient is one chain of roundings over
+// the channels in order (IndirectGridSample2D.cu:354-367): every thread forms
+// the terms of its channels, then the chain passes from thread to thread.
+template <int Q>
 __global__ void __launch_bounds__(256)
     gs2_bwd_cl_kernel(const float* __restrict__ grid, int64_t N, int C, int H, int W,
                       const int64_t* __restrict__ index, const float* __restrict__ uv, int64_t S,
                       const float* __restrict__ gout, float* __restrict__ ggrid, float* __restrict__ guv, int32_t* err)
 {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= S) return;
-    const int64_t n = index[i];
-    if (n < 0 || n >= N) {
-        set_err(err, ATDF_DEVERR_INDEX);
-        return;
-    }
-    const Corner2 k = corners2(uv[2 * i], uv[2 * i + 1], H, W);
-    const int64_t base = n * (int64_t)H * W * C;
+    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t i = e / Q;
+    const int q = (int)(e % Q);
+    const int64_t n = i < S ? index[i] : -1;
+    const bool ok = n >= 0 && n < N;
+    if (i < S && !ok) set_err(err, ATDF_DEVERR_INDEX);
+    const Corner2 k = corners2(ok ? uv[2 * i] : 0.0f, ok ? uv[2 * i + 1] : 0.0f, H, W);
+    const int64_t base = (ok ? n : 0) * (int64_t)H * W * C;
     const int64_t o[4] = {base + (int64_t)(k.y0 * W + k.x0) * C, base + (int64_t)(k.y0 * W + k.x1) * C,
                           base + (int64_t)(k.y1 * W + k.x0) * C, base + (int64_t)(k.y1 * W + k.x1) * C};
     float gix = 0.0f, giy = 0.0f;
     const float ay1 = __fsub_rn(k.fy1, k.iy), ay0 = __fsub_rn(k.iy, k.fy0);
     const float ax1 = __fsub_rn(k.fx1, k.ix), ax0 = __fsub_rn(k.ix, k.fx0);
-    for (int c = 0; c < C; c += 4) {
-        const Vec<4> go = load_vec<4>(gout + i * C + c);
-        add_vec<4>(ggrid + o[0] + c, k.w_nw, go);
-        add_vec<4>(ggrid + o[1] + c, k.w_ne, go);
-        add_vec<4>(ggrid + o[2] + c, k.w_sw, go);
-        add_vec<4>(ggrid + o[3] + c, k.w_se, go);
-        const Vec<4> nw = load_vec<4>(grid + o[0] + c), ne = load_vec<4>(grid + o[1] + c),
-                     sw = load_vec<4>(grid + o[2] + c), se = load_vec<4>(grid + o[3] + c);
+    // the Q threads take neighbouring groups of 4 channels, round by round
+    for (int c0 = 0; c0 < C; c0 += 4 * Q) {
+        const int c = c0 + 4 * q;
+        float tx[16], ty[16];
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-            coord_grad2(nw.v[j], ne.v[j], sw.v[j], se.v[j], ax0, ax1, ay0, ay1, go.v[j], gix, giy);
+        for (int j = 0; j < 16; ++j) tx[j] = ty[j] = 0.0f;
+        if (ok) {
+            const Vec<4> go = load_vec<4>(gout + i * C + c);
+            add_vec<4>(ggrid + o[0] + c, k.w_nw, go);
+            add_vec<4>(ggrid + o[1] + c, k.w_ne, go);
+            add_vec<4>(ggrid + o[2] + c, k.w_sw, go);
+            add_vec<4>(ggrid + o[3] + c, k.w_se, go);
+            const Vec<4> nw = load_vec<4>(grid + o[0] + c), ne = load_vec<4>(grid + o[1] + c),
+                         sw = load_vec<4>(grid + o[2] + c), se = load_vec<4>(grid + o[3] + c);
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                coord_terms2(nw.v[j], ne.v[j], sw.v[j], se.v[j], ax0, ax1, ay0, ay1, go.v[j], tx + 4 * j, ty + 4 * j);
+        }
+#pragma unroll
+        for (int r = 0; r < Q; ++r) {
+            float sx = gix, sy = giy;
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+                sx = __fadd_rn(sx, tx[j]);
+                sy = __fadd_rn(sy, ty[j]);
+            }
+            gix = Q == 1 ? sx : __shfl_sync(0xffffffffu, sx, r, Q);
+            giy = Q == 1 ? sy : __shfl_sync(0xffffffffu, sy, r, Q);
+        }
     }
+    if (!ok || q != 0) return;
     guv[2 * i] = __fadd_rn(guv[2 * i], __fdiv_rn(__fmul_rn(gix, (float)(W - 1)), 2.0f));
     guv[2 * i + 1] = __fadd_rn(guv[2 * i + 1], __fdiv_rn(__fmul_rn(giy, (float)(H - 1)), 2.0f));
+}
+
+// [N][C][HW] to [N][HW][C] or back, a block per 128 texels of one n: whole rows
+// of either layout through shared memory.
+constexpr int kLayoutTexels = 128;
+
+__global__ void __launch_bounds__(256)
+    grid_layout_kernel(const float* __restrict__ src, int C, int HW, bool to_cl, float* __restrict__ dst)
+{
+    extern __shared__ float s_tile[];  // [C][kLayoutTexels + 1]
+    const int chunks = (HW + kLayoutTexels - 1) / kLayoutTexels;
+    const int64_t base = (int64_t)(blockIdx.x / chunks) * C * HW;
+    const int x0 = (int)(blockIdx.x % chunks) * kLayoutTexels, nx = min(kLayoutTexels, HW - x0);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    // channel rows by warps, texel rows as one run of nx * C values (c and x of
+    // a thread's next value without a division)
+    const int dc = blockDim.x % C, dx = blockDim.x / C;
+    auto rows = [&](auto move) {
+        for (int c = warp; c < C; c += warps)
+#pragma unroll
+            for (int x = lane; x < kLayoutTexels; x += 32)
+                if (x < nx) move(c, x, base + (int64_t)c * HW + x0 + x);
+    };
+    auto texels = [&](auto move) {
+        int c = threadIdx.x % C, x = threadIdx.x / C;
+#pragma unroll 4
+        for (int e = threadIdx.x; e < C * nx; e += blockDim.x) {
+            move(c, x, base + (int64_t)x0 * C + e);
+            c += dc;
+            x += dx;
+            if (c >= C) {
+                c -= C;
+                ++x;
+            }
+        }
+    };
+    auto in = [&](int c, int x, int64_t at) { s_tile[c * (kLayoutTexels + 1) + x] = __ldg(src + at); };
+    auto out = [&](int c, int x, int64_t at) { dst[at] = s_tile[c * (kLayoutTexels + 1) + x]; };
+    if (to_cl)
+        rows(in);
+    else
+        texels(in);
+    __syncthreads();
+    if (to_cl)
+        texels(out);
+    else
+        rows(out);
 }
 
 // V channels at a time: 16-byte stores when the channel count allows (V = 4).
@@ -267,6 +340,56 @@ __global__ void __launch_bounds__(256)
         const float v = s_sum[j];
         if (v != 0.0f) atomicAdd(&ggrid[j], v);
     }
+}
+
+// The 1D adjoint with 16-byte reductions into one of `copies` channels-last
+// copies of the gradient ([copy][n][W][C], zeroed): a few hundred entries take
+// every sample, so one copy would serialise them, and shared-memory float adds
+// (a compare-and-swap loop) took 146 us for 1 M samples of 16 channels.
+__global__ void __launch_bounds__(256)
+    gs1_bwd_copies_kernel(const float* __restrict__ grid, int64_t N, int C, int W, int64_t sN, int64_t sC, int64_t sW,
+                          const int64_t* __restrict__ index, const float* __restrict__ uv, int64_t S,
+                          const float* __restrict__ gout, float* __restrict__ rep, int copies,
+                          float* __restrict__ guv, int32_t* err)
+{
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= S) return;
+    const int64_t n = index[i];
+    if (n < 0 || n >= N) {
+        set_err(err, ATDF_DEVERR_INDEX);
+        return;
+    }
+    const Corner1 k = corners1(uv[i], W);
+    const float* g = grid + n * sN;
+    float* r0 = rep + (((int64_t)(blockIdx.x % copies) * N + n) * W + k.x0) * C;
+    float* r1 = rep + (((int64_t)(blockIdx.x % copies) * N + n) * W + k.x1) * C;
+    float gix = 0.0f;
+    const float a1 = __fsub_rn(k.fx1, k.ix), a0 = __fsub_rn(k.ix, k.fx0);
+    for (int c = 0; c < C; c += 4) {
+        const Vec<4> go = load_vec<4>(gout + i * C + c);
+        add_vec<4>(r0 + c, k.w0, go);
+        add_vec<4>(r1 + c, k.w1, go);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float v0 = g[(c + j) * sC + k.x0 * sW], v1 = g[(c + j) * sC + k.x1 * sW];
+            gix = __fadd_rn(gix, __fmul_rn(__fmul_rn(__fmul_rn(-1.0f, v0), a1), go.v[j]));
+            gix = __fadd_rn(gix, __fmul_rn(__fmul_rn(v1, a0), go.v[j]));
+        }
+    }
+    guv[i] = __fadd_rn(guv[i], __fdiv_rn(__fmul_rn(gix, (float)(W - 1)), 2.0f));
+}
+
+// ggrid [N][C][W] += the sum of the copies (in FP64, one rounding).
+__global__ void gs1_sum_copies_kernel(const float* __restrict__ rep, int copies, int64_t N, int C, int W,
+                                      float* __restrict__ ggrid)
+{
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, total = N * C * W;
+    if (i >= total) return;
+    double acc = 0.0;
+    for (int r = 0; r < copies; ++r) acc += (double)rep[r * total + i];
+    const int64_t n = i / ((int64_t)W * C);
+    const int x = (int)(i / C % W), c = (int)(i % C);
+    ggrid[(n * C + c) * W + x] += (float)acc;
 }
 
 __global__ void gradcorr_bwd_kernel(const float* __restrict__ dir, const int64_t* __restrict__ ray, int64_t R,
@@ -610,8 +733,24 @@ int atdf_grid_sample2d_backward_channels_last(const float* grid, int64_t N, int6
                         reinterpret_cast<uintptr_t>(grad_out)) & 15) != 0)
         return ATDF_ERR_UNSUPPORTED;
     if (S == 0) return ATDF_OK;
-    gs2_bwd_cl_kernel<<<blocks_for(S), 256, 0, (cudaStream_t)stream>>>(grid, N, (int)C, (int)H, (int)W, index, uv, S,
-                                                                       grad_out, grad_grid, grad_uv, dev_error);
+    const int q = C % 32 == 0 ? 8 : C % 16 == 0 ? 4 : C % 8 == 0 ? 2 : 1;
+    auto kernel = q == 8 ? gs2_bwd_cl_kernel<8> : q == 4 ? gs2_bwd_cl_kernel<4> : q == 2 ? gs2_bwd_cl_kernel<2>
+                                                                                     : gs2_bwd_cl_kernel<1>;
+    kernel<<<blocks_for(S * q), 256, 0, (cudaStream_t)stream>>>(grid, N, (int)C, (int)H, (int)W, index, uv, S, grad_out,
+                                                                grad_grid, grad_uv, dev_error);
+    ATDF_LAUNCH_CHECK();
+    return ATDF_OK;
+}
+
+int atdf_grid_layout(const float* src, int64_t N, int64_t C, int64_t HW, int32_t to_channels_last, float* dst,
+                     atdf_stream_t stream)
+{
+    if (N < 0 || C <= 0 || HW <= 0 || (N > 0 && (!src || !dst))) return ATDF_ERR_INVALID_ARGUMENT;
+    const int64_t smem = C * (kLayoutTexels + 1) * 4, blocks = N * div_up(HW, kLayoutTexels);
+    if (smem > 48 * 1024 || blocks > INT32_MAX || C * HW > INT32_MAX) return ATDF_ERR_UNSUPPORTED;
+    if (N == 0) return ATDF_OK;
+    grid_layout_kernel<<<(unsigned)blocks, 256, smem, (cudaStream_t)stream>>>(src, (int)C, (int)HW,
+                                                                             to_channels_last != 0, dst);
     ATDF_LAUNCH_CHECK();
     return ATDF_OK;
 }
@@ -652,6 +791,28 @@ int atdf_grid_sample1d_backward(const float* grid, int64_t N, int64_t C, int64_t
     }
     gs1_bwd_kernel<<<blocks, 256, smem_sum ? (size_t)(N * C * W * 4) : 0, (cudaStream_t)stream>>>(
         grid, N, C, (int)W, s[0], s[1], s[2], index, uv, S, grad_out, grad_grid, grad_uv, smem_sum, dev_error);
+    ATDF_LAUNCH_CHECK();
+    return ATDF_OK;
+}
+
+int atdf_grid_sample1d_backward_copies(const float* grid, int64_t N, int64_t C, int64_t W, const int64_t* s,
+                                       const int64_t* index, const float* uv, int64_t S, const float* grad_out,
+                                       float* grad_grid, float* grad_uv, float* scratch, int32_t copies,
+                                       int32_t* dev_error, atdf_stream_t stream)
+{
+    if (!grid || !s || !grad_grid || !grad_uv || !scratch || copies <= 0 || N <= 0 || C <= 0 || W <= 0 || S < 0 ||
+        (S > 0 && (!index || !uv || !grad_out)))
+        return ATDF_ERR_INVALID_ARGUMENT;
+    if (C % 4 != 0 || C > INT32_MAX / 4 || W > INT32_MAX || N * C * W > INT32_MAX ||
+        ((reinterpret_cast<uintptr_t>(grad_out) | reinterpret_cast<uintptr_t>(scratch)) & 15) != 0)
+        return ATDF_ERR_UNSUPPORTED;
+    if (S == 0) return ATDF_OK;
+    const cudaStream_t st = (cudaStream_t)stream;
+    ATDF_CUDA_TRY(cudaMemsetAsync(scratch, 0, (size_t)copies * N * C * W * 4, st));
+    gs1_bwd_copies_kernel<<<blocks_for(S), 256, 0, st>>>(grid, N, (int)C, (int)W, s[0], s[1], s[2], index, uv, S,
+                                                         grad_out, scratch, copies, grad_uv, dev_error);
+    ATDF_LAUNCH_CHECK();
+    gs1_sum_copies_kernel<<<blocks_for(N * C * W), 256, 0, st>>>(scratch, copies, N, (int)C, (int)W, grad_grid);
     ATDF_LAUNCH_CHECK();
     return ATDF_OK;
 }

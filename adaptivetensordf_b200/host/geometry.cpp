@@ -49,9 +49,9 @@ int activation_id(const std::string& a)
 // 16-byte accesses. Grids of another layout are copied for them when there are
 // enough samples to pay for it: a copy moves every texel once each way, a
 // sample gathers four texels whose channels lie in separate sectors otherwise
-// (1 M samples on 1.2 M texels of 16 channels: forward 252 -> 75 us, adjoint
-// 771 -> 175 us with the copies; below one sample per 4 texels the copy costs
-// more than it saves).
+// (1 M samples on 1.2 M texels of 16 channels: forward 252 -> 85 us, adjoint
+// 771 -> 207 us with the copies of 40 us each; below one sample per 4 texels
+// the copies cost more than they save).
 static bool samples_in_channels_last(const Tensor& grid, int64_t samples)
 {
     const int64_t texels = grid.size(0) * grid.size(2) * grid.size(3);
@@ -71,7 +71,23 @@ static Tensor channels_last_copy(const Tensor& grid)
     const bool dense = grid.stride(1) == 1 && grid.stride(3) == C && grid.stride(2) == C * W &&
                        grid.stride(0) == C * W * H;
     if (dense) return aligned16(grid);
+    if (grid.is_contiguous()) {
+        auto out = torch::empty({grid.size(0), H, W, C}, grid.options());
+        if (atdf_grid_layout(grid.data_ptr<float>(), grid.size(0), C, H * W, 1, out.data_ptr<float>(), stream_arg()) ==
+            ATDF_OK)
+            return out.permute({0, 3, 1, 2});
+    }
     return grid.permute({0, 2, 3, 1}).contiguous().permute({0, 3, 1, 2});
+}
+
+// A gradient in dense NHWC storage as contiguous [N, C, H, W].
+static Tensor contiguous_from_channels_last(const Tensor& t)
+{
+    auto out = torch::empty(t.sizes(), t.options().memory_format(torch::MemoryFormat::Contiguous));
+    if (atdf_grid_layout(t.data_ptr<float>(), t.size(0), t.size(1), t.size(2) * t.size(3), 0, out.data_ptr<float>(),
+                         stream_arg()) == ATDF_OK)
+        return out;
+    return t.contiguous();
 }
 
 class GridSample2DFn : public torch::autograd::Function<GridSample2DFn> {
@@ -120,7 +136,7 @@ class GridSample2DFn : public torch::autograd::Function<GridSample2DFn> {
                              ggrid.data_ptr<float>(), guv.data_ptr<float>(), err.data_ptr<int32_t>(), stream_arg()),
                          "IndirectGridSample2D backward");
             check_dev_error(err, "IndirectGridSample2D backward");
-            return {ggrid.contiguous(), Tensor(), guv};
+            return {contiguous_from_channels_last(ggrid), Tensor(), guv};
         }
         auto ggrid = torch::zeros(grid.sizes(), grid.options().memory_format(torch::MemoryFormat::Contiguous));
         int64_t st[4] = {grid.stride(0), grid.stride(1), grid.stride(2), grid.stride(3)};
@@ -168,11 +184,26 @@ class GridSample1DFn : public torch::autograd::Function<GridSample1DFn> {
         auto guv = torch::zeros_like(u);
         int64_t st[3] = {grid.stride(0), grid.stride(1), grid.stride(2)};
         auto err = ctx->saved_data["err"].toTensor();
-        check_status(atdf_grid_sample1d_backward(grid.data_ptr<float>(), grid.size(0), grid.size(1), grid.size(2), st,
-                                                 idx.data_ptr<int64_t>(), u.data_ptr<float>(), idx.size(0),
-                                                 g.data_ptr<float>(), ggrid.data_ptr<float>(), guv.data_ptr<float>(),
-                                                 err.data_ptr<int32_t>(), stream_arg()),
-                     "IndirectGridSample1D backward");
+        // many samples on few entries: up to 64 copies of the gradient (8 MB at most) share the adds
+        const int64_t S = idx.size(0), entries = grid.size(0) * grid.size(2);
+        const int64_t copies = std::min<int64_t>({64, S / std::max<int64_t>(8 * entries, 1),
+                                                  (2 << 20) / std::max<int64_t>(grid.numel(), 1)});
+        int st1 = ATDF_ERR_UNSUPPORTED;
+        if (copies >= 2) {
+            g = aligned16(g);
+            auto scratch = torch::empty({copies * grid.numel()}, grid.options().memory_format(torch::MemoryFormat::Contiguous));
+            st1 = atdf_grid_sample1d_backward_copies(grid.data_ptr<float>(), grid.size(0), grid.size(1), grid.size(2),
+                                                     st, idx.data_ptr<int64_t>(), u.data_ptr<float>(), S,
+                                                     g.data_ptr<float>(), ggrid.data_ptr<float>(),
+                                                     guv.data_ptr<float>(), scratch.data_ptr<float>(), (int32_t)copies,
+                                                     err.data_ptr<int32_t>(), stream_arg());
+        }
+        if (st1 == ATDF_ERR_UNSUPPORTED)
+            st1 = atdf_grid_sample1d_backward(grid.data_ptr<float>(), grid.size(0), grid.size(1), grid.size(2), st,
+                                              idx.data_ptr<int64_t>(), u.data_ptr<float>(), S, g.data_ptr<float>(),
+                                              ggrid.data_ptr<float>(), guv.data_ptr<float>(), err.data_ptr<int32_t>(),
+                                              stream_arg());
+        check_status(st1, "IndirectGridSample1D backward");
         check_dev_error(err, "IndirectGridSample1D backward");
         return {ggrid, Tensor(), guv};
     }

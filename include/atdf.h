@@ -211,12 +211,23 @@ int atdf_grid_sample2d_backward_channels_last(const float* grid, int64_t N, int6
                                               const int64_t* index, const float* uv, int64_t num_samples,
                                               const float* grad_out, float* grad_grid, float* grad_uv,
                                               int32_t* dev_error, atdf_stream_t stream);
+/* Dense [N][C][HW] to channels-last [N][HW][C], or back (C up to 95, else
+ * ATDF_ERR_UNSUPPORTED). */
+int atdf_grid_layout(const float* src, int64_t N, int64_t C, int64_t HW, int32_t to_channels_last, float* dst,
+                     atdf_stream_t stream);
 int atdf_grid_sample1d_forward(const float* grid, int64_t N, int64_t C, int64_t W, const int64_t* grid_stride,
                                const int64_t* index, const float* uv, int64_t num_samples, float* out,
                                int32_t* dev_error, atdf_stream_t stream);
 int atdf_grid_sample1d_backward(const float* grid, int64_t N, int64_t C, int64_t W, const int64_t* grid_stride,
                                 const int64_t* index, const float* uv, int64_t num_samples, const float* grad_out,
                                 float* grad_grid, float* grad_uv, int32_t* dev_error, atdf_stream_t stream);
+/* The 1D adjoint through `copies` channels-last copies of the gradient in
+ * scratch (copies * N * C * W floats; scratch and grad_out 16-byte aligned, C a
+ * multiple of 4, else ATDF_ERR_UNSUPPORTED): for many samples on few entries. */
+int atdf_grid_sample1d_backward_copies(const float* grid, int64_t N, int64_t C, int64_t W, const int64_t* grid_stride,
+                                       const int64_t* index, const float* uv, int64_t num_samples,
+                                       const float* grad_out, float* grad_grid, float* grad_uv, float* scratch,
+                                       int32_t copies, int32_t* dev_error, atdf_stream_t stream);
 
 /* GradientCorrection backward (GradientCorrection.cu:22-48): g - (g.d) d. */
 int atdf_gradient_correction_backward(const float* ray_direction, const int64_t* ray_index, int64_t num_rays,
