@@ -48,25 +48,38 @@ static int launch_ray_segments_ws(const atdf_tree_t& tree, const float* origin, 
 // segment partials, idle until the forward). A segment whose node id or plane
 // slot is out of range sets the index bit and joins the out-of-ROI bucket
 // (zero features, no gradient).
-__global__ void bucket_count_kernel(Ws w, atdf_field_t f, int64_t num_nodes, int32_t* err)
+__device__ __forceinline__ void count_segments(const Ws& w, const atdf_field_t& f, int64_t num_nodes, int32_t* err,
+                                               int64_t first, int64_t step)
 {
     const int64_t nseg = min(w.totals[0], w.cap);
     int32_t* rank = reinterpret_cast<int32_t*>(w.seg_partial);
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nseg; i += (int64_t)gridDim.x * blockDim.x) {
+    for (int64_t i = first; i < nseg; i += step) {
         const int32_t nd = w.node[i];
         if (nd < 0 || nd >= num_nodes || f.leaf_slot[nd] >= f.num_slots) set_err(err, ATDF_DEVERR_INDEX);
         rank[i] = atomicAdd(&w.slot_offset[seg_slot(f, num_nodes, nd)], 1);
     }
 }
 
-__global__ void bucket_scatter_kernel(Ws w, atdf_field_t f, int64_t num_nodes)
+__device__ __forceinline__ void scatter_segments(const Ws& w, const atdf_field_t& f, int64_t num_nodes, int64_t first,
+                                                 int64_t step)
 {
     const int64_t nseg = min(w.totals[0], w.cap);
     const int32_t* rank = reinterpret_cast<const int32_t*>(w.seg_partial);
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nseg; i += (int64_t)gridDim.x * blockDim.x) {
+    for (int64_t i = first; i < nseg; i += step) {
         const int64_t s = seg_slot(f, num_nodes, w.node[i]);
         w.bucket[w.slot_offset[s] + rank[i]] = (int32_t)i;
     }
+}
+
+__global__ void bucket_count_kernel(Ws w, atdf_field_t f, int64_t num_nodes, int32_t* err)
+{
+    count_segments(w, f, num_nodes, err, (int64_t)blockIdx.x * blockDim.x + threadIdx.x,
+                   (int64_t)gridDim.x * blockDim.x);
+}
+
+__global__ void bucket_scatter_kernel(Ws w, atdf_field_t f, int64_t num_nodes)
+{
+    scatter_segments(w, f, num_nodes, (int64_t)blockIdx.x * blockDim.x + threadIdx.x, (int64_t)gridDim.x * blockDim.x);
 }
 
 // From the slots' segment counts, in one block and launch (each step is a few
@@ -80,13 +93,26 @@ __global__ void bucket_scatter_kernel(Ws w, atdf_field_t f, int64_t num_nodes)
 //    (longest-processing-time-first), a counting sort on min(count / 2, 255);
 //  * the item queue: each slot's items in the slot queue's order;
 //    counters[4] = the number of items.
-__global__ void __launch_bounds__(1024) plan_kernel(Ws w, int items)
+// SMALL (at most kSmallCap segments by capacity: small calls, whose time is
+// launches): the block also clears, counts and scatters, in place of a memset
+// and the two bucket kernels.
+constexpr int64_t kSmallCap = 16384;
+
+template <bool SMALL>
+__global__ void __launch_bounds__(1024) plan_kernel(Ws w, int items, atdf_field_t f, int64_t num_nodes, int32_t* err)
 {
     __shared__ int warp_sum[32];
     __shared__ int hist[256];
     __shared__ int s_base;
     const int n = (int)w.nslot + 1;  // plane slots and the out-of-ROI bucket
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    if (SMALL) {
+        for (int i = tid; i < n; i += 1024) w.slot_offset[i] = 0;
+        if (tid < 8) w.counters[tid] = 0;
+        __syncthreads();
+        count_segments(w, f, num_nodes, err, tid, 1024);
+        __syncthreads();
+    }
     int per = kSegItem;
     if (items > 0) per = (int)max((int64_t)kMinItem, min((int64_t)kSegItem, min(w.totals[0], w.cap) / items));
     for (int i = tid; i < 256; i += 1024) hist[i] = 0;
@@ -152,6 +178,7 @@ __global__ void __launch_bounds__(1024) plan_kernel(Ws w, int items)
     if (tid == 0) w.counters[4] = s_base;
     block_scan_exclusive<int32_t>(w.slot_offset, n + 1, nullptr, warp_sum);
     block_scan_exclusive<int32_t>(w.item_offset, n + 1, nullptr, warp_sum);
+    if (SMALL) scatter_segments(w, f, num_nodes, tid, 1024);
 }
 
 // Zeroes the plane gradients of the slots that no segment touches; the
@@ -444,14 +471,20 @@ static int project_forward(const atdf_tree_t* tree, const atdf_field_t* field, c
         if (st != ATDF_OK) return st;
     }
     if (bins) ATDF_CUDA_TRY(cudaMemsetAsync(bins, 0, (size_t)w.cap * kBins * sizeof(float), s));
-    // counters and slot counts lie side by side
-    ATDF_CUDA_TRY(cudaMemsetAsync(w.counters, 0, 256 + (w.nslot + 2) * 4, s));
-    bucket_count_kernel<<<592, 256, 0, s>>>(w, *field, tree->num_nodes, dev_error);
-    ATDF_LAUNCH_CHECK();
-    plan_kernel<<<1, 1024, 0, s>>>(w, var ? kSimtItems : 0);
-    ATDF_LAUNCH_CHECK();
-    bucket_scatter_kernel<<<592, 256, 0, s>>>(w, *field, tree->num_nodes);
-    ATDF_LAUNCH_CHECK();
+    const int items = var ? kSimtItems : 0;
+    if (w.cap <= kSmallCap) {
+        plan_kernel<true><<<1, 1024, 0, s>>>(w, items, *field, tree->num_nodes, dev_error);
+        ATDF_LAUNCH_CHECK();
+    } else {
+        // counters and slot counts lie side by side
+        ATDF_CUDA_TRY(cudaMemsetAsync(w.counters, 0, 256 + (w.nslot + 2) * 4, s));
+        bucket_count_kernel<<<592, 256, 0, s>>>(w, *field, tree->num_nodes, dev_error);
+        ATDF_LAUNCH_CHECK();
+        plan_kernel<false><<<1, 1024, 0, s>>>(w, items, *field, tree->num_nodes, dev_error);
+        ATDF_LAUNCH_CHECK();
+        bucket_scatter_kernel<<<592, 256, 0, s>>>(w, *field, tree->num_nodes);
+        ATDF_LAUNCH_CHECK();
+    }
     st = var ? launch_persistent(var->fwd, var->smem(false), p, s) : launch_tc_forward(p, s);
     if (st != ATDF_OK) return st;
     if (num_rays > 0) {
