@@ -11,6 +11,8 @@
 namespace atdf {
 
 constexpr int kSegItem = 128;         // segments per work item
+// Items that a forward by runs aims at: two for each of its CTAs.
+constexpr int kRunItems = 8 * 148;
 constexpr int kMinItem = 8;           // smallest share of a slot that becomes an item
 constexpr int kSegTabArrays = 17;     // per-segment arrays of the per-item segment table
 constexpr int kSegMapCap = 4096;      // samples of an item covered by the sample -> segment map
@@ -270,6 +272,13 @@ __device__ __forceinline__ int perm_index(int k, int total, double inv_total)
     return (int)r;
 }
 
+// Plane slot of segment si of an item taken by segments (-1 outside the ROI),
+// in the array that its kind of samples leaves free.
+__device__ __forceinline__ int item_slot(const FusedParams& p, const SegTab& tab, int si)
+{
+    return p.xt ? (int)tab.key_lo[si] : tab.first[si];
+}
+
 // Work is handed out by leaf slot: a CTA takes the next slot with segments
 // from the queue (counters[queue] counts slots) and then walks that slot's
 // work items of up to kSegItem segments itself, so each slot's planes are
@@ -290,14 +299,26 @@ __device__ __forceinline__ void init_item_queue(int* s_ctl)
 // in a row), so the items of a large slot spread over several CTAs; a CTA
 // stages a slot's planes when its next item is of another slot. bar null: the
 // kernel reads the planes from global memory, nothing is staged.
+// per_item > 0 (kernels that keep no per-slot state and read the planes from
+// global memory): items are runs of per_item segments of the bucketed list,
+// whatever slots they fall in (item_slot; box unused), so every item but the
+// last has the same number of segments and the tiles are full also where the
+// slots have few. bar is unused then, and the returned slot is 0.
 __device__ __forceinline__ ItemInfo next_item(const FusedParams& p, int queue, float* sm, SegTab tab, uint64_t* bar,
                                               int* s_ctl, bool want_dI, int map_cap = kSegMapCap,
-                                              bool by_item = false)
+                                              bool by_item = false, int per_item = 0)
 {
     const Ws& w = p.ws;
     const int tid = threadIdx.x;
     if (tid < 32) {
-        if (tid == 0 && by_item) {
+        if (tid == 0 && per_item > 0) {
+            const int64_t total = min(w.totals[0], w.cap);
+            const int64_t at = (int64_t)atomicAdd(&w.counters[queue], 1) * per_item;
+            s_ctl[0] = at < total ? 0 : -1;
+            s_ctl[1] = (int)at;
+            s_ctl[2] = (int)min((int64_t)per_item, total - at);
+            s_ctl[3] = 0;
+        } else if (tid == 0 && by_item) {
             int slot = -1, b0 = 0, nseg = 0, flags = 0;
             const int q = atomicAdd(&w.counters[queue], 1);
             if (q < w.counters[4]) {
@@ -430,7 +451,15 @@ __device__ __forceinline__ ItemInfo next_item(const FusedParams& p, int queue, f
         const uint64_t key = p.seed ? jitter_key(p.seed, r) : 0ull;
         tab.key_lo[tid] = (unsigned)key;
         tab.key_hi[tid] = (unsigned)(key >> 32);
-        if (tid == 0) {  // the item's leaf (segment 0's; other leaves read the tree)
+        if (per_item > 0) {
+            const int64_t sl = seg_slot(p.field, p.tree.num_nodes, node);
+            const int v = sl < p.field.num_slots ? (int)sl : -1;
+            if (p.xt)
+                tab.key_lo[tid] = (unsigned)v;
+            else
+                tab.first[tid] = v;
+        }
+        if (tid == 0 && per_item == 0) {  // the item's leaf (segment 0's; other leaves read the tree)
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
                 const float mn = p.tree.node_position_min[3 * node + k], mx = p.tree.node_position_max[3 * node + k];
@@ -549,19 +578,23 @@ __device__ __forceinline__ SampleState sample_state(const FusedParams& p, const 
 
 // sample_geo with the segment's box from the table and division-free
 // coordinates where the divisor is a power of two (bit-identical).
-__device__ __forceinline__ SampleGeo sample_geo_fast(const FusedParams& p, const SegTab& tab, int node,
+// tab null: an item of several leaves, always from the tree.
+__device__ __forceinline__ SampleGeo sample_geo_fast(const FusedParams& p, const SegTab* tab, int node,
                                                      const float pos[3])
 {
     float loc[3];
-    if (node == reinterpret_cast<const int*>(tab.box)[9]) {
+    if (tab && node == reinterpret_cast<const int*>(tab->box)[9]) {
 #pragma unroll
-        for (int k = 0; k < 3; ++k) loc[k] = local_coord_fast(pos[k], tab.box[k], tab.box[3 + k], tab.box[6 + k]);
+        for (int k = 0; k < 3; ++k) loc[k] = local_coord_fast(pos[k], tab->box[k], tab->box[3 + k], tab->box[6 + k]);
     } else {  // a slot shared by several leaves: this sample's box from the tree
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
             const float mn = p.tree.node_position_min[3 * node + k], mx = p.tree.node_position_max[3 * node + k];
             const float sz = __fsub_rn(mx, mn);
-            loc[k] = local_coord_fast(pos[k], mn, sz, pow2_reciprocal(sz));
+            // 1 / sz of a (normal) power of two: the exponent mirrored
+            const uint32_t bits = __float_as_uint(sz);
+            const bool pow2 = (bits & 0x807fffffu) == 0 && bits > 0x00ffffffu && bits < 0x7e800000u;
+            loc[k] = local_coord_fast(pos[k], mn, sz, pow2 ? __uint_as_float(0x7f000000u - bits) : 0.0f);
         }
     }
     SampleGeo g;
@@ -581,6 +614,12 @@ __device__ __forceinline__ SampleGeo sample_geo_fast(const FusedParams& p, const
     return g;
 }
 
+// Segments per item for a call of `items` items or more.
+__device__ __forceinline__ int segments_per_item(const Ws& w, int items)
+{
+    return (int)max((int64_t)kMinItem, min((int64_t)kSegItem, (min(w.totals[0], w.cap) + items - 1) / items));
+}
+
 // Adds rho * w of a sample at t into its segment's bins (forward, optional).
 __device__ __forceinline__ void add_to_bins(const FusedParams& p, const SegTab& tab, int si, float t, float v)
 {
@@ -588,6 +627,49 @@ __device__ __forceinline__ void add_to_bins(const FusedParams& p, const SegTab& 
     int b = len > 0.0f ? (int)((t - tmin) / len * (float)kBins) : 0;
     b = b < 0 ? 0 : (b >= kBins ? kBins - 1 : b);
     atomicAdd(&p.bins[(int64_t)tab.id[si] * kBins + b], v);
+}
+
+// Whether a tensor-core forward takes its work by runs of segments (planes from
+// global memory) rather than by slot (planes staged in shared memory). By slot
+// every item ends in a partly filled tile and every slot costs the staging of
+// its planes, which few segments a slot do not repay: forward of 16 channels,
+// 24 samples a segment, by slot and by runs, 1000 rays at depth 4: 231 and 110
+// us; 4096 rays: 299 and 244; 1000 rays at depth 2: 90 and 67. With more
+// segments the staged planes are read faster: 8192 rays at depth 4: 430 and
+// 474, 16384 rays: 669 and 741, at depth 3: 361 and 418. The line lies between
+// (4096 rays at depth 4 are 208,896 segments by capacity). 24 channels, whose
+// planes take half again the staging, stay level or better by runs wherever the
+// slots are many: 4096 slots of depth 6, 119 samples a segment, 4096 rays 315 and
+// 243 us, 16384 rays 759 and 734; depth 4, 16384 rays 678 and 668, 65536 rays
+// 2401 and 2339. Not so with 512 slots (16384 rays 370 and 396) or beyond
+// (65536 rays at depth 6: 2548 and 2607).
+static inline bool forward_by_runs(const FusedParams& p)
+{
+    if (p.ws.cap <= (1 << 18)) return true;
+    return p.field.channels == 24 && p.ws.nslot >= 2048 && p.ws.cap <= (1 << 22);
+}
+
+// Launches a persistent tensor-core kernel with `most` CTAs an SM (by its TMEM
+// columns and launch bounds) or what shared memory leaves of them.
+static inline int launch_tc_persistent(void (*fn)(FusedParams), int threads, int smem, int most, cudaStream_t st,
+                                       const FusedParams& p)
+{
+    int dev = 0, sms = 0, smem_sm = 0, per = 0;
+    ATDF_CUDA_TRY(cudaGetDevice(&dev));
+    ATDF_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    ATDF_CUDA_TRY(cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
+    ATDF_CUDA_TRY(cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    // staged planes want the whole carve-out; a forward by runs leaves the rest
+    // of the L1 to the texels
+    const int carveout =
+        most == 4 ? std::min(100, most * (smem + 1536) * 100 / smem_sm + 1) : (int)cudaSharedmemCarveoutMaxShared;
+    ATDF_CUDA_TRY(cudaFuncSetAttribute((const void*)fn, cudaFuncAttributePreferredSharedMemoryCarveout, carveout));
+    ATDF_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, (const void*)fn, threads, smem));
+    if (per < 1) return ATDF_ERR_UNSUPPORTED;
+    per = std::max(1, std::min(most, smem_sm / (smem + 1024)));
+    fn<<<sms * per, threads, smem, st>>>(p);
+    ATDF_LAUNCH_CHECK();
+    return ATDF_OK;
 }
 
 // BF16 tensor-core variants: 16 channels (fused_tc.cu) and 24 channels

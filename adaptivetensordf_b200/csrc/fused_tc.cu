@@ -36,12 +36,13 @@ namespace tcf {
 constexpr int kC = 16;
 constexpr int kH = 64;
 constexpr int kRows = 128;          // samples per tile
-constexpr int kThreadsTC = 256;     // two halves
+constexpr int kThreadsTC = 256;     // two halves (a forward by runs: one)
 constexpr int kHBCols = 96;         // H0 (64) | X (16) | ones | zero pad
 constexpr int kGCols = 128;         // dA1 (64) | dA0 (64)
 constexpr int kLineWinTC = 32;      // line-gradient window entries per line (shared memory)
 constexpr int kLineRowsTC = 21;     // rows per line in the line-gradient MMA (3 lines <= 64 rows)
-constexpr uint32_t kTmemFwd = 256;  // columns per CTA (2 CTAs per SM)
+constexpr uint32_t kTmemFwd = 256;  // columns per CTA (2 CTAs per SM; by runs 4 of 128)
+constexpr int kMapCapRuns = 2048;   // forward by runs: samples of an item covered by the sample -> segment map
 constexpr uint32_t kTmemBwd = 512;
 
 __device__ __forceinline__ uint32_t hb_off(int s, int c) { return tc::mnmajor_off(c, s, kHBCols); }
@@ -51,6 +52,13 @@ __device__ __forceinline__ uint32_t w1_off(int n, int k) { return tc::kmajor_off
 
 struct TCSmem {
     uint32_t planes, w0, w1, bias, hb[2], g[2], gplanes, gline, segi, total;
+    // The forward's by runs: one tile, the planes read from global memory.
+    __host__ __device__ TCSmem() : TCSmem(0, 0, false)
+    {
+        segi -= hb[1] - hb[0];
+        hb[1] = hb[0];
+        total = segi + (kSegTabFloats - (kSegMapCap - kMapCapRuns) / 4) * 4;
+    }
     __host__ __device__ TCSmem(int plane_elems, int gplane_elems, bool bwd)
     {
         auto al = [](uint32_t x) { return (x + 127u) & ~127u; };
@@ -100,8 +108,12 @@ __device__ __forceinline__ int first_corner(const Corner2& k, int Wp, int sel)
 // 8 * hf .. 8 * hf + 7, fb = the other eight, hf = lane mod 2. Lane p of an
 // 8-lane phase loads at step j the corner of residue p / 2 + j, first half
 // hf, then half 1 - hf: 8 distinct bank groups per instruction and phase.
-__device__ __forceinline__ void gather_features(const FusedParams& p, const unsigned char* sm, const SampleGeo& g,
-                                                float (&fa)[8], float (&fb)[8])
+// RUNS: the planes of `slot` are in global memory instead (unpadded; a texel is
+// one 32-byte sector, and a warp's rows walk along a ray, so they share
+// sectors). The corner order stays: it is part of a feature's rounding.
+template <bool RUNS>
+__device__ __forceinline__ void gather_features(const FusedParams& p, const unsigned char* sm, int64_t slot,
+                                                const SampleGeo& g, float (&fa)[8], float (&fb)[8])
 {
     const int lane = threadIdx.x & 31, hf = lane & 1;
 #pragma unroll
@@ -110,17 +122,18 @@ __device__ __forceinline__ void gather_features(const FusedParams& p, const unsi
         const int Wp = p.plane_pitch[m];
         const Corner2 k = corners2(g.pu[m], g.pv[m], Hm, Wm);
         const Corner1 l = corners1(g.lu[m], L);
-        const unsigned char* P = sm + (size_t)p.plane_off[m] * 2;
+        const uint4* P = RUNS ? reinterpret_cast<const uint4*>(p.field.plane[m]) + slot * (int64_t)(Hm * Wm * 2)
+                              : reinterpret_cast<const uint4*>(sm + (size_t)p.plane_off[m] * 2);
         const uint4* V = reinterpret_cast<const uint4*>(p.field.line[m]);
         const int c0 = first_corner(k, Wp, (lane & 7) >> 1);
         float ma[8], mb[8];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             float w;
-            const unsigned char* tx = P + corner_texel(k, (c0 + j) & 3, Wp, w) * (kC * 2);
+            const uint4* tx = P + 2 * corner_texel(k, (c0 + j) & 3, RUNS ? Wm : Wp, w);
             float u[8], v[8];
-            unpack_bf16x8(*reinterpret_cast<const uint4*>(tx + 16 * hf), u);
-            unpack_bf16x8(*reinterpret_cast<const uint4*>(tx + 16 * (hf ^ 1)), v);
+            unpack_bf16x8(RUNS ? __ldg(tx + hf) : tx[hf], u);
+            unpack_bf16x8(RUNS ? __ldg(tx + (hf ^ 1)) : tx[hf ^ 1], v);
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
                 ma[i] = j == 0 ? u[i] * w : fmaf(u[i], w, ma[i]);
@@ -183,6 +196,7 @@ __device__ __forceinline__ void issue_l1(const unsigned char* sm, const TCSmem& 
 // Forward sample features of tile row t into HB (X columns); returns validity.
 // The forward walks an item's samples in order: a warp's rows follow one ray,
 // so their plane gathers and segment-table reads share addresses.
+template <bool RUNS>
 __device__ __forceinline__ bool tile_features(const FusedParams& p, unsigned char* sm, const TCSmem& L,
                                               const SegTab& tab, const ItemInfo& it, bool real, int h, int k,
                                               int t, float& w, int& si, SampleGeo& g, float& ts)
@@ -199,9 +213,10 @@ __device__ __forceinline__ bool tile_features(const FusedParams& p, unsigned cha
         w = st.w;
         ts = st.t;
         si = st.si;
-        if (real) {
-            g = sample_geo_fast(p, tab, st.node, st.pos);
-            gather_features(p, sm, g, fa, fb);
+        const int slot = RUNS ? item_slot(p, tab, si) : real ? 0 : -1;
+        if (slot >= 0) {
+            g = sample_geo_fast(p, RUNS ? nullptr : &tab, st.node, st.pos);
+            gather_features<RUNS>(p, sm, slot, g, fa, fb);
         }
     }
     const int hf = threadIdx.x & 1;
@@ -227,16 +242,23 @@ __device__ __forceinline__ void epilogue_l0(unsigned char* sm, const TCSmem& L, 
     }
 }
 
-__global__ void __launch_bounds__(kThreadsTC, 2) tc_forward_kernel(FusedParams p)
+// By slot: two tiles a CTA of one plane slot, two CTAs an SM. By runs
+// (forward_by_runs): four CTAs of one tile each (46 KB of shared memory, 128
+// TMEM columns), so one's item set-up and last partial tile overlap the others'
+// tiles.
+template <bool RUNS>
+__global__ void __launch_bounds__(RUNS ? kRows : kThreadsTC, RUNS ? 4 : 2) tc_forward_kernel(FusedParams p)
 {
     extern __shared__ __align__(128) unsigned char sm[];
     __shared__ __align__(8) uint64_t bar_tma;
     __shared__ __align__(8) uint64_t bar_mma[2];
     __shared__ uint32_t s_tmem;
     __shared__ int s_ctl[8];
-    const TCSmem L(p.plane_off[3], p.gplane_off[3], false);
-    const int tid = threadIdx.x, h = tid / kRows, t = tid % kRows;
-    if (tid < 32) tc::tmem_alloc(&s_tmem, kTmemFwd);
+    constexpr int kHalves = RUNS ? 1 : 2;
+    constexpr uint32_t tmem_cols = kTmemFwd / 2 * kHalves;
+    const TCSmem L = RUNS ? TCSmem() : TCSmem(p.plane_off[3], p.gplane_off[3], false);
+    const int tid = threadIdx.x, h = RUNS ? 0 : tid / kRows, t = tid % kRows;
+    if (tid < 32) tc::tmem_alloc(&s_tmem, tmem_cols);
     if (tid == 0) {
         mbar_init(&bar_tma, 1);
         init_item_queue(s_ctl);
@@ -254,13 +276,15 @@ __global__ void __launch_bounds__(kThreadsTC, 2) tc_forward_kernel(FusedParams p
     const float* bias = reinterpret_cast<const float*>(sm + L.bias);
     const float beta = p.mlp.softplus_beta;
     const int lact = p.mlp.last_activation;
+    const int per_item = RUNS ? segments_per_item(p.ws, kRunItems) : 0;
     uint32_t tma_phase = 0, mma_phase = 0;
     bool alive = true;
     while (alive) {
-        const ItemInfo it = next_item(p, 0, reinterpret_cast<float*>(sm), tab, &bar_tma, s_ctl, false, kSegMapCap, true);
+        const ItemInfo it = next_item(p, 0, reinterpret_cast<float*>(sm), tab, &bar_tma, s_ctl, false,
+                                      RUNS ? kMapCapRuns : kSegMapCap, true, per_item);
         if (it.slot < 0) break;
         const bool real = it.slot < p.ws.nslot;
-        if (real && it.first) {
+        if (!RUNS && real && it.first) {
             if (!mbar_wait(&bar_tma, tma_phase)) {
                 set_err(p.err, ATDF_DEVERR_TREE);
                 mbar_wait(&bar_tma, tma_phase);
@@ -269,11 +293,11 @@ __global__ void __launch_bounds__(kThreadsTC, 2) tc_forward_kernel(FusedParams p
             tma_phase ^= 1;
         }
         alive = __syncthreads_and(alive);
-        for (int t0 = h * kRows; alive && t0 < it.total; t0 += 2 * kRows) {
+        for (int t0 = h * kRows; alive && t0 < it.total; t0 += kHalves * kRows) {
             float w, ts;
             int si;
             SampleGeo g;
-            const bool valid = tile_features(p, sm, L, tab, it, real, h, t0 + t, t, w, si, g, ts);
+            const bool valid = tile_features<RUNS>(p, sm, L, tab, it, real, h, t0 + t, t, w, si, g, ts);
             tc::fence_smem_to_async();
             tc::fence_before_sync();
             half_barrier(h);
@@ -330,7 +354,7 @@ __global__ void __launch_bounds__(kThreadsTC, 2) tc_forward_kernel(FusedParams p
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
-    if (tid < 32) tc::tmem_dealloc(s_tmem, kTmemFwd);
+    if (tid < 32) tc::tmem_dealloc(s_tmem, tmem_cols);
 }
 
 // ---------------------------------------------------------------------------
@@ -408,7 +432,7 @@ __device__ __forceinline__ bool tile_features_half(const FusedParams& p, unsigne
         w = st.w;
         si = st.si;
         if (real) {
-            g = sample_geo_fast(p, tab, st.node, st.pos);
+            g = sample_geo_fast(p, &tab, st.node, st.pos);
             // planes 2, 1, 0, as in gather_features
 #pragma unroll
             for (int m = 2; m >= 0; --m) {
@@ -969,36 +993,20 @@ static int max_optin()
     return v;
 }
 
-static int launch_tc(void (*fn)(FusedParams), bool bwd, const FusedParams& p, cudaStream_t st,
-                     int threads = tcf::kThreadsTC)
+static int launch_tc(void (*fn)(FusedParams), bool bwd, const FusedParams& p, cudaStream_t st, int threads,
+                     bool runs = false)
 {
-    const int smem = (int)tcf::TCSmem(p.plane_off[3], p.gplane_off[3], bwd).total;
+    int smem = (int)tcf::TCSmem(p.plane_off[3], p.gplane_off[3], bwd).total;
     if (smem > max_optin()) return ATDF_ERR_UNSUPPORTED;
-    ATDF_CUDA_TRY(cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    // without an explicit carveout the occupancy query assumes a smaller
-    // shared-memory partition and reports one forward CTA per SM
-    ATDF_CUDA_TRY(cudaFuncSetAttribute((const void*)fn, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                       (int)cudaSharedmemCarveoutMaxShared));
-    int dev = 0, sms = 0, per = 0;
-    ATDF_CUDA_TRY(cudaGetDevice(&dev));
-    ATDF_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    ATDF_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, (const void*)fn, threads, smem));
-    if (per < 1) return ATDF_ERR_UNSUPPORTED;
-    // TMEM: 256 columns per forward CTA, 512 per backward CTA (512 per SM).
-    // The forward fits two CTAs per SM by shared memory and registers
-    // (launch bounds); the occupancy query reports one, so size it here.
-    int smem_sm = 0;
-    ATDF_CUDA_TRY(cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
-    per = bwd ? 1 : std::max(1, std::min(2, smem_sm / (smem + 1024)));
-    fn<<<sms * per, threads, smem, st>>>(p);
-    ATDF_LAUNCH_CHECK();
-    return ATDF_OK;
+    if (runs) smem = (int)tcf::TCSmem().total;
+    return launch_tc_persistent(fn, threads, smem, bwd ? 1 : runs ? 4 : 2, st, p);
 }
 
 int launch_tc_forward(const FusedParams& p, cudaStream_t st)
 {
     if (p.field.channels == 24) return launch_tc24_forward(p, st);
-    return launch_tc(tcf::tc_forward_kernel, false, p, st);
+    if (forward_by_runs(p)) return launch_tc(tcf::tc_forward_kernel<true>, false, p, st, tcf::kRows, true);
+    return launch_tc(tcf::tc_forward_kernel<false>, false, p, st, tcf::kThreadsTC);
 }
 // The backward runs two threads per sample row (512 threads per CTA).
 int launch_tc_backward(const FusedParams& p, cudaStream_t st)

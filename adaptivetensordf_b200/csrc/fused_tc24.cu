@@ -82,6 +82,13 @@ __device__ __forceinline__ uint32_t w1_off(int n, int k) { return tc::kmajor_off
 struct Smem24 {
     uint32_t planes, w0, w1, bias, hb[2], g, gplanes, lwin, segi, total;
     // gplane_elems: the unpadded plane-gradient elements (texels x 24)
+    // The forward's by runs: one tile, planes and lines read from global memory.
+    __host__ __device__ Smem24() : Smem24(0, 0, false)
+    {
+        hb[1] = hb[0];
+        segi = hb[0] + kRows * kHBColsF * 2;
+        total = segi + (kSegTabFloats - (kSegMapCap - kMapCapF) / 4) * 4;
+    }
     __host__ __device__ Smem24(int plane_elems, int gplane_elems, bool bwd)
     {
         auto al = [](uint32_t x) { return (x + 127u) & ~127u; };
@@ -206,8 +213,10 @@ __device__ __forceinline__ void stage_line_windows(const FusedParams& p, const f
 // VM feature of one sample, all 24 channels: planes (BF16, shared memory) and
 // lines (BF16, the slot's window in shared memory when both taps are inside
 // it, else global), plane 2 first, corners in order.
+// RUNS: the planes of `slot` (unpadded) and all line taps from global memory.
+template <bool RUNS>
 __device__ __forceinline__ void gather24(const FusedParams& p, const unsigned char* sm, const unsigned char* LW,
-                                         const int* s_lo, const SampleGeo& g, float (&f)[kC])
+                                         const int* s_lo, int64_t slot, const SampleGeo& g, float (&f)[kC])
 {
 #pragma unroll
     for (int m = 2; m >= 0; --m) {
@@ -215,22 +224,27 @@ __device__ __forceinline__ void gather24(const FusedParams& p, const unsigned ch
         const int Wp = p.plane_pitch[m];
         const Corner2 k = corners2(g.pu[m], g.pv[m], Hm, Wm);
         const Corner1 l = corners1(g.lu[m], L);
-        const unsigned char* P = sm + (size_t)p.plane_off[m] * 2;
-        const int r0 = l.x0 - s_lo[m], r1 = l.x1 - s_lo[m];
-        const bool inwin = (unsigned)r0 < (unsigned)kLineRows && (unsigned)r1 < (unsigned)kLineRows;
-        const unsigned char* V0 = inwin ? LW + (size_t)m * (kLineRows * kC * 2) + r0 * (kC * 2)
-                                        : reinterpret_cast<const unsigned char*>(p.field.line[m]) + l.x0 * (kC * 2);
-        const unsigned char* V1 = inwin ? LW + (size_t)m * (kLineRows * kC * 2) + r1 * (kC * 2)
-                                        : reinterpret_cast<const unsigned char*>(p.field.line[m]) + l.x1 * (kC * 2);
+        const uint4* P = RUNS ? reinterpret_cast<const uint4*>(p.field.plane[m]) + slot * (int64_t)(Hm * Wm * 3)
+                              : reinterpret_cast<const uint4*>(sm + (size_t)p.plane_off[m] * 2);
+        const uint4* V = reinterpret_cast<const uint4*>(p.field.line[m]);
+        const uint4 *V0 = V + l.x0 * 3, *V1 = V + l.x1 * 3;
+        if (!RUNS) {
+            const int r0 = l.x0 - s_lo[m], r1 = l.x1 - s_lo[m];
+            if ((unsigned)r0 < (unsigned)kLineRows && (unsigned)r1 < (unsigned)kLineRows) {
+                const uint4* W = reinterpret_cast<const uint4*>(LW + (size_t)m * (kLineRows * kC * 2));
+                V0 = W + r0 * 3;
+                V1 = W + r1 * 3;
+            }
+        }
         float ma[kC];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             float w;
-            const unsigned char* tx = P + corner_texel(k, j, Wp, w) * (kC * 2);
+            const uint4* tx = P + corner_texel(k, j, RUNS ? Wm : Wp, w) * 3;
 #pragma unroll
             for (int q = 0; q < 3; ++q) {
                 float u[8];
-                unpack_bf16x8(*reinterpret_cast<const uint4*>(tx + 16 * q), u);
+                unpack_bf16x8(RUNS ? __ldg(tx + q) : tx[q], u);
 #pragma unroll
                 for (int i = 0; i < 8; ++i) ma[8 * q + i] = j == 0 ? u[i] * w : fmaf(u[i], w, ma[8 * q + i]);
             }
@@ -238,8 +252,8 @@ __device__ __forceinline__ void gather24(const FusedParams& p, const unsigned ch
 #pragma unroll
         for (int q = 0; q < 3; ++q) {
             float v0[8], v1[8];
-            unpack_bf16x8(*reinterpret_cast<const uint4*>(V0 + 16 * q), v0);
-            unpack_bf16x8(*reinterpret_cast<const uint4*>(V1 + 16 * q), v1);
+            unpack_bf16x8(RUNS ? __ldg(V0 + q) : V0[q], v0);
+            unpack_bf16x8(RUNS ? __ldg(V1 + q) : V1[q], v1);
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
                 const float ve = fmaf(v0[i], l.w0, v1[i] * l.w1);
@@ -249,7 +263,9 @@ __device__ __forceinline__ void gather24(const FusedParams& p, const unsigned ch
     }
 }
 
-__global__ void __launch_bounds__(kThreadsF, 2) tc24_forward_kernel(FusedParams p)
+// By slot or by runs, as tc_forward_kernel of fused_tc.cu.
+template <bool RUNS>
+__global__ void __launch_bounds__(RUNS ? kRows : kThreadsF, RUNS ? 4 : 2) tc24_forward_kernel(FusedParams p)
 {
     extern __shared__ __align__(128) unsigned char sm[];
     __shared__ __align__(8) uint64_t bar_tma;
@@ -257,9 +273,11 @@ __global__ void __launch_bounds__(kThreadsF, 2) tc24_forward_kernel(FusedParams 
     __shared__ uint32_t s_tmem;
     __shared__ int s_ctl[8];
     __shared__ int s_lo[3];
-    const Smem24 L(p.plane_off[3], p.gplane_off[3], false);
-    const int tid = threadIdx.x, h = tid / kRows, t = tid % kRows;
-    if (tid < 32) tc::tmem_alloc(&s_tmem, kTmemF);
+    constexpr int kHalves = RUNS ? 1 : 2;
+    constexpr uint32_t tmem_cols = kTmemF / 2 * kHalves;
+    const Smem24 L = RUNS ? Smem24() : Smem24(p.plane_off[3], p.gplane_off[3], false);
+    const int tid = threadIdx.x, h = RUNS ? 0 : tid / kRows, t = tid % kRows;
+    if (tid < 32) tc::tmem_alloc(&s_tmem, tmem_cols);
     if (tid == 0) {
         mbar_init(&bar_tma, 1);
         init_item_queue(s_ctl);
@@ -278,13 +296,15 @@ __global__ void __launch_bounds__(kThreadsF, 2) tc24_forward_kernel(FusedParams 
     const float beta = p.mlp.softplus_beta;
     const int lact = p.mlp.last_activation;
     unsigned char* hbh = sm + L.hb[h];
+    const int per_item = RUNS ? segments_per_item(p.ws, kRunItems) : 0;
     uint32_t tma_phase = 0, mma_phase = 0;
     bool alive = true;
     while (alive) {
-        const ItemInfo it = next_item(p, 0, reinterpret_cast<float*>(sm), tab, &bar_tma, s_ctl, false, kMapCapF, true);
+        const ItemInfo it = next_item(p, 0, reinterpret_cast<float*>(sm), tab, &bar_tma, s_ctl, false, kMapCapF, true,
+                                      per_item);
         if (it.slot < 0) break;
         const bool real = it.slot < p.ws.nslot;
-        if (real && it.first) {
+        if (!RUNS && real && it.first) {
             stage_line_windows(p, tab.box, sm + L.lwin, s_lo);
             if (!mbar_wait(&bar_tma, tma_phase)) {
                 set_err(p.err, ATDF_DEVERR_TREE);
@@ -294,7 +314,7 @@ __global__ void __launch_bounds__(kThreadsF, 2) tc24_forward_kernel(FusedParams 
             tma_phase ^= 1;
         }
         alive = __syncthreads_and(alive);
-        for (int t0 = h * kRows; alive && t0 < it.total; t0 += 2 * kRows) {
+        for (int t0 = h * kRows; alive && t0 < it.total; t0 += kHalves * kRows) {
             const int k = t0 + t;
             const bool valid = k < it.total;
             float f[kC];
@@ -307,9 +327,10 @@ __global__ void __launch_bounds__(kThreadsF, 2) tc24_forward_kernel(FusedParams 
                 w = st.w;
                 ts = st.t;
                 si = st.si;
-                if (real) {
-                    const SampleGeo g = sample_geo_fast(p, tab, st.node, st.pos);
-                    gather24(p, sm, sm + L.lwin, s_lo, g, f);
+                const int slot = RUNS ? item_slot(p, tab, si) : real ? 0 : -1;
+                if (slot >= 0) {
+                    const SampleGeo g = sample_geo_fast(p, RUNS ? nullptr : &tab, st.node, st.pos);
+                    gather24<RUNS>(p, sm, sm + L.lwin, s_lo, slot, g, f);
                 }
             }
 #pragma unroll
@@ -387,7 +408,7 @@ __global__ void __launch_bounds__(kThreadsF, 2) tc24_forward_kernel(FusedParams 
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
-    if (tid < 32) tc::tmem_dealloc(s_tmem, kTmemF);
+    if (tid < 32) tc::tmem_dealloc(s_tmem, tmem_cols);
 }
 
 // ---------------------------------------------------------------------------
@@ -555,7 +576,7 @@ __global__ void __launch_bounds__(kThreadsB, 1) tc24_backward_kernel(FusedParams
                 w = st.w;
                 si = st.si;
                 if (real) {
-                    g = sample_geo_fast(p, tab, st.node, st.pos);
+                    g = sample_geo_fast(p, &tab, st.node, st.pos);
                     act = true;
                 }
             }
@@ -726,7 +747,7 @@ __global__ void __launch_bounds__(kThreadsB, 1) tc24_backward_kernel(FusedParams
             } else if (real && t0 + kRows < it.total && s_pre_si[t] >= 0) {
                 // group 2, part 2: the next tile's plane and line coordinates
                 const float pos[3] = {s_pre[6][t], s_pre[7][t], s_pre[8][t]};
-                const SampleGeo g2 = sample_geo_fast(p, tab, s_pre_node[t], pos);
+                const SampleGeo g2 = sample_geo_fast(p, &tab, s_pre_node[t], pos);
 #pragma unroll
                 for (int q = 0; q < 3; ++q) {
                     s_pre[q][t] = g2.pu[q];
@@ -1066,33 +1087,22 @@ bool tc24_supported(const atdf_field_t* f, const atdf_mlp_t* m)
            m->hidden_activation == ATDF_ACT_SILU;
 }
 
-static int launch24(void (*fn)(FusedParams), bool bwd, const FusedParams& p, cudaStream_t st)
+static int launch24(void (*fn)(FusedParams), bool bwd, const FusedParams& p, cudaStream_t st, bool runs = false)
 {
-    const int smem = (int)tc24::Smem24(p.plane_off[3], p.gplane_off[3], bwd).total;
-    int dev = 0, optin = 0, sms = 0, per = 0;
+    int smem = (int)tc24::Smem24(p.plane_off[3], p.gplane_off[3], bwd).total;
+    int dev = 0, optin = 0, sms = 0;
     ATDF_CUDA_TRY(cudaGetDevice(&dev));
     ATDF_CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     if (smem > optin) return ATDF_ERR_UNSUPPORTED;
-    ATDF_CUDA_TRY(cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    ATDF_CUDA_TRY(cudaFuncSetAttribute((const void*)fn, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                       (int)cudaSharedmemCarveoutMaxShared));
-    ATDF_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    const int threads = bwd ? tc24::kThreadsB : tc24::kThreadsF;
-    ATDF_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, (const void*)fn, threads, smem));
-    if (per < 1) return ATDF_ERR_UNSUPPORTED;
-    // the forward fits two CTAs per SM (shared memory, 2 x 256 TMEM columns);
-    // the backward one (its shared memory, all 512 TMEM columns)
-    int smem_sm = 0;
-    ATDF_CUDA_TRY(cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
-    per = bwd ? 1 : std::max(1, std::min(2, smem_sm / (smem + 1024)));
-    fn<<<sms * per, threads, smem, st>>>(p);
-    ATDF_LAUNCH_CHECK();
-    return ATDF_OK;
+    if (runs) smem = (int)tc24::Smem24().total;
+    const int threads = bwd ? tc24::kThreadsB : runs ? tc24::kRows : tc24::kThreadsF;
+    return launch_tc_persistent(fn, threads, smem, bwd ? 1 : runs ? 4 : 2, st, p);
 }
 
 int launch_tc24_forward(const FusedParams& p, cudaStream_t st)
 {
-    return launch24(tc24::tc24_forward_kernel, false, p, st);
+    if (forward_by_runs(p)) return launch24(tc24::tc24_forward_kernel<true>, false, p, st, true);
+    return launch24(tc24::tc24_forward_kernel<false>, false, p, st);
 }
 int launch_tc24_backward(const FusedParams& p, cudaStream_t st)
 {
