@@ -294,131 +294,174 @@ __device__ __forceinline__ void init_item_queue(int* s_ctl)
     s_ctl[7] = 0;
 }
 
-// by_item (kernels that keep no per-slot state between items): work is handed
-// out by item from the item queue (the slot queue's order, each slot's items
-// in a row), so the items of a large slot spread over several CTAs; a CTA
-// stages a slot's planes when its next item is of another slot. bar null: the
-// kernel reads the planes from global memory, nothing is staged.
-// per_item > 0 (kernels that keep no per-slot state and read the planes from
-// global memory): items are runs of per_item segments of the bucketed list,
-// whatever slots they fall in (item_slot; box unused), so every item but the
-// last has the same number of segments and the tiles are full also where the
-// slots have few. bar is unused then, and the returned slot is 0.
-__device__ __forceinline__ ItemInfo next_item(const FusedParams& p, int queue, float* sm, SegTab tab, uint64_t* bar,
-                                              int* s_ctl, bool want_dI, int map_cap = kSegMapCap,
-                                              bool by_item = false, int per_item = 0)
+// Takes the next item of the CTA's slot, or of the next slot with work, in one
+// thread: s_ctl[0..2] = slot (-1: the queue is empty), first bucket entry and
+// number of segments. Returns 1: first of its slot, 2: last, 4: its planes are
+// to be staged.
+__device__ __forceinline__ int pop_item(const Ws& w, int queue, int* s_ctl)
+{
+    int slot = -1, b0 = 0, nseg = 0, flags = 0;
+    if (s_ctl[5] >= s_ctl[6]) {  // the current slot is done: take the next one with work
+        const int nslots = (int)w.nslot + 1;  // plane slots + the out-of-ROI bucket
+        s_ctl[4] = -1;
+        while (true) {
+            const int q = atomicAdd(&w.counters[queue], 1);
+            if (q >= nslots) break;
+            const int sl = w.slot_order[q];  // largest slots first (plan_kernel)
+            const int i0 = w.item_offset[sl], i1 = w.item_offset[sl + 1];
+            const int o0 = w.slot_offset[sl], o1 = w.slot_offset[sl + 1];
+            if (i1 > i0) {
+                s_ctl[4] = sl;
+                s_ctl[5] = 0;
+                s_ctl[6] = s_ctl[7] = i1 - i0;
+                s_ctl[8] = o0;
+                s_ctl[9] = o1;
+                flags |= 1;
+                break;
+            }
+        }
+        if (s_ctl[4] >= 0 && s_ctl[4] < w.nslot) flags |= 4;
+    }
+    if (s_ctl[4] >= 0 && s_ctl[5] < s_ctl[6]) {
+        slot = s_ctl[4];
+        const int it = s_ctl[5]++;
+        // the slot's segments in s_ctl[7] items of equal size (<= kSegItem)
+        const int per = (s_ctl[9] - s_ctl[8] + s_ctl[7] - 1) / s_ctl[7];
+        b0 = s_ctl[8] + it * per;
+        nseg = min(b0 + per, s_ctl[9]) - b0;
+        if (s_ctl[5] == s_ctl[6]) flags |= 2;
+    }
+    s_ctl[0] = slot;
+    s_ctl[1] = b0;
+    s_ctl[2] = nseg;
+    return flags;
+}
+
+// Bytes of a slot's three planes, announced to bar by one thread.
+__device__ __forceinline__ void expect_planes(const FusedParams& p, uint64_t* bar)
+{
+    // plane_off counts elements of the plane type (4 or 2 bytes)
+    const int esz = p.field.dtype == ATDF_BF16 ? 2 : 4;
+    uint32_t bytes = 0;
+    for (int m = 0; m < 3; ++m)
+        bytes += (uint32_t)(p.field.plane_h[m] * p.field.plane_w[m] * p.field.channels * esz);
+    mbar_expect_tx(bar, bytes);
+}
+
+// One warp's copies of slot sl's three planes to sm, spread over its lanes.
+__device__ __forceinline__ void stage_planes(const FusedParams& p, float* sm, int64_t sl, uint64_t* bar)
+{
+    const int lane = threadIdx.x & 31;
+    const int esz = p.field.dtype == ATDF_BF16 ? 2 : 4;
+    fence_proxy_async();
+    // copy c of plane m: its whole plane (unpadded) or its row c (padded)
+    int c0 = 0;
+    for (int m = 0; m < 3; ++m) {
+        const int64_t pf = (int64_t)p.field.plane_h[m] * p.field.plane_w[m] * p.field.channels;
+        char* dst = reinterpret_cast<char*>(sm) + (size_t)p.plane_off[m] * esz;
+        const char* src = reinterpret_cast<const char*>(p.field.plane[m]) + (size_t)sl * pf * esz;
+        const bool padded = p.plane_pitch[m] != p.field.plane_w[m];
+        const int ncopy = padded ? p.field.plane_h[m] : 1;
+        const uint32_t row = (uint32_t)(p.field.plane_w[m] * p.field.channels * esz);
+        const uint32_t pitch = (uint32_t)(p.plane_pitch[m] * p.field.channels * esz);
+        for (int c = ((lane - c0) % 32 + 32) % 32; c < ncopy; c += 32) {
+            if (padded)
+                tma_bulk_load(dst + (size_t)c * pitch, src + (size_t)c * row, row, bar);
+            else
+                tma_bulk_load(dst, src, (uint32_t)(pf * esz), bar);
+        }
+        c0 += ncopy;
+    }
+}
+
+// A segment's row of the table. The loads come before the first store, so that
+// they wait for memory together: bucket, then the segment's entries, then its
+// ray's.
+struct SegRow {
+    int id, node, n, ray, first;
+    float tmin, tmax, dI, org[3], dir[3];
+};
+
+__device__ __forceinline__ SegRow load_row(const FusedParams& p, int at, bool want_dI)
 {
     const Ws& w = p.ws;
-    const int tid = threadIdx.x;
-    if (tid < 32) {
-        if (tid == 0 && per_item > 0) {
-            const int64_t total = min(w.totals[0], w.cap);
-            const int64_t at = (int64_t)atomicAdd(&w.counters[queue], 1) * per_item;
-            s_ctl[0] = at < total ? 0 : -1;
-            s_ctl[1] = (int)at;
-            s_ctl[2] = (int)min((int64_t)per_item, total - at);
-            s_ctl[3] = 0;
-        } else if (tid == 0 && by_item) {
-            int slot = -1, b0 = 0, nseg = 0, flags = 0;
-            const int q = atomicAdd(&w.counters[queue], 1);
-            if (q < w.counters[4]) {
-                const int2 e = w.item_queue[q];
-                slot = e.x;
-                const int nit = w.item_offset[slot + 1] - w.item_offset[slot];
-                if (slot != s_ctl[4]) {
-                    s_ctl[4] = slot;
-                    flags |= 1;
-                    if (slot < w.nslot && bar) {
-                        const int esz = p.field.dtype == ATDF_BF16 ? 2 : 4;
-                        uint32_t bytes = 0;
-                        for (int m = 0; m < 3; ++m)
-                            bytes += (uint32_t)(p.field.plane_h[m] * p.field.plane_w[m] * p.field.channels * esz);
-                        mbar_expect_tx(bar, bytes);
-                        flags |= 4;
-                    }
-                }
-                const int cnt = w.slot_offset[slot + 1] - w.slot_offset[slot];
-                const int per = (cnt + nit - 1) / nit;
-                b0 = w.slot_offset[slot] + e.y * per;
-                nseg = min(b0 + per, w.slot_offset[slot + 1]) - b0;
-                if (e.y == nit - 1) flags |= 2;
-                s_ctl[7] = nit;
-            }
-            s_ctl[0] = slot;
-            s_ctl[1] = b0;
-            s_ctl[2] = nseg;
-            s_ctl[3] = flags;
-        } else if (tid == 0) {
-            int slot = -1, b0 = 0, nseg = 0, flags = 0;
-            if (s_ctl[5] >= s_ctl[6]) {  // the current slot is done: take the next one with work
-                const int nslots = (int)w.nslot + 1;  // plane slots + the out-of-ROI bucket
-                s_ctl[4] = -1;
-                while (true) {
-                    const int q = atomicAdd(&w.counters[queue], 1);
-                    if (q >= nslots) break;
-                    const int sl = w.slot_order[q];  // largest slots first (plan_kernel)
-                    const int i0 = w.item_offset[sl], i1 = w.item_offset[sl + 1];
-                    if (i1 > i0) {
-                        s_ctl[4] = sl;
-                        s_ctl[5] = i0;
-                        s_ctl[6] = i1;
-                        s_ctl[7] = i1 - i0;
-                        flags |= 1;
-                        break;
-                    }
-                }
-                if (s_ctl[4] >= 0 && s_ctl[4] < w.nslot) {
-                    // plane_off counts elements of the plane type (4 or 2 bytes)
-                    const int esz = p.field.dtype == ATDF_BF16 ? 2 : 4;
-                    uint32_t bytes = 0;
-                    for (int m = 0; m < 3; ++m)
-                        bytes += (uint32_t)(p.field.plane_h[m] * p.field.plane_w[m] * p.field.channels * esz);
-                    mbar_expect_tx(bar, bytes);
-                    flags |= 4;  // warp 0 issues the slot's plane copies below
-                }
-            }
-            if (s_ctl[4] >= 0 && s_ctl[5] < s_ctl[6]) {
-                slot = s_ctl[4];
-                const int it = s_ctl[5]++;
-                // the slot's segments in s_ctl[7] items of equal size (<= kSegItem)
-                const int cnt = w.slot_offset[slot + 1] - w.slot_offset[slot];
-                const int per = (cnt + s_ctl[7] - 1) / s_ctl[7];
-                b0 = w.slot_offset[slot] + (it - w.item_offset[slot]) * per;
-                const int b1 = min(b0 + per, w.slot_offset[slot + 1]);
-                nseg = b1 - b0;
-                if (s_ctl[5] == s_ctl[6]) flags |= 2;
-            }
-            s_ctl[0] = slot;
-            s_ctl[1] = b0;
-            s_ctl[2] = nseg;
-            s_ctl[3] = flags;
-        }
-        __syncwarp();
-        if (s_ctl[3] & 4) {  // a new plane slot: its three planes, the copies spread over warp 0's lanes
-            const int64_t sl = s_ctl[4];
-            const int esz = p.field.dtype == ATDF_BF16 ? 2 : 4;
-            fence_proxy_async();
-            // copy c of plane m: its whole plane (unpadded) or its row c (padded)
-            int c0 = 0;
-            for (int m = 0; m < 3; ++m) {
-                const int64_t pf = (int64_t)p.field.plane_h[m] * p.field.plane_w[m] * p.field.channels;
-                char* dst = reinterpret_cast<char*>(sm) + (size_t)p.plane_off[m] * esz;
-                const char* src = reinterpret_cast<const char*>(p.field.plane[m]) + (size_t)sl * pf * esz;
-                const bool padded = p.plane_pitch[m] != p.field.plane_w[m];
-                const int ncopy = padded ? p.field.plane_h[m] : 1;
-                const uint32_t row = (uint32_t)(p.field.plane_w[m] * p.field.channels * esz);
-                const uint32_t pitch = (uint32_t)(p.plane_pitch[m] * p.field.channels * esz);
-                for (int c = ((tid - c0) % 32 + 32) % 32; c < ncopy; c += 32) {
-                    if (padded)
-                        tma_bulk_load(dst + (size_t)c * pitch, src + (size_t)c * row, row, bar);
-                    else
-                        tma_bulk_load(dst, src, (uint32_t)(pf * esz), bar);
-                }
-                c0 += ncopy;
-            }
-        }
+    SegRow r;
+    r.id = w.bucket[at];
+    r.ray = w.ray[r.id];
+    r.node = w.node[r.id];
+    r.n = w.nsamp[r.id];
+    r.tmin = w.tmin[r.id];
+    r.tmax = w.tmax[r.id];
+    r.first = p.xt ? w.first[r.id] : 0;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        r.org[k] = p.origin[3 * r.ray + k];
+        r.dir[k] = p.dir[3 * r.ray + k];
     }
-    __syncthreads();
+    r.dI = want_dI ? p.grad_image[r.ray] : 0.0f;
+    if (p.xt) r.first += (int)w.ray_sample_offset[r.ray];
+    return r;
+}
+
+// slots: the row keeps its segment's plane slot too (item_slot).
+__device__ __forceinline__ void store_row(const FusedParams& p, const SegTab& tab, int i, const SegRow& r, bool slots)
+{
+    tab.id[i] = r.id;
+    tab.node[i] = r.node;
+    tab.n[i] = r.n;
+    tab.tmin[i] = r.tmin;
+    tab.tmax[i] = r.tmax;
+    tab.step[i] = __fdiv_rn(__fsub_rn(r.tmax, r.tmin), (float)r.n);  // sample_t's step
+    tab.acc[i] = r.dI;
+    tab.first[i] = r.first;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        tab.org[k][i] = r.org[k];
+        tab.dir[k][i] = r.dir[k];
+    }
+    const uint64_t key = p.seed ? jitter_key(p.seed, r.ray) : 0ull;
+    tab.key_lo[i] = (unsigned)key;
+    tab.key_hi[i] = (unsigned)(key >> 32);
+    if (slots) {
+        const int64_t sl = seg_slot(p.field, p.tree.num_nodes, r.node);
+        const int v = sl < p.field.num_slots ? (int)sl : -1;
+        if (p.xt)
+            tab.key_lo[i] = (unsigned)v;
+        else
+            tab.first[i] = v;
+    }
+}
+
+// The item's leaf (segment 0's; other leaves read the tree): an axis a lane for
+// t = 96, 97 and 98 of 128 threads, beside the rows.
+struct BoxLane {
+    int node;
+    float mn, mx;
+};
+
+__device__ __forceinline__ BoxLane load_box(const FusedParams& p, int t, int b0)
+{
+    BoxLane b = {};
+    if (t < 96 || t > 98) return b;
+    b.node = p.ws.node[p.ws.bucket[b0]];
+    b.mn = p.tree.node_position_min[3 * b.node + t - 96];
+    b.mx = p.tree.node_position_max[3 * b.node + t - 96];
+    return b;
+}
+
+__device__ __forceinline__ void store_box(const SegTab& tab, int t, const BoxLane& b)
+{
+    if (t < 96 || t > 98) return;
+    const float sz = __fsub_rn(b.mx, b.mn);
+    tab.box[t - 96] = b.mn;
+    tab.box[3 + t - 96] = sz;
+    tab.box[6 + t - 96] = pow2_reciprocal(sz);
+    if (t == 96) reinterpret_cast<int*>(tab.box)[9] = b.node;
+}
+
+// The item that s_ctl describes, without its samples.
+__device__ __forceinline__ ItemInfo item_info(const int* s_ctl)
+{
     ItemInfo info;
     info.slot = s_ctl[0];
     info.nseg = s_ctl[2];
@@ -428,49 +471,13 @@ __device__ __forceinline__ ItemInfo next_item(const FusedParams& p, int queue, f
     info.total = 0;
     info.inv_total = 0.0;
     info.use_map = false;
-    if (info.slot < 0) return info;
-    const int b0 = s_ctl[1];
-    if (tid < info.nseg) {
-        const int sid = w.bucket[b0 + tid];
-        tab.id[tid] = sid;
-        tab.node[tid] = w.node[sid];
-        tab.n[tid] = w.nsamp[sid];
-        const float tmin = w.tmin[sid], tmax = w.tmax[sid];
-        const int n = w.nsamp[sid], node = w.node[sid];
-        tab.tmin[tid] = tmin;
-        tab.tmax[tid] = tmax;
-        tab.step[tid] = __fdiv_rn(__fsub_rn(tmax, tmin), (float)n);  // sample_t's step
-        tab.acc[tid] = want_dI ? p.grad_image[w.ray[sid]] : 0.0f;
-        tab.first[tid] = p.xt ? (int)(w.ray_sample_offset[w.ray[sid]] + w.first[sid]) : 0;
-        const int r = w.ray[sid];
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            tab.org[k][tid] = p.origin[3 * r + k];
-            tab.dir[k][tid] = p.dir[3 * r + k];
-        }
-        const uint64_t key = p.seed ? jitter_key(p.seed, r) : 0ull;
-        tab.key_lo[tid] = (unsigned)key;
-        tab.key_hi[tid] = (unsigned)(key >> 32);
-        if (per_item > 0) {
-            const int64_t sl = seg_slot(p.field, p.tree.num_nodes, node);
-            const int v = sl < p.field.num_slots ? (int)sl : -1;
-            if (p.xt)
-                tab.key_lo[tid] = (unsigned)v;
-            else
-                tab.first[tid] = v;
-        }
-        if (tid == 0 && per_item == 0) {  // the item's leaf (segment 0's; other leaves read the tree)
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                const float mn = p.tree.node_position_min[3 * node + k], mx = p.tree.node_position_max[3 * node + k];
-                const float sz = __fsub_rn(mx, mn);
-                tab.box[k] = mn;
-                tab.box[3 + k] = sz;
-                tab.box[6 + k] = pow2_reciprocal(sz);
-            }
-            reinterpret_cast<int*>(tab.box)[9] = node;
-        }
-    }
+    return info;
+}
+
+// Sample offsets of the item's segments, their total and the sample -> segment map.
+__device__ __forceinline__ void scan_item(const SegTab& tab, ItemInfo& info, int map_cap)
+{
+    const int tid = threadIdx.x;
     __syncthreads();
     if (tid < 32) {
         // exclusive scan of the sample counts (kSegItem = 128: four per lane)
@@ -507,6 +514,74 @@ __device__ __forceinline__ ItemInfo next_item(const FusedParams& p, int queue, f
         for (int k = b; k < e; ++k) tab.map[k] = (unsigned char)tid;
     }
     __syncthreads();
+}
+
+
+// by_item (kernels that keep no per-slot state between items): work is handed
+// out by item from the item queue (the slot queue's order, each slot's items
+// in a row), so the items of a large slot spread over several CTAs; a CTA
+// stages a slot's planes when its next item is of another slot. bar null: the
+// kernel reads the planes from global memory, nothing is staged.
+// per_item > 0 (kernels that keep no per-slot state and read the planes from
+// global memory): items are runs of per_item segments of the bucketed list,
+// whatever slots they fall in (item_slot; box unused), so every item but the
+// last has the same number of segments and the tiles are full also where the
+// slots have few. bar is unused then, and the returned slot is 0.
+__device__ __forceinline__ ItemInfo next_item(const FusedParams& p, int queue, float* sm, SegTab tab, uint64_t* bar,
+                                              int* s_ctl, bool want_dI, int map_cap = kSegMapCap,
+                                              bool by_item = false, int per_item = 0)
+{
+    const Ws& w = p.ws;
+    const int tid = threadIdx.x;
+    if (tid < 32) {
+        if (tid == 0 && per_item > 0) {
+            const int64_t total = min(w.totals[0], w.cap);
+            const int64_t at = (int64_t)atomicAdd(&w.counters[queue], 1) * per_item;
+            s_ctl[0] = at < total ? 0 : -1;
+            s_ctl[1] = (int)at;
+            s_ctl[2] = (int)min((int64_t)per_item, total - at);
+            s_ctl[3] = 0;
+        } else if (tid == 0 && by_item) {
+            int slot = -1, b0 = 0, nseg = 0, flags = 0;
+            const int q = atomicAdd(&w.counters[queue], 1);
+            if (q < w.counters[4]) {
+                const int2 e = w.item_queue[q];
+                slot = e.x;
+                const int nit = w.item_offset[slot + 1] - w.item_offset[slot];
+                if (slot != s_ctl[4]) {
+                    s_ctl[4] = slot;
+                    flags |= 1;
+                    if (slot < w.nslot && bar) {
+                        expect_planes(p, bar);
+                        flags |= 4;
+                    }
+                }
+                const int cnt = w.slot_offset[slot + 1] - w.slot_offset[slot];
+                const int per = (cnt + nit - 1) / nit;
+                b0 = w.slot_offset[slot] + e.y * per;
+                nseg = min(b0 + per, w.slot_offset[slot + 1]) - b0;
+                if (e.y == nit - 1) flags |= 2;
+                s_ctl[7] = nit;
+            }
+            s_ctl[0] = slot;
+            s_ctl[1] = b0;
+            s_ctl[2] = nseg;
+            s_ctl[3] = flags;
+        } else if (tid == 0) {
+            const int flags = pop_item(w, queue, s_ctl);
+            s_ctl[3] = flags;
+            if (flags & 4) expect_planes(p, bar);  // warp 0 issues the slot's plane copies below
+        }
+        __syncwarp();
+        if (s_ctl[3] & 4) stage_planes(p, sm, s_ctl[4], bar);
+    }
+    __syncthreads();
+    ItemInfo info = item_info(s_ctl);
+    if (info.slot < 0) return info;
+    const int b0 = s_ctl[1];
+    if (tid < info.nseg) store_row(p, tab, tid, load_row(p, b0 + tid, want_dI), per_item > 0);
+    if (per_item == 0) store_box(tab, tid, load_box(p, tid, b0));
+    scan_item(tab, info, map_cap);
     return info;
 }
 

@@ -332,7 +332,7 @@ __global__ void __launch_bounds__(kThreads, 3) forward_kernel(FusedParams p)
     using K = Cfg<C, MODE, H, NH>;
     using S = Smem<C, MODE, H, NH, false>;
     extern __shared__ __align__(16) float sm[];
-    __shared__ int s_ctl[8];
+    __shared__ int s_ctl[10];
     const int tid = threadIdx.x;
     int rg, cg, cw;
     tile_place<K>(rg, cg, cw);
@@ -401,7 +401,7 @@ __global__ void __launch_bounds__(kThreads, NH == 1 ? 3 : 2) backward_kernel(Fus
     using S = Smem<C, MODE, H, NH, true>;
     constexpr int T = K::T, F = K::F;
     extern __shared__ __align__(16) float sm[];
-    __shared__ int s_ctl[8];
+    __shared__ int s_ctl[10];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     int rg, cg, cw;
     tile_place<K>(rg, cg, cw);

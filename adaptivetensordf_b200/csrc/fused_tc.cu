@@ -253,7 +253,7 @@ __global__ void __launch_bounds__(RUNS ? kRows : kThreadsTC, RUNS ? 4 : 2) tc_fo
     __shared__ __align__(8) uint64_t bar_tma;
     __shared__ __align__(8) uint64_t bar_mma[2];
     __shared__ uint32_t s_tmem;
-    __shared__ int s_ctl[8];
+    __shared__ int s_ctl[10];
     constexpr int kHalves = RUNS ? 1 : 2;
     constexpr uint32_t tmem_cols = kTmemFwd / 2 * kHalves;
     const TCSmem L = RUNS ? TCSmem() : TCSmem(p.plane_off[3], p.gplane_off[3], false);
@@ -466,7 +466,7 @@ __global__ void __launch_bounds__(kThreadsB2, 1) tc_backward2_kernel(FusedParams
     __shared__ __align__(8) uint64_t bar_tma;
     __shared__ __align__(8) uint64_t bar_mma[2];
     __shared__ uint32_t s_tmem;
-    __shared__ int s_ctl[8];
+    __shared__ int s_ctl[10];
     __shared__ int s_lo[3];
     __shared__ float s_z[2][2][kRows];  // partial last-layer sums [half][group][row]
     // fixed-point plane-gradient accumulation of the current slot
@@ -518,9 +518,35 @@ __global__ void __launch_bounds__(kThreadsB2, 1) tc_backward2_kernel(FusedParams
     const int crot = 2 * (lane & 7) + ((lane >> 3) & 1) + 2 * (lane >> 4);
     float scale = 0.f;  // the slot's fixed-point scale
     int ntiles = 0;     // tiles of this half in the slot
+    // Half 1 has as many tiles of an item as half 0 or one fewer; its first group
+    // fetches the next item (a chain of queue, slot, bucket, segment and ray
+    // loads) into registers before it waits for half 0. Taken by the whole CTA
+    // between items that chain was 12.4k of an item's 155k clocks.
+    const bool fetcher = h == 1 && grp == 0;
+    SegRow row;
+    BoxLane box;
+    auto fetch = [&]() {
+        if (t == 0) s_ctl[3] = pop_item(p.ws, 1, s_ctl);
+        asm volatile("bar.sync 12, 128;" ::: "memory");
+        if (s_ctl[0] < 0) return;
+        if (t < s_ctl[2]) row = load_row(p, s_ctl[1] + t, true);
+        box = load_box(p, t, s_ctl[1]);
+    };
+    if (fetcher) fetch();
+    __syncthreads();
     while (alive) {
-        const ItemInfo it = next_item(p, 1, reinterpret_cast<float*>(sm), tab, &bar_tma, s_ctl, true);
+        ItemInfo it = item_info(s_ctl);
         if (it.slot < 0) break;
+        if (tid < 32 && (s_ctl[3] & 4)) {
+            if (tid == 0) expect_planes(p, &bar_tma);
+            __syncwarp();
+            stage_planes(p, reinterpret_cast<float*>(sm), it.slot, &bar_tma);
+        }
+        if (fetcher) {
+            if (t < it.nseg) store_row(p, tab, t, row, false);
+            store_box(tab, t, box);
+        }
+        scan_item(tab, it, kSegMapCap);
         const bool real = it.slot < p.ws.nslot;
         if (real && it.first) {
             for (int i = tid * 4; i < gplane_elems; i += kThreadsB2 * 4)
@@ -908,6 +934,7 @@ __global__ void __launch_bounds__(kThreadsB2, 1) tc_backward2_kernel(FusedParams
             tc::fence_before_sync();
             half_barrier2(h);
         }
+        if (fetcher) fetch();
         alive = __syncthreads_and(alive);
         if (real && it.last) {
             // this CTA owns the slot: plain stores, unless a tile went to

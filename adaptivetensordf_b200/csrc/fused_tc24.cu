@@ -271,7 +271,7 @@ __global__ void __launch_bounds__(RUNS ? kRows : kThreadsF, RUNS ? 4 : 2) tc24_f
     __shared__ __align__(8) uint64_t bar_tma;
     __shared__ __align__(8) uint64_t bar_mma[2];
     __shared__ uint32_t s_tmem;
-    __shared__ int s_ctl[8];
+    __shared__ int s_ctl[10];
     __shared__ int s_lo[3];
     constexpr int kHalves = RUNS ? 1 : 2;
     constexpr uint32_t tmem_cols = kTmemF / 2 * kHalves;
@@ -460,7 +460,7 @@ __global__ void __launch_bounds__(kThreadsB, 1) tc24_backward_kernel(FusedParams
     __shared__ __align__(8) uint64_t bar_tma;
     __shared__ __align__(8) uint64_t bar_mma;
     __shared__ uint32_t s_tmem;
-    __shared__ int s_ctl[8];
+    __shared__ int s_ctl[10];
     __shared__ int s_lo[3];
     __shared__ float s_z[2][kRows];  // partial last-layer sums [group 0 / 1][row]
     // the next tile's sample states, computed by group 2 while groups 0 and 1
