@@ -451,15 +451,6 @@ __device__ __forceinline__ bool tile_features_half(const FusedParams& p, unsigne
     return valid;
 }
 
-// Scratch float j (0..47) of sample t: HB columns 48..79 for j < 16, G
-// columns 64..127 (free once the dX and dW MMAs have read them) for the rest.
-__device__ __forceinline__ float* scratch2(unsigned char* hbh, unsigned char* gh, int t, int j)
-{
-    if (j < 16) return reinterpret_cast<float*>(hbh + hb_off(t, 48 + 8 * (j >> 2)) + (j & 3) * 4);
-    const int q = j - 16;
-    return reinterpret_cast<float*>(gh + g_off(t, 64 + 8 * (q >> 2)) + (q & 3) * 4);
-}
-
 __global__ void __launch_bounds__(kThreadsB2, 1) tc_backward2_kernel(FusedParams p)
 {
     extern __shared__ __align__(128) unsigned char sm[];
@@ -515,7 +506,6 @@ __global__ void __launch_bounds__(kThreadsB2, 1) tc_backward2_kernel(FusedParams
     uint32_t tma_phase = 0, mma_phase = 0;
     bool alive = true, had_tile = false;
     float gw2 = 0.f, gb2 = 0.f;  // lane owns one last-layer column of its group
-    const int crot = 2 * (lane & 7) + ((lane >> 3) & 1) + 2 * (lane >> 4);
     float scale = 0.f;  // the slot's fixed-point scale
     int ntiles = 0;     // tiles of this half in the slot
     // Half 1 has as many tiles of an item as half 0 or one fewer; its first group
@@ -764,8 +754,8 @@ __global__ void __launch_bounds__(kThreadsB2, 1) tc_backward2_kernel(FusedParams
             }
             had_tile = true;
             alive = wait_mma(&bar_mma[h], mma_phase, p.err) && alive;
-            // scatter, phase 1 (own channels): dX * line values into the
-            // scratch row, dX * plane values as the line MMA's B operand, and
+            // scatter, phase 1 (own channels): dX * line values, kept in
+            // registers; dX * plane values as the line MMA's B operand, and
             // (group 0) the tap column of the line MMA's A operand
             float dx[8];
             uint32_t pk[3][4];  // BF16 bilinear plane values kept by the feature step
@@ -780,12 +770,13 @@ __global__ void __launch_bounds__(kThreadsB2, 1) tc_backward2_kernel(FusedParams
 #pragma unroll
                     for (int q = 0; q < 8; ++q) *reinterpret_cast<uint4*>(gh + g_off(t, 8 * q)) = z4;
                 }
+                float gv[3][8];    // dX * line value
                 float tsum = 0.f;  // sum of |dX * line value| of this thread's 24 values
                 if (valid) {
 #pragma unroll
                     for (int m = 0; m < 3; ++m) {
                         const int Ln = p.field.line_len[m];
-                        float mat[8], vec[8], lv[8], gv[8];
+                        float mat[8], vec[8], lv[8];
 #pragma unroll
                         for (int i = 0; i < 4; ++i) {
                             const float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&pk[m][i]));
@@ -795,13 +786,9 @@ __global__ void __launch_bounds__(kThreadsB2, 1) tc_backward2_kernel(FusedParams
                         line_half(p, g, m, cb, vec);
 #pragma unroll
                         for (int c = 0; c < 8; ++c) {
-                            gv[c] = dx[c] * vec[c];
-                            tsum += fabsf(gv[c]);
+                            gv[m][c] = dx[c] * vec[c];
+                            tsum += fabsf(gv[m][c]);
                         }
-#pragma unroll
-                        for (int q = 0; q < 2; ++q)
-                            *reinterpret_cast<float4*>(scratch2(hbh, gh, t, 16 * m + cb + 4 * q)) =
-                                make_float4(gv[4 * q], gv[4 * q + 1], gv[4 * q + 2], gv[4 * q + 3]);
 #pragma unroll
                         for (int c = 0; c < 8; ++c) lv[c] = dx[c] * mat[c];
                         store_bf16x8(hbh + hb_off(t, 16 * m + cb), lv);
@@ -873,45 +860,63 @@ __global__ void __launch_bounds__(kThreadsB2, 1) tc_backward2_kernel(FusedParams
                     }
                     tc::commit(&bar_mma[h]);
                 }
-                // scatter, phase 2: plane gradients as fixed-point integers
-                // (shared-memory integer atomics run several times faster than
-                // FP32 ones); group 0 adds the two upper corners, group 1 the
-                // two lower ones. A texel's 16 channels fill one half of the
-                // 32 banks (the half given by the parity of its index), and the two corners of a row have
-                // opposite parities: lanes 0-15 take first the corner in banks
-                // 0-15, lanes 16-31 the one in banks 16-31, and channel
-                // (r + crot) mod 16 with crot a permutation of 0..15 within
-                // each half-warp, so every warp-wide atomic touches 32 distinct
-                // banks. crot mod 4 also differs among the four lanes that share
-                // lane mod 8, which keeps the scratch-row reads conflict-free.
-                if (valid) {
-#pragma unroll 1
+                // scatter, phase 2: the group's 8 channels to the four
+                // corners, as fixed-point integers (shared-memory integer
+                // atomics run several times faster than FP32 ones). A warp's
+                // rows are consecutive samples of a ray, several in one cell:
+                // lane l takes the corners from (l mod 4) on and the channels
+                // from (l / 4 mod 8) on, so up to 32 lanes in one cell add to
+                // 32 different words at each step. The products never leave
+                // the registers: with each group adding all 16 channels to two
+                // corners they went through 48 shared floats a row (step of
+                // 16384 rays at depth 4: 2928 us, 2895 fully unrolled, now
+                // 2785). Gradient rows padded by 8 words, 32 distinct banks as
+                // well: 2766, not worth another layout.
+                if (valid && to_smem) {
+                    const int crot = (lane >> 2) & 7;
+#pragma unroll
                     for (int m = 0; m < 3; ++m) {
                         const int Hm = p.field.plane_h[m], Wm = p.field.plane_w[m];
                         const Corner2 kc = corners2(g.pu[m], g.pv[m], Hm, Wm);
-                        const int ya = grp == 0 ? kc.y0 : kc.y1;
-                        const float wl = grp == 0 ? kc.w_nw : kc.w_sw, wr = grp == 0 ? kc.w_ne : kc.w_se;
-                        const int tl = ya * Wm + kc.x0, tr = ya * Wm + kc.x1;
-                        const bool swap = (tl & 1) != (lane >> 4);
-                        const int ta = (swap ? tr : tl) * C, tb = (swap ? tl : tr) * C;
-                        const float wa = swap ? wr : wl, wb = swap ? wl : wr;
-                        if (to_smem) {
-                            int* GP = gpl + p.gplane_off[m];
-                            const float was = wa * scale, wbs = wb * scale;
-#pragma unroll 4
-                            for (int r = 0; r < kC; ++r) {
-                                const int c = (r + crot) & (kC - 1);
-                                const float v = *scratch2(hbh, gh, t, 16 * m + c);
-                                atomicAdd(&GP[ta + c], __float2int_rn(was * v));
-                                atomicAdd(&GP[tb + c], __float2int_rn(wbs * v));
-                            }
-                        } else {
-                            float* GG = p.gfield.plane[m] + it.slot * (int64_t)(Hm * Wm * C);
-                            for (int r = 0; r < kC; ++r) {
-                                const float v = *scratch2(hbh, gh, t, 16 * m + r);
-                                atomicAdd(&GG[ta + r], wa * v);
-                                atomicAdd(&GG[tb + r], wb * v);
-                            }
+                        // gr[i] = gv[m][(i + crot) mod 8] (a three-stage rotation)
+                        float gr[8];
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) gr[i] = gv[m][i];
+#pragma unroll
+                        for (int b = 0; b < 3; ++b) {
+                            const bool on = (crot >> b) & 1;
+                            float nx[8];
+#pragma unroll
+                            for (int i = 0; i < 8; ++i) nx[i] = on ? gr[(i + (1 << b)) & 7] : gr[i];
+#pragma unroll
+                            for (int i = 0; i < 8; ++i) gr[i] = nx[i];
+                        }
+                        int* GP = gpl + p.gplane_off[m] + cb;
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            float wj;
+                            const int tx = corner_texel(kc, (j + lane) & 3, Wm, wj) * C;
+                            const float ws = wj * scale;
+#pragma unroll
+                            for (int i = 0; i < 8; ++i)
+                                atomicAdd(&GP[tx + ((i + crot) & 7)], __float2int_rn(ws * gr[i]));
+                        }
+                    }
+                }
+                // a tile beyond the fixed-point range: FP32 atomics to the
+                // slot's global gradient (rare; kept out of the unrolled code)
+                if (valid && !to_smem) {
+#pragma unroll
+                    for (int m = 0; m < 3; ++m) {
+                        const int Hm = p.field.plane_h[m], Wm = p.field.plane_w[m];
+                        const Corner2 kc = corners2(g.pu[m], g.pv[m], Hm, Wm);
+                        float* GG = p.gfield.plane[m] + it.slot * (int64_t)(Hm * Wm * C);
+#pragma unroll 1
+                        for (int j = 0; j < 4; ++j) {
+                            float wj;
+                            const int tx = corner_texel(kc, j, Wm, wj) * C;
+#pragma unroll
+                            for (int i = 0; i < 8; ++i) atomicAdd(&GG[tx + cb + i], wj * gv[m][i]);
                         }
                     }
                 }
