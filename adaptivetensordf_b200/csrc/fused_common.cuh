@@ -231,46 +231,15 @@ __device__ __forceinline__ SegTab seg_tab(float* base)
     return t;
 }
 
-// Takes the next work item; fills the segment table; issues the plane TMA
-// when the item starts a new slot. Returns the item's slot, or -1 when the
-// queue is empty. Items of up to map_cap (<= kSegMapCap) samples get the
-// sample -> segment byte map, larger ones a binary search.
-// sample_state(permute = true) visits a work item's samples in the order
-// k -> k * 104729 mod total (a permutation: the prime exceeds any item's
-// sample count). Consecutive samples, which share a warp, then come from
-// different rays and depths in the leaf and touch different texels, so their
-// shared-memory atomics do not collide the way the samples along one ray
-// would. The FP32 kernels and the 16-channel tensor-core backward use it; the
-// tensor-core forwards and the 24-channel backward visit samples in order
-// (gathers along a ray share texels; that backward rotates its atomics
-// instead).
-constexpr int kSamplePermPrime = 104729;
-
 struct ItemInfo {
     int64_t slot;
     int nseg;
     int total;
-    double inv_total;  // 1 / total (for the sample permutation)
     bool first;        // first item of its slot: the slot's planes were just requested
     bool last;         // last item of its slot
     int slot_items;    // work items of the slot
     bool use_map;      // total <= kSegMapCap: the table's map gives each sample's segment
 };
-
-// (k * kSamplePermPrime) mod total without a 64-bit integer division: the
-// product is below 2^34 and exact in double, the quotient estimate from the
-// reciprocal is off by at most one, and q * total and the remainder are exact.
-__device__ __forceinline__ int perm_index(int k, int total, double inv_total)
-{
-    const double kp = (double)k * (double)kSamplePermPrime;
-    const double q = floor(kp * inv_total);
-    double r = kp - q * (double)total;
-    if (r < 0.0)
-        r += (double)total;
-    else if (r >= (double)total)
-        r -= (double)total;
-    return (int)r;
-}
 
 // Plane slot of segment si of an item taken by segments (-1 outside the ROI),
 // in the array that its kind of samples leaves free.
@@ -469,7 +438,6 @@ __device__ __forceinline__ ItemInfo item_info(const int* s_ctl)
     info.last = (s_ctl[3] & 2) != 0;
     info.slot_items = s_ctl[7];
     info.total = 0;
-    info.inv_total = 0.0;
     info.use_map = false;
     return info;
 }
@@ -505,7 +473,6 @@ __device__ __forceinline__ void scan_item(const SegTab& tab, ItemInfo& info, int
     }
     __syncthreads();
     info.total = tab.start[info.nseg];
-    info.inv_total = info.total > 0 ? 1.0 / (double)info.total : 0.0;
     // sample -> segment map (one byte per sample), in place of a binary
     // search of the count scan per sample
     info.use_map = info.total <= map_cap;
@@ -517,6 +484,10 @@ __device__ __forceinline__ void scan_item(const SegTab& tab, ItemInfo& info, int
 }
 
 
+// Takes the next work item; fills the segment table; issues the plane TMA
+// when the item starts a new slot. Returns the item's slot, or -1 when the
+// queue is empty. Items of up to map_cap (<= kSegMapCap) samples get the
+// sample -> segment byte map, larger ones a binary search.
 // by_item (kernels that keep no per-slot state between items): work is handed
 // out by item from the item queue (the slot queue's order, each slot's items
 // in a row), so the items of a large slot spread over several CTAs; a CTA
@@ -617,16 +588,14 @@ __device__ __forceinline__ float sample_t_step(float tmin, float step, int j, fl
     return __fadd_rn(__fmul_rn(t1, oma), __fmul_rn(t2, a));
 }
 
-// permute: visit the item's samples in the permuted order (kernels that
-// scatter with shared-memory atomics); without it sample k is the item's k-th
-// (consecutive rows walk along a ray, so their gathers share texels).
+// Sample k of the item (consecutive rows walk along a ray, so their gathers
+// share texels).
 __device__ __forceinline__ SampleState sample_state(const FusedParams& p, const SegTab& tab, const ItemInfo& it,
-                                                    int k, bool permute = true)
+                                                    int k)
 {
     SampleState s;
-    const int kk = permute && it.total < kSamplePermPrime ? perm_index(k, it.total, it.inv_total) : k;
-    s.si = it.use_map ? (int)tab.map[kk] : find_seg(tab, it.nseg, kk);
-    const int j = kk - tab.start[s.si];
+    s.si = it.use_map ? (int)tab.map[k] : find_seg(tab, it.nseg, k);
+    const int j = k - tab.start[s.si];
     const int n = tab.n[s.si];
     s.node = tab.node[s.si];
     const float tmin = tab.tmin[s.si], tmax = tab.tmax[s.si], step = tab.step[s.si];

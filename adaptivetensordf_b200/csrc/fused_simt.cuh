@@ -264,7 +264,7 @@ __device__ __forceinline__ void geometry_pass(const FusedParams& p, const SegTab
 {
     const int s = threadIdx.x, k = t0 + s;
     if (k < it.total) {
-        const SampleState st = sample_state(p, tab, it, k, false);
+        const SampleState st = sample_state(p, tab, it, k);
         const SampleGeo g = sample_geo_fast(p, &tab, st.node, st.pos);
         store_geo(geo, s, g, dI ? __fmul_rn(tab.acc[st.si], st.w) : st.w);
         si[s] = st.si;

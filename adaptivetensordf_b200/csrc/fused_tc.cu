@@ -209,7 +209,7 @@ __device__ __forceinline__ bool tile_features(const FusedParams& p, unsigned cha
     ts = 0.0f;
     si = -1;
     if (valid) {
-        const SampleState st = sample_state(p, tab, it, k, false);
+        const SampleState st = sample_state(p, tab, it, k);
         w = st.w;
         ts = st.t;
         si = st.si;
@@ -428,7 +428,7 @@ __device__ __forceinline__ bool tile_features_half(const FusedParams& p, unsigne
     w = 0.0f;
     si = -1;
     if (valid) {
-        const SampleState st = sample_state(p, tab, it, k, false);
+        const SampleState st = sample_state(p, tab, it, k);
         w = st.w;
         si = st.si;
         if (real) {

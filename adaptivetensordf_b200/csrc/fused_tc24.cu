@@ -323,7 +323,7 @@ __global__ void __launch_bounds__(RUNS ? kRows : kThreadsF, RUNS ? 4 : 2) tc24_f
             float w = 0.0f, ts = 0.0f;
             int si = -1;
             if (valid) {
-                const SampleState st = sample_state(p, tab, it, k, false);
+                const SampleState st = sample_state(p, tab, it, k);
                 w = st.w;
                 ts = st.t;
                 si = st.si;
@@ -572,7 +572,7 @@ __global__ void __launch_bounds__(kThreadsB, 1) tc24_backward_kernel(FusedParams
                     }
                 }
             } else if (valid) {
-                const SampleState st = sample_state(p, tab, it, k, false);
+                const SampleState st = sample_state(p, tab, it, k);
                 w = st.w;
                 si = st.si;
                 if (real) {
@@ -705,7 +705,7 @@ __global__ void __launch_bounds__(kThreadsB, 1) tc24_backward_kernel(FusedParams
                 int si2 = -1;
                 float w2 = 0.0f;
                 if (k2 < it.total) {
-                    const SampleState st = sample_state(p, tab, it, k2, false);
+                    const SampleState st = sample_state(p, tab, it, k2);
                     si2 = st.si;
                     w2 = st.w;
 #pragma unroll

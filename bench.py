@@ -812,10 +812,10 @@ def run_ours(args, rank, world):
     # the same for the C5 rank-24 backward (full-size capture, 3 launches)
     roof5["traffic"] = 177041835 + 283314176 if R == 16384 else None
     roof5["traffic_source"] = "profiles/launches_c5_bf16_16384rays.md" if R == 16384 else None
-    # this library's kernels per uniform training step of the BF16 form: 12
-    # for sampling, bucketing (slot order, item queue) and the forward, the
-    # loss, 2 for the backward and one Adam launch for the 12 parameters
-    launches_per_step = 16
+    # this library's kernels per uniform training step of the BF16 form: 2 for
+    # the segments, 3 for bucketing, the forward, the ray sums, the loss, 2 for
+    # the backward and one Adam launch for the 12 parameters
+    launches_per_step = 11
     h2d = sum(t.numel() * t.element_size() for t in make_host_shapes(R))
     line = {
         "metric": METRIC,
