@@ -296,6 +296,10 @@ __device__ __forceinline__ void decode_tile(float* sm, int rg, int cg, int cw, i
     const int tid = threadIdx.x;
                     uint64_t acc[8][4];
                     layer0<C, MODE, H, NH, false>(sm, rg, cg, acc);
+                    // every warp has read all rows of x before any of them
+                    // gathers the geometry pass's next tile into it (two
+                    // hidden layers: the barrier after H0)
+                    if (NH == 1 && K::T < kGeo) __syncthreads();
                     if (NH == 2) {
     #pragma unroll
                         for (int j = 0; j < 4; ++j) {

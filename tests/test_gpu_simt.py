@@ -68,3 +68,53 @@ def test_tile_edges(oracle, hidden, n):
 def test_other_activations(oracle, activation):
     tree, geo, o, d = gpu_scene(2, 8, 9, (32, 9, 32), [64, 64], 200, seed=21, activation=activation)
     _check(oracle, tree, geo, o, d, 9, 0)
+
+
+@pytest.mark.parametrize("C", [8, 16])
+@pytest.mark.parametrize("n", [65, 127, 128, 129, 257])
+def test_tile_edges_one_wide_layer(oracle, C, n):
+    """As test_tile_edges for one hidden layer of 64 units: two tiles of 64
+    samples share a geometry pass and the feature tile."""
+    tree, geo, _, _ = gpu_scene(0, C, 17, (40, 17, 33), [64], 1, seed=n)
+    o, d = np.array([[0.13, -0.37, -2.0]], np.float32), np.array([[0.0, 0.0, 1.0]], np.float32)
+    assert _check(oracle, tree, geo, o, d, int(np.floor(n * np.sqrt(3.0))), 5) == n
+
+
+# Largest error of one value of the FP32 form: its features, 80 products and
+# sums and the activations at a few ulp each (2^-24 of the largest terms), far
+# below a feature row taken from another sample.
+MAX_TOL = 1e-4
+
+
+@pytest.mark.parametrize("C", [8, 16])
+def test_tiles_of_a_pass_keep_their_features(oracle, C):
+    """One hidden layer of 64 units on every SM, several times: density at
+    points where every second tile is outside the ROI (no texels to wait for,
+    so its warps run ahead) and the projection, each value against the FP64
+    oracle."""
+    import adaptivetensordf_b200 as ab
+
+    n = 128 * 148 * 6 + 77
+    tree, geo, o, d = gpu_scene(1, C, 17, (33, 17, 33), [64], 3000, seed=C)
+    slot = geo.leaf_slot.clone()
+    slot[tree.active_node_ids[0]] = -1
+    geo.leaf_slot = slot
+    td, fd, md = oracle_views(tree, geo)
+    rng = np.random.default_rng(C)
+    pts = rng.uniform(0.0, 1.0, (n, 3)).astype(np.float32)
+    outside = np.arange(n) // 64 % 2 == 1
+    pts[outside] -= 1.0  # the lowest leaf
+    pt = torch.from_numpy(pts).cuda()
+    node, _ = tree.NodeIdForPositionGPU(pt)
+    so = {"global_coordinate": pts, "node_id": node.cpu().numpy(), "weight": np.ones(n, np.float32),
+          "ray_index": np.arange(n)}
+    ref = oracle.project_forward(fd, md, td, so, n, np.float64).reshape(n)
+    segs = oracle.ray_segments(td, o, d, 300)
+    ref_img = oracle.project_forward(fd, md, td, oracle.emit_samples(segs, o, d, None), len(o), np.float64).reshape(-1)
+    rays = ab.RayList(torch.from_numpy(o).cuda(), torch.from_numpy(d).cuda())
+    for _ in range(5):
+        with torch.no_grad():
+            got = geo.SampleVolumeIndirect(tree, pt, node).cpu().numpy().reshape(n)
+            img = geo.ProjectRays(tree, rays, 300, 0).cpu().numpy().reshape(-1)
+        assert np.abs(got - ref).max() < MAX_TOL * np.abs(ref).max()
+        assert np.abs(img - ref_img).max() < MAX_TOL * np.abs(ref_img).max()
