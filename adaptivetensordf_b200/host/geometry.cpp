@@ -368,8 +368,11 @@ static DecoderInputs decoder_inputs(const Decoder& dec)
     DecoderInputs t;
     t.fill(dec.bias[0].detach());
     for (size_t l = 0; l < dec.weight.size(); ++l) {
-        t[2 * l] = dec.weight[l];
-        t[2 * l + 1] = dec.bias[l];
+        // the gradients come back as [out, in] and [out]: parameters of another
+        // rank ([out, in, 1, 1], [1, out], a scalar bias) go through a view
+        const Tensor &w = dec.weight[l], &b = dec.bias[l];
+        t[2 * l] = w.dim() == 2 ? w : w.reshape({w.size(0), -1});
+        t[2 * l + 1] = b.dim() == 1 ? b : b.reshape({-1});
     }
     return t;
 }

@@ -198,3 +198,29 @@ def test_density_without_gradients(oracle, C, hidden, op, n):
     node[0] = tree.NumNodes()
     with torch.no_grad(), pytest.raises(RuntimeError, match="index out of range"):
         geo.SampleVolumeIndirect(tree, torch.from_numpy(pts).cuda(), node)
+
+
+def test_decoder_parameters_of_another_rank():
+    """Weights [out, in, 1, 1], biases [1, out] and a scalar last bias give
+    what [out, in] and [out] give, and gradients of their own shapes."""
+    import adaptivetensordf_b200 as ab
+
+    tree, geo, o, d = gpu_scene(2, 8, 9, (32, 9, 32), [32], 300, seed=3)
+    rays = ab.RayList(torch.from_numpy(o).cuda(), torch.from_numpy(d).cuda())
+    x = torch.randn(77, 8, generator=torch.Generator().manual_seed(1)).cuda()
+    w, b = [t.detach() for t in geo.decoder_weight], [t.detach() for t in geo.decoder_bias]
+    other = ([t[:, :, None, None] for t in w], [b[0][None], b[1].reshape([])])
+    res = []
+    for ws, bs in ((w, b), other):
+        ws, bs = ([t.clone().requires_grad_(True) for t in v] for v in (ws, bs))
+        y = ab.DecodeFeatures(ws, bs, "silu", "softplus", 1.0, x)
+        geo.decoder_weight, geo.decoder_bias = ws, bs
+        img = geo.ProjectRays(tree, rays, 9, 0)
+        out = [y, img]
+        for v in (y, img):
+            gs = torch.autograd.grad(v, ws + bs, torch.ones_like(v))
+            assert [g.shape for g in gs] == [p.shape for p in ws + bs]
+            out += gs
+        res.append([v.detach().cpu().numpy().reshape(-1) for v in out])
+    for got, want in zip(res[1], res[0]):
+        assert rel_err(got, want) < REL_TOL
