@@ -52,25 +52,24 @@ int activation_id(const std::string& a)
 // (1 M samples on 1.2 M texels of 16 channels: forward 252 -> 85 us, adjoint
 // 771 -> 207 us with the copies of 40 us each; below one sample per 4 texels
 // the copies cost more than they save).
+static bool aligned(const Tensor& t) { return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0; }
+
 static bool samples_in_channels_last(const Tensor& grid, int64_t samples)
 {
     const int64_t texels = grid.size(0) * grid.size(2) * grid.size(3);
     return grid.size(1) % 4 == 0 && grid.numel() > 0 &&
-           (grid.is_contiguous(torch::MemoryFormat::ChannelsLast) || 4 * samples >= texels);
+           ((grid.is_contiguous(torch::MemoryFormat::ChannelsLast) && aligned(grid)) || 4 * samples >= texels);
 }
 
-static Tensor aligned16(const Tensor& t)
-{
-    return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0 ? t : t.clone();
-}
+static Tensor aligned16(const Tensor& t) { return aligned(t) ? t : t.clone(); }
 
 // Dense NHWC storage, 16-byte aligned.
 static Tensor channels_last_copy(const Tensor& grid)
 {
     const int64_t C = grid.size(1), H = grid.size(2), W = grid.size(3);
-    const bool dense = grid.stride(1) == 1 && grid.stride(3) == C && grid.stride(2) == C * W &&
-                       grid.stride(0) == C * W * H;
-    if (dense) return aligned16(grid);
+    // a dimension of size 1 may have any stride: the dense one in its place
+    if (grid.is_contiguous(torch::MemoryFormat::ChannelsLast))
+        return aligned16(grid.as_strided(grid.sizes(), {C * W * H, 1, C * W, C}));
     if (grid.is_contiguous()) {
         auto out = torch::empty({grid.size(0), H, W, C}, grid.options());
         if (atdf_grid_layout(grid.data_ptr<float>(), grid.size(0), C, H * W, 1, out.data_ptr<float>(), stream_arg()) ==

@@ -224,3 +224,29 @@ def test_decoder_parameters_of_another_rank():
         res.append([v.detach().cpu().numpy().reshape(-1) for v in out])
     for got, want in zip(res[1], res[0]):
         assert rel_err(got, want) < REL_TOL
+
+
+@pytest.mark.parametrize("N,batch_stride", [(1, 8 * 9 * 6 + 5), (3, 8 * 9 * 6)])
+@pytest.mark.parametrize("S", [5, 700])
+@pytest.mark.parametrize("start", [0, 1])
+def test_grid_sample_unaligned_channels_last(oracle, N, batch_stride, S, start):
+    """Channels-last grids that start off a 16-byte boundary, and one slot
+    whose batch stride is any number (a dimension of one entry)."""
+    import adaptivetensordf_b200 as ab
+
+    C, H, W = 8, 9, 6
+    rng = np.random.default_rng(S + N)
+    g = rng.normal(size=(N, C, H, W)).astype(np.float32)
+    idx = rng.integers(0, N, S)
+    uv = rng.uniform(-1.2, 1.2, (S, 2)).astype(np.float32)
+    go = rng.normal(size=(S, C)).astype(np.float32)
+    gt = torch.zeros(start + N * batch_stride, device="cuda").as_strided(
+        (N, C, H, W), (batch_stride, 1, C * W, C), start)
+    gt = gt.copy_(torch.from_numpy(g)).detach().requires_grad_(True)
+    assert gt.is_contiguous(memory_format=torch.channels_last) and gt.data_ptr() % 16 == 4 * start
+    ut = torch.from_numpy(uv).cuda().requires_grad_(True)
+    out = ab.IndirectGridSample2D(gt, torch.from_numpy(idx).cuda(), ut)
+    assert np.array_equal(out.detach().cpu().numpy(), oracle.grid_sample2d(g, idx, uv, np.float32))
+    gg, gu = torch.autograd.grad(out, [gt, ut], torch.from_numpy(go).cuda())
+    assert rel_err(gg.cpu().numpy(), oracle.grid_sample2d_bwd(g, idx, uv, go, np.float64)[0]) < REL_TOL
+    assert np.array_equal(gu.cpu().numpy(), oracle.grid_sample2d_bwd(g, idx, uv, go, np.float32)[1])
