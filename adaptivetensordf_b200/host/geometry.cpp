@@ -79,14 +79,17 @@ static Tensor channels_last_copy(const Tensor& grid)
     return grid.permute({0, 2, 3, 1}).contiguous().permute({0, 3, 1, 2});
 }
 
-// A gradient in dense NHWC storage as contiguous [N, C, H, W].
-static Tensor contiguous_from_channels_last(const Tensor& t)
+// Runs the allocations of a path that trades memory for speed; false where they
+// do not fit, and the caller takes the path that needs none of them.
+template <class Alloc>
+static bool if_memory_allows(Alloc alloc)
 {
-    auto out = torch::empty(t.sizes(), t.options().memory_format(torch::MemoryFormat::Contiguous));
-    if (atdf_grid_layout(t.data_ptr<float>(), t.size(0), t.size(1), t.size(2) * t.size(3), 0, out.data_ptr<float>(),
-                         stream_arg()) == ATDF_OK)
-        return out;
-    return t.contiguous();
+    try {
+        alloc();
+        return true;
+    } catch (const c10::OutOfMemoryError&) {
+        return false;
+    }
 }
 
 class GridSample2DFn : public torch::autograd::Function<GridSample2DFn> {
@@ -104,7 +107,8 @@ class GridSample2DFn : public torch::autograd::Function<GridSample2DFn> {
         const int64_t S = idx.size(0), C = grid.size(1);
         auto out = torch::empty({S, C}, grid.options().memory_format(torch::MemoryFormat::Contiguous));
         auto grid_read = grid;
-        if (samples_in_channels_last(grid, S)) grid_read = channels_last_copy(grid);
+        if (samples_in_channels_last(grid, S))
+            if_memory_allows([&] { grid_read = channels_last_copy(grid); });
         int64_t st[4] = {grid_read.stride(0), grid_read.stride(1), grid_read.stride(2), grid_read.stride(3)};
         auto err = err_word(grid.device());
         check_status(atdf_grid_sample2d_forward(grid_read.data_ptr<float>(), grid.size(0), C, grid.size(2), grid.size(3), st,
@@ -126,16 +130,25 @@ class GridSample2DFn : public torch::autograd::Function<GridSample2DFn> {
         auto guv = torch::zeros_like(u);
         auto err = ctx->saved_data["err"].toTensor();
         if (samples_in_channels_last(grid, idx.size(0)) && idx.size(0) > 0) {
-            auto grid_read = channels_last_copy(grid);
-            auto ggrid = torch::zeros_like(grid_read);
-            g = aligned16(g);
-            check_status(atdf_grid_sample2d_backward_channels_last(
-                             grid_read.data_ptr<float>(), grid.size(0), grid.size(1), grid.size(2), grid.size(3),
-                             idx.data_ptr<int64_t>(), u.data_ptr<float>(), idx.size(0), g.data_ptr<float>(),
-                             ggrid.data_ptr<float>(), guv.data_ptr<float>(), err.data_ptr<int32_t>(), stream_arg()),
-                         "IndirectGridSample2D backward");
-            check_dev_error(err, "IndirectGridSample2D backward");
-            return {contiguous_from_channels_last(ggrid), Tensor(), guv};
+            Tensor grid_read, g_read, ggrid, out;
+            if (if_memory_allows([&] {
+                    grid_read = channels_last_copy(grid);
+                    g_read = aligned16(g);
+                    ggrid = torch::zeros_like(grid_read);
+                    out = torch::empty(grid.sizes(), grid.options().memory_format(torch::MemoryFormat::Contiguous));
+                })) {
+                check_status(atdf_grid_sample2d_backward_channels_last(
+                                 grid_read.data_ptr<float>(), grid.size(0), grid.size(1), grid.size(2), grid.size(3),
+                                 idx.data_ptr<int64_t>(), u.data_ptr<float>(), idx.size(0), g_read.data_ptr<float>(),
+                                 ggrid.data_ptr<float>(), guv.data_ptr<float>(), err.data_ptr<int32_t>(), stream_arg()),
+                             "IndirectGridSample2D backward");
+                check_dev_error(err, "IndirectGridSample2D backward");
+                if (atdf_grid_layout(ggrid.data_ptr<float>(), grid.size(0), grid.size(1), grid.size(2) * grid.size(3), 0,
+                                     out.data_ptr<float>(), stream_arg()) != ATDF_OK)
+                    out.copy_(ggrid);
+                return {out, Tensor(), guv};
+            }
+            grid_read = g_read = ggrid = out = Tensor();
         }
         auto ggrid = torch::zeros(grid.sizes(), grid.options().memory_format(torch::MemoryFormat::Contiguous));
         int64_t st[4] = {grid.stride(0), grid.stride(1), grid.stride(2), grid.stride(3)};
@@ -188,12 +201,15 @@ class GridSample1DFn : public torch::autograd::Function<GridSample1DFn> {
         const int64_t copies = std::min<int64_t>({64, S / std::max<int64_t>(8 * entries, 1),
                                                   (2 << 20) / std::max<int64_t>(grid.numel(), 1)});
         int st1 = ATDF_ERR_UNSUPPORTED;
-        if (copies >= 2) {
-            g = aligned16(g);
-            auto scratch = torch::empty({copies * grid.numel()}, grid.options().memory_format(torch::MemoryFormat::Contiguous));
+        Tensor g_read, scratch;
+        if (copies >= 2 && if_memory_allows([&] {
+                g_read = aligned16(g);
+                scratch = torch::empty({copies * grid.numel()},
+                                       grid.options().memory_format(torch::MemoryFormat::Contiguous));
+            })) {
             st1 = atdf_grid_sample1d_backward_copies(grid.data_ptr<float>(), grid.size(0), grid.size(1), grid.size(2),
                                                      st, idx.data_ptr<int64_t>(), u.data_ptr<float>(), S,
-                                                     g.data_ptr<float>(), ggrid.data_ptr<float>(),
+                                                     g_read.data_ptr<float>(), ggrid.data_ptr<float>(),
                                                      guv.data_ptr<float>(), scratch.data_ptr<float>(), (int32_t)copies,
                                                      err.data_ptr<int32_t>(), stream_arg());
         }

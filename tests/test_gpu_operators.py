@@ -250,3 +250,37 @@ def test_grid_sample_unaligned_channels_last(oracle, N, batch_stride, S, start):
     gg, gu = torch.autograd.grad(out, [gt, ut], torch.from_numpy(go).cuda())
     assert rel_err(gg.cpu().numpy(), oracle.grid_sample2d_bwd(g, idx, uv, go, np.float64)[0]) < REL_TOL
     assert np.array_equal(gu.cpu().numpy(), oracle.grid_sample2d_bwd(g, idx, uv, go, np.float32)[1])
+
+
+def test_grid_sample_without_memory_for_copies():
+    """The channels-last copies of a large grid are taken only where they fit:
+    with memory for no more than the results the operator reads the grid as it
+    is, with the same values."""
+    import adaptivetensordf_b200 as ab
+
+    N, C, H, W, S = 1024, 16, 64, 64, 1 << 20  # the grid: 256 MiB, a sample per 4 texels
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    grid = torch.randn(N, C, H, W, generator=gen, device="cuda").requires_grad_(True)
+    idx = torch.randint(0, N, (S,), generator=gen, device="cuda")
+    uv = (torch.rand(S, 2, generator=gen, device="cuda") * 2 - 1).requires_grad_(True)
+    go = torch.randn(S, C, generator=gen, device="cuda")
+    total = torch.cuda.get_device_properties(0).total_memory
+    res = []
+    for more in (None, (64 + 128, 256 + 64)):  # MiB beyond what is held: out and half a copy; the gradient and a quarter
+        out = None
+        try:
+            for step in range(2):
+                torch.cuda.synchronize()
+                torch.cuda.empty_cache()
+                if more:
+                    torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (more[step] << 20)) / total)
+                if step == 0:
+                    out = ab.IndirectGridSample2D(grid, idx, uv)
+                else:
+                    grads = torch.autograd.grad(out, [grid, uv], go)
+        finally:
+            torch.cuda.set_per_process_memory_fraction(1.0)
+        res.append([out.detach().cpu()] + [g.cpu() for g in grads])
+        del out, grads
+    assert torch.equal(res[0][0], res[1][0]) and torch.equal(res[0][2], res[1][2])
+    assert rel_err(res[1][1].numpy(), res[0][1].numpy()) < REL_TOL
