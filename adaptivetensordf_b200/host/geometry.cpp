@@ -757,13 +757,15 @@ static Tensor density_no_grad(GeometryTensorQO& geo, HyperTreeBase& tree, const 
 Tensor GeometryTensorQO::SampleVolumeIndirect(HyperTreeBase& tree, Tensor global_coordinate, Tensor node_id)
 {
     if (global_coordinate.numel() == 0) return global_coordinate;
-    // without gradients (evaluation) one kernel does both, where it takes the shapes
-    bool grad = false;
-    if (torch::GradMode::is_enabled()) {
-        grad = global_coordinate.requires_grad();
-        for (const auto* v : {&planes, &lines, &decoder.weight, &decoder.bias})
-            for (const auto& t : *v) grad = grad || t.requires_grad();
-    }
+    // without gradients (evaluation) one kernel does both, where it takes the
+    // shapes; forward-mode tangents go to the operators, which refuse them
+    const bool reverse = torch::GradMode::is_enabled();
+    auto wanted = [&](const Tensor& t) {
+        return t.defined() && ((reverse && t.requires_grad()) || t._fw_grad(/*level=*/0).defined());
+    };
+    bool grad = wanted(global_coordinate);
+    for (const auto* v : {&planes, &lines, &decoder.weight, &decoder.bias})
+        for (const auto& t : *v) grad = grad || wanted(t);
     if (!grad) {
         Tensor out = density_no_grad(*this, tree, global_coordinate, node_id);
         if (out.defined()) return out;

@@ -284,3 +284,35 @@ def test_grid_sample_without_memory_for_copies():
         del out, grads
     assert torch.equal(res[0][0], res[1][0]) and torch.equal(res[0][2], res[1][2])
     assert rel_err(res[1][1].numpy(), res[0][1].numpy()) < REL_TOL
+
+
+@pytest.mark.parametrize("which", ["position", "plane", "line", "weight", "bias"])
+@pytest.mark.parametrize("no_grad", [False, True])
+def test_density_refuses_tangents(which, no_grad):
+    """A forward-mode tangent is refused (the operators have no jvp), not
+    dropped, also where no reverse-mode gradient is wanted."""
+    import torch.autograd.forward_ad as fwd
+
+    tree, geo, _, _ = gpu_scene(1, 8, 9, (16, 9, 16), [32], 1)
+    pts = torch.rand(50, 3, generator=torch.Generator().manual_seed(2)).cuda()
+    node, _ = tree.NodeIdForPositionGPU(pts)
+    geo.planes, geo.lines = [t.detach() for t in geo.planes], [t.detach() for t in geo.lines]
+    geo.decoder_weight = [t.detach() for t in geo.decoder_weight]
+    geo.decoder_bias = [t.detach() for t in geo.decoder_bias]
+
+    def dual(v, i):
+        return [fwd.make_dual(t, torch.ones_like(t)) if k == i else t for k, t in enumerate(v)]
+
+    with fwd.dual_level(), torch.set_grad_enabled(not no_grad):
+        if which == "position":
+            pts = fwd.make_dual(pts, torch.ones_like(pts))
+        elif which == "plane":
+            geo.planes = dual(geo.planes, 2)
+        elif which == "line":
+            geo.lines = dual(geo.lines, 1)
+        elif which == "weight":
+            geo.decoder_weight = dual(geo.decoder_weight, 1)
+        else:
+            geo.decoder_bias = dual(geo.decoder_bias, 0)
+        with pytest.raises(RuntimeError, match="jvp"):
+            geo.SampleVolumeIndirect(tree, pts, node)
