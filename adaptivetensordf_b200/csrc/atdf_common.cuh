@@ -24,6 +24,21 @@ __device__ __forceinline__ void set_err(int32_t* e, int32_t bit)
     if (e) atomicOr(e, bit);
 }
 
+// Lets fn take dynamic shared memory up to the device's limit. The attribute
+// belongs to the kernel, not to a launch: set to the size of each launch, a host
+// thread could lower it between another's set and launch. Every call sets the
+// same value.
+inline int allow_dynamic_shared(const void* fn)
+{
+    int dev = 0, optin = 0;
+    cudaFuncAttributes a;
+    ATDF_CUDA_TRY(cudaGetDevice(&dev));
+    ATDF_CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    ATDF_CUDA_TRY(cudaFuncGetAttributes(&a, fn));
+    ATDF_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)a.sharedSizeBytes));
+    return ATDF_OK;
+}
+
 __host__ __device__ __forceinline__ int64_t div_up(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
 // ---------------------------------------------------------------------------
