@@ -14,6 +14,7 @@
 // kernels.
 
 #include <algorithm>
+#include <cfloat>
 #include <type_traits>
 
 #include "atdf_common.cuh"
@@ -103,13 +104,16 @@ __device__ void load_weights(const atdf_mlp_t& m, const Plan& pl, float* sm, boo
     }
 }
 
+__device__ __forceinline__ bool not_finite(float v) { return !(fabsf(v) <= FLT_MAX); }
+
 // Rows [row0, row0 + T) of x [S][n] into dst [T][pitch] (zeros past S and in
-// the columns n .. round4(n)).
+// the columns n .. round4(n)). Returns whether the thread met an infinity or NaN.
 template <int NT, int T>
-__device__ __forceinline__ void load_rows(const float* __restrict__ x, int64_t row0, int64_t S, int n, float* dst)
+__device__ __forceinline__ bool load_rows(const float* __restrict__ x, int64_t row0, int64_t S, int n, float* dst)
 {
     const int pitch = pitch_of(n), n4 = round4(n) / 4;
     const bool vec = n % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
+    bool wild = false;
     for (int i = threadIdx.x; i < T * n4; i += NT) {
         const int r = i / n4, c = i % n4 * 4;
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -125,7 +129,9 @@ __device__ __forceinline__ void load_rows(const float* __restrict__ x, int64_t r
             }
         }
         *reinterpret_cast<float4*>(dst + r * pitch + c) = v;
+        wild = wild || not_finite(v.x) || not_finite(v.y) || not_finite(v.z) || not_finite(v.w);
     }
+    return wild;
 }
 
 // acc = A B^T for RM rows (row0 + RG i) and CN columns (col0 + 16 j), K contiguous.
@@ -249,17 +255,22 @@ __global__ void __launch_bounds__(NT, 384 / NT)
 
 // gW [on][ip] += D^T H over the tile's T rows: 8 x 4 values a thread; where
 // that leaves threads idle, the rows are split over groups of threads, which
-// add their sums one after the other.
+// add their sums one after the other. wild: H holds infinities or NaN, whose
+// products with a zero D do not count (rows that want no gradient must not
+// spoil the others' sums): a thread a weight then, as for few outputs.
 template <int NT, int T>
 __device__ __forceinline__ void weight_gradient(const float* D, int dp, const float* H, int ip, int in, int on,
-                                                float* gw)
+                                                float* gw, bool wild)
 {
-    if (on <= 4) {  // a thread per weight (and group of rows)
+    if (on <= 4 || wild) {  // a thread per weight (and group of rows)
         const int n = on * in, g = max(1, min(NT / n, T / 8)), per = (T + g - 1) / g;
         for (int e = threadIdx.x; e < n * g; e += NT) {
             const int o = e % n / in, k = e % n % in, s0 = e / n * per, s1 = min(T, s0 + per);
             float s = 0.0f;
-            for (int r = s0; r < s1; ++r) s = fmaf(D[r * dp + o], H[r * ip + k], s);
+            for (int r = s0; r < s1; ++r) {
+                const float d = D[r * dp + o];
+                if (!wild || d != 0.0f) s = fmaf(d, H[r * ip + k], s);
+            }
             atomicAdd(&gw[o * ip + k], s);
         }
         __syncthreads();
@@ -309,7 +320,7 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 3 : 1)
     const int L = m.num_layers, last_n = m.dims[L];
     for (int64_t row0 = (int64_t)blockIdx.x * T; row0 < S; row0 += (int64_t)gridDim.x * T) {
         __syncthreads();
-        load_rows<NT, T>(x, row0, S, m.dims[0], sm + pl.h[0]);
+        bool wild = load_rows<NT, T>(x, row0, S, m.dims[0], sm + pl.h[0]);
         __syncthreads();
         // forward: h[l + 1] = activation, d[l] = derivative (last layer: dA)
         for (int l = 0; l < L; ++l) {
@@ -327,10 +338,12 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 3 : 1)
                                        g = real && row0 + r < S ? g * gout[(row0 + r) * last_n + c] : 0.0f;
                                    else
                                        h[r * np + c] = act_v;
+                                   wild = wild || not_finite(act_v);
                                    d[r * np + c] = g;
                                });
             __syncthreads();
         }
+        wild = __syncthreads_or(wild) != 0;
         // adjoint, last layer first: d[l] holds dA
         for (int l = L - 1; l >= 0; --l) {
             const int in = m.dims[l], on = m.dims[l + 1], ip = pitch_of(in), op = pitch_of(on);
@@ -355,7 +368,7 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 3 : 1)
                     }
                 });
             }
-            weight_gradient<NT, T>(D, op, sm + pl.h[l], ip, in, on, sm + pl.gw[l]);
+            weight_gradient<NT, T>(D, op, sm + pl.h[l], ip, in, on, sm + pl.gw[l], wild);
         }
     }
     __syncthreads();

@@ -316,3 +316,29 @@ def test_density_refuses_tangents(which, no_grad):
             geo.decoder_bias = dual(geo.decoder_bias, 0)
         with pytest.raises(RuntimeError, match="jvp"):
             geo.SampleVolumeIndirect(tree, pts, node)
+
+
+@pytest.mark.parametrize("dims", [[8, 32, 1], [16, 64, 64, 3], [12, 20, 17], [256, 256, 256, 1]])
+@pytest.mark.parametrize("value", [float("nan"), float("inf"), -float("inf")])
+def test_decoder_rows_without_gradient(dims, value):
+    """Rows that are not finite and want no gradient leave the weights'
+    gradients as they are without them (relu, whose derivative is finite
+    everywhere)."""
+    import adaptivetensordf_b200 as ab
+
+    S = 333
+    g = torch.Generator().manual_seed(sum(dims))
+    ws = [torch.randn(b, a, generator=g) * (2.0 / a) ** 0.5 for a, b in zip(dims, dims[1:])]
+    bs = [torch.rand(b, generator=g) - 0.5 for b in dims[1:]]
+    x, gy = torch.randn(S, dims[0], generator=g), torch.randn(S, dims[-1], generator=g)
+    masked = torch.arange(S) % 7 == 3
+    gy[masked] = 0.0
+    res = []
+    for fill in (0.0, value):
+        x[masked, : dims[0] // 2] = fill
+        leaf = [t.clone().cuda().requires_grad_(True) for t in ws + bs]
+        y = ab.DecodeFeatures(leaf[: len(ws)], leaf[len(ws):], "relu", "id", 1.0, x.cuda())
+        y.backward(gy.cuda())
+        res.append([t.grad.cpu().numpy() for t in leaf])
+    for got, want in zip(res[1], res[0]):
+        assert rel_err(got, want) < REL_TOL
