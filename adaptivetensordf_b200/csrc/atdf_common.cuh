@@ -26,10 +26,12 @@ __device__ __forceinline__ void set_err(int32_t* e, int32_t bit)
 
 // Lets fn take dynamic shared memory up to the device's limit. The attribute
 // belongs to the kernel, not to a launch: set to the size of each launch, a host
-// thread could lower it between another's set and launch. Every call sets the
-// same value.
-inline int allow_dynamic_shared(const void* fn)
+// thread could lower it between another's set and launch. Every call that needs
+// more than the default (48 KB with up to 8 KB of static arrays) sets the same
+// value.
+inline int allow_dynamic_shared(const void* fn, int smem)
 {
+    if (smem <= 40 * 1024) return ATDF_OK;
     int dev = 0, optin = 0;
     cudaFuncAttributes a;
     ATDF_CUDA_TRY(cudaGetDevice(&dev));

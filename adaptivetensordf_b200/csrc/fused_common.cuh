@@ -702,7 +702,7 @@ static inline int launch_tc_persistent(void (*fn)(FusedParams), int threads, int
     ATDF_CUDA_TRY(cudaGetDevice(&dev));
     ATDF_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     ATDF_CUDA_TRY(cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
-    if (const int e = allow_dynamic_shared((const void*)fn)) return e;
+    if (const int e = allow_dynamic_shared((const void*)fn, smem)) return e;
     // staged planes want the whole carve-out; a forward by runs leaves the rest
     // of the L1 to the texels
     const int carveout =

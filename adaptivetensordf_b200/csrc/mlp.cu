@@ -514,7 +514,7 @@ template <class Fn, class... Args>
 static int launch_tiles(Fn fn, Shape sh, const mlp::Plan& plan, int64_t S, int sms, cudaStream_t st, Args... args)
 {
     const int smem = plan.total * 4;
-    if (const int e = allow_dynamic_shared((const void*)fn)) return e;
+    if (const int e = allow_dynamic_shared((const void*)fn, smem)) return e;
     int per = 0;
     ATDF_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, (const void*)fn, sh.nt, smem));
     if (per < 1) return ATDF_ERR_CUDA;

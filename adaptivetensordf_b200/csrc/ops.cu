@@ -783,7 +783,7 @@ int atdf_grid_sample1d_backward(const float* grid, int64_t N, int64_t C, int64_t
     if (smem_sum) {
         int dev = 0, sms = 0, per = 0;
         const int smem = (int)(N * C * W * 4);
-        if (const int e = allow_dynamic_shared((const void*)gs1_bwd_kernel)) return e;
+        if (const int e = allow_dynamic_shared((const void*)gs1_bwd_kernel, smem)) return e;
         ATDF_CUDA_TRY(cudaGetDevice(&dev));
         ATDF_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
         ATDF_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, (const void*)gs1_bwd_kernel, 256, smem));
@@ -885,7 +885,7 @@ int atdf_vm_features_backward(const atdf_field_t* field, const float* pmin, cons
     const int smem = smem_lines ? (int)line_bytes : 0;
     unsigned blocks = blocks_for(threads);
     if (smem_lines) {
-        if (const int e = allow_dynamic_shared((const void*)kernel)) return e;
+        if (const int e = allow_dynamic_shared((const void*)kernel, smem)) return e;
         int dev = 0, sms = 0, per = 0;
         ATDF_CUDA_TRY(cudaGetDevice(&dev));
         ATDF_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
