@@ -104,16 +104,13 @@ __device__ void load_weights(const atdf_mlp_t& m, const Plan& pl, float* sm, boo
     }
 }
 
-__device__ __forceinline__ bool not_finite(float v) { return !(fabsf(v) <= FLT_MAX); }
-
 // Rows [row0, row0 + T) of x [S][n] into dst [T][pitch] (zeros past S and in
-// the columns n .. round4(n)). Returns whether the thread met an infinity or NaN.
+// the columns n .. round4(n)).
 template <int NT, int T>
-__device__ __forceinline__ bool load_rows(const float* __restrict__ x, int64_t row0, int64_t S, int n, float* dst)
+__device__ __forceinline__ void load_rows(const float* __restrict__ x, int64_t row0, int64_t S, int n, float* dst)
 {
     const int pitch = pitch_of(n), n4 = round4(n) / 4;
     const bool vec = n % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
-    bool wild = false;
     for (int i = threadIdx.x; i < T * n4; i += NT) {
         const int r = i / n4, c = i % n4 * 4;
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -129,9 +126,7 @@ __device__ __forceinline__ bool load_rows(const float* __restrict__ x, int64_t r
             }
         }
         *reinterpret_cast<float4*>(dst + r * pitch + c) = v;
-        wild = wild || not_finite(v.x) || not_finite(v.y) || not_finite(v.z) || not_finite(v.w);
     }
-    return wild;
 }
 
 // acc = A B^T for RM rows (row0 + RG i) and CN columns (col0 + 16 j), K contiguous.
@@ -255,21 +250,24 @@ __global__ void __launch_bounds__(NT, 384 / NT)
 
 // gW [on][ip] += D^T H over the tile's T rows: 8 x 4 values a thread; where
 // that leaves threads idle, the rows are split over groups of threads, which
-// add their sums one after the other. wild: H holds infinities or NaN, whose
-// products with a zero D do not count (rows that want no gradient must not
-// spoil the others' sums): a thread a weight then, as for few outputs.
+// add their sums one after the other. skip_zeros: without the products of a
+// zero in D, a thread a weight as for few outputs.
 template <int NT, int T>
 __device__ __forceinline__ void weight_gradient(const float* D, int dp, const float* H, int ip, int in, int on,
-                                                float* gw, bool wild)
+                                                float* gw, bool skip_zeros)
 {
-    if (on <= 4 || wild) {  // a thread per weight (and group of rows)
+    if (on <= 4 || skip_zeros) {  // a thread per weight (and group of rows)
         const int n = on * in, g = max(1, min(NT / n, T / 8)), per = (T + g - 1) / g;
         for (int e = threadIdx.x; e < n * g; e += NT) {
             const int o = e % n / in, k = e % n % in, s0 = e / n * per, s1 = min(T, s0 + per);
             float s = 0.0f;
-            for (int r = s0; r < s1; ++r) {
-                const float d = D[r * dp + o];
-                if (!wild || d != 0.0f) s = fmaf(d, H[r * ip + k], s);
+            if (skip_zeros) {
+                for (int r = s0; r < s1; ++r) {
+                    const float d = D[r * dp + o];
+                    if (d != 0.0f) s = fmaf(d, H[r * ip + k], s);
+                }
+            } else {
+                for (int r = s0; r < s1; ++r) s = fmaf(D[r * dp + o], H[r * ip + k], s);
             }
             atomicAdd(&gw[o * ip + k], s);
         }
@@ -318,60 +316,75 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 3 : 1)
     extern __shared__ __align__(16) float sm[];
     load_weights<NT>(m, pl, sm, true);
     const int L = m.num_layers, last_n = m.dims[L];
-    for (int64_t row0 = (int64_t)blockIdx.x * T; row0 < S; row0 += (int64_t)gridDim.x * T) {
-        __syncthreads();
-        bool wild = load_rows<NT, T>(x, row0, S, m.dims[0], sm + pl.h[0]);
-        __syncthreads();
-        // forward: h[l + 1] = activation, d[l] = derivative (last layer: dA)
-        for (int l = 0; l < L; ++l) {
-            const int in = m.dims[l], on = m.dims[l + 1], np = pitch_of(on);
-            const bool last = l == L - 1;
-            const float* bias = sm + pl.b[l];
-            float* d = sm + pl.d[l];
-            float* h = sm + (last ? 0 : pl.h[l + 1]);
-            const int act = last ? m.last_activation : m.hidden_activation;
-            tile_layer<NT, RM>(sm + pl.h[l], pitch_of(in), sm + pl.w[l], pitch_of(in), round4(in), on, bias,
-                               [&](int r, int c, float v, bool real) {
-                                   float act_v = 0.0f, g = 0.0f;
-                                   if (real) act_pair(act, v, m.softplus_beta, act_v, g);
-                                   if (last)
-                                       g = real && row0 + r < S ? g * gout[(row0 + r) * last_n + c] : 0.0f;
-                                   else
-                                       h[r * np + c] = act_v;
-                                   wild = wild || not_finite(act_v);
-                                   d[r * np + c] = g;
-                               });
+    // The products of a row that wants no gradient count as nothing, also with
+    // infinite or NaN inputs. The fast products add 0 * input like any other, so
+    // a block whose sums are not finite takes its rows again without the zeros.
+    for (bool skip_zeros = false;; skip_zeros = true) {
+        for (int64_t row0 = (int64_t)blockIdx.x * T; row0 < S; row0 += (int64_t)gridDim.x * T) {
             __syncthreads();
-        }
-        wild = __syncthreads_or(wild) != 0;
-        // adjoint, last layer first: d[l] holds dA
-        for (int l = L - 1; l >= 0; --l) {
-            const int in = m.dims[l], on = m.dims[l + 1], ip = pitch_of(in), op = pitch_of(on);
-            const float* D = sm + pl.d[l];
-            {  // bias: column sums, a thread per output and group of rows
-                const int g = max(1, min(NT / on, T / 8)), per = (T + g - 1) / g;
-                for (int e = threadIdx.x; e < on * g; e += NT) {
-                    const int o = e % on, s0 = e / on * per, s1 = min(T, s0 + per);
-                    float s = 0.0f;
-                    for (int r = s0; r < s1; ++r) s += D[r * op + o];
-                    atomicAdd(&sm[pl.gb[l] + o], s);
-                }
+            load_rows<NT, T>(x, row0, S, m.dims[0], sm + pl.h[0]);
+            __syncthreads();
+            // forward: h[l + 1] = activation, d[l] = derivative (last layer: dA)
+            for (int l = 0; l < L; ++l) {
+                const int in = m.dims[l], on = m.dims[l + 1], np = pitch_of(on);
+                const bool last = l == L - 1;
+                const float* bias = sm + pl.b[l];
+                float* d = sm + pl.d[l];
+                float* h = sm + (last ? 0 : pl.h[l + 1]);
+                const int act = last ? m.last_activation : m.hidden_activation;
+                tile_layer<NT, RM>(sm + pl.h[l], pitch_of(in), sm + pl.w[l], pitch_of(in), round4(in), on, bias,
+                                   [&](int r, int c, float v, bool real) {
+                                       float act_v = 0.0f, g = 0.0f;
+                                       if (real) act_pair(act, v, m.softplus_beta, act_v, g);
+                                       if (last)
+                                           g = real && row0 + r < S ? g * gout[(row0 + r) * last_n + c] : 0.0f;
+                                       else
+                                           h[r * np + c] = act_v;
+                                       d[r * np + c] = g;
+                                   });
+                __syncthreads();
             }
-            if (l > 0 || gx) {
-                float* dn = sm + (l > 0 ? pl.d[l - 1] : 0);
-                tile_layer<NT, RM>(D, op, sm + pl.wt[l], op, round4(on), in, nullptr, [&](int r, int c, float v, bool real) {
-                    if (!real) return;
-                    if (l > 0) {  // the derivative there is read and replaced by this thread alone
-                        dn[r * ip + c] *= v;
-                    } else if (row0 + r < S) {
-                        gx[(row0 + r) * in + c] = v;
+            // adjoint, last layer first: d[l] holds dA
+            for (int l = L - 1; l >= 0; --l) {
+                const int in = m.dims[l], on = m.dims[l + 1], ip = pitch_of(in), op = pitch_of(on);
+                const float* D = sm + pl.d[l];
+                {  // bias: column sums, a thread per output and group of rows
+                    const int g = max(1, min(NT / on, T / 8)), per = (T + g - 1) / g;
+                    for (int e = threadIdx.x; e < on * g; e += NT) {
+                        const int o = e % on, s0 = e / on * per, s1 = min(T, s0 + per);
+                        float s = 0.0f;
+                        for (int r = s0; r < s1; ++r) s += D[r * op + o];
+                        atomicAdd(&sm[pl.gb[l] + o], s);
                     }
-                });
+                }
+                if (l > 0 || gx) {
+                    float* dn = sm + (l > 0 ? pl.d[l - 1] : 0);
+                    tile_layer<NT, RM>(D, op, sm + pl.wt[l], op, round4(on), in, nullptr, [&](int r, int c, float v, bool real) {
+                        if (!real) return;
+                        if (l > 0) {  // the derivative there is read and replaced by this thread alone
+                            dn[r * ip + c] *= v;
+                        } else if (row0 + r < S) {
+                            gx[(row0 + r) * in + c] = v;
+                        }
+                    });
+                }
+                weight_gradient<NT, T>(D, op, sm + pl.h[l], ip, in, on, sm + pl.gw[l], skip_zeros);
             }
-            weight_gradient<NT, T>(D, op, sm + pl.h[l], ip, in, on, sm + pl.gw[l], wild);
+        }
+        __syncthreads();
+        float wild = 0.0f;  // NaN as soon as a sum (or a padding column's product) is not finite
+        for (int l = 0; l < L; ++l)
+            for (int i = threadIdx.x * 4; i < m.dims[l + 1] * pitch_of(m.dims[l]); i += NT * 4) {
+                const float4 v = *reinterpret_cast<const float4*>(sm + pl.gw[l] + i);
+                wild += v.x * 0.0f + v.y * 0.0f + v.z * 0.0f + v.w * 0.0f;
+            }
+        if (__syncthreads_and(wild == 0.0f) || skip_zeros) break;
+        for (int l = 0; l < L; ++l) {
+            const int on = m.dims[l + 1];
+            for (int i = threadIdx.x; i < ((on + 7) & ~7) * pitch_of(m.dims[l]); i += NT) sm[pl.gw[l] + i] = 0.0f;
+            for (int i = threadIdx.x; i < on; i += NT) sm[pl.gb[l] + i] = 0.0f;
         }
     }
-    __syncthreads();
     for (int l = 0; l < L; ++l) {
         const int in = m.dims[l], on = m.dims[l + 1], ip = pitch_of(in);
         if (gr.weight[l])
