@@ -306,14 +306,15 @@ __device__ __forceinline__ int pop_item(const Ws& w, int queue, int* s_ctl)
     return flags;
 }
 
+// Only the tensor-core kernels stage planes: BF16 (plane_off counts elements).
+constexpr int kPlaneBytes = 2;
+
 // Bytes of a slot's three planes, announced to bar by one thread.
 __device__ __forceinline__ void expect_planes(const FusedParams& p, uint64_t* bar)
 {
-    // plane_off counts elements of the plane type (4 or 2 bytes)
-    const int esz = p.field.dtype == ATDF_BF16 ? 2 : 4;
     uint32_t bytes = 0;
     for (int m = 0; m < 3; ++m)
-        bytes += (uint32_t)(p.field.plane_h[m] * p.field.plane_w[m] * p.field.channels * esz);
+        bytes += (uint32_t)(p.field.plane_h[m] * p.field.plane_w[m] * p.field.channels * kPlaneBytes);
     mbar_expect_tx(bar, bytes);
 }
 
@@ -321,23 +322,22 @@ __device__ __forceinline__ void expect_planes(const FusedParams& p, uint64_t* ba
 __device__ __forceinline__ void stage_planes(const FusedParams& p, float* sm, int64_t sl, uint64_t* bar)
 {
     const int lane = threadIdx.x & 31;
-    const int esz = p.field.dtype == ATDF_BF16 ? 2 : 4;
     fence_proxy_async();
     // copy c of plane m: its whole plane (unpadded) or its row c (padded)
     int c0 = 0;
     for (int m = 0; m < 3; ++m) {
         const int64_t pf = (int64_t)p.field.plane_h[m] * p.field.plane_w[m] * p.field.channels;
-        char* dst = reinterpret_cast<char*>(sm) + (size_t)p.plane_off[m] * esz;
-        const char* src = reinterpret_cast<const char*>(p.field.plane[m]) + (size_t)sl * pf * esz;
+        char* dst = reinterpret_cast<char*>(sm) + (size_t)p.plane_off[m] * kPlaneBytes;
+        const char* src = reinterpret_cast<const char*>(p.field.plane[m]) + (size_t)sl * pf * kPlaneBytes;
         const bool padded = p.plane_pitch[m] != p.field.plane_w[m];
         const int ncopy = padded ? p.field.plane_h[m] : 1;
-        const uint32_t row = (uint32_t)(p.field.plane_w[m] * p.field.channels * esz);
-        const uint32_t pitch = (uint32_t)(p.plane_pitch[m] * p.field.channels * esz);
+        const uint32_t row = (uint32_t)(p.field.plane_w[m] * p.field.channels * kPlaneBytes);
+        const uint32_t pitch = (uint32_t)(p.plane_pitch[m] * p.field.channels * kPlaneBytes);
         for (int c = ((lane - c0) % 32 + 32) % 32; c < ncopy; c += 32) {
             if (padded)
                 tma_bulk_load(dst + (size_t)c * pitch, src + (size_t)c * row, row, bar);
             else
-                tma_bulk_load(dst, src, (uint32_t)(pf * esz), bar);
+                tma_bulk_load(dst, src, (uint32_t)(pf * kPlaneBytes), bar);
         }
         c0 += ncopy;
     }
@@ -556,8 +556,7 @@ __device__ __forceinline__ ItemInfo next_item(const FusedParams& p, int queue, f
     return info;
 }
 
-// Geometry of sample k of the current item (computed by all 8 threads of the
-// sample): segment index, weight, position.
+// Geometry of sample k of the current item: segment index, weight, position.
 struct SampleState {
     int si;
     float w;
@@ -680,13 +679,21 @@ __device__ __forceinline__ void add_to_bins(const FusedParams& p, const SegTab& 
 // 24 samples a segment, by slot and by runs, 1000 rays at depth 4: 231 and 110
 // us; 4096 rays: 299 and 244; 1000 rays at depth 2: 90 and 67. With more
 // segments the staged planes are read faster: 8192 rays at depth 4: 430 and
-// 474, 16384 rays: 669 and 741, at depth 3: 361 and 418. The line lies between
-// (4096 rays at depth 4 are 208,896 segments by capacity). 24 channels, whose
-// planes take half again the staging, stay level or better by runs wherever the
-// slots are many: 4096 slots of depth 6, 119 samples a segment, 4096 rays 315 and
-// 243 us, 16384 rays 759 and 734; depth 4, 16384 rays 678 and 668, 65536 rays
-// 2401 and 2339. Not so with 512 slots (16384 rays 370 and 396) or beyond
-// (65536 rays at depth 6: 2548 and 2607).
+// 474, 16384 rays: 669 and 741, at depth 3: 361 and 418.
+// The host knows the segments by capacity only (3 * 2^depth + 3 a ray), so that
+// is what the line is drawn by: exact for full trees (4096 rays at depth 4 are
+// 208,896), early for adaptive ones, whose rays meet a few per cent of it. 16
+// channels, depth 6, 80 samples a segment, 4096 leaves, by slot and by runs:
+// 1300 rays (the last below the line) 173 and 123 us, beyond it by slot although
+// runs are faster up to about 8192 rays (4096: 269 and 196, 8192: 380 and 321,
+// 16384: 575 and 586; 400 leaves: 190 and 142, 216 and 228, 349 and 378). Below
+// the line the runs' worst is a tree of few leaves under few rays (400 leaves,
+// 256 rays: 74 and 84). 24 channels, whose planes take half again the staging,
+// stay level or better by runs wherever the slots are many: 4096 slots of depth
+// 6, 119 samples a segment, 4096 rays 315 and 243 us, 16384 rays 759 and 734;
+// depth 4, 16384 rays 678 and 668, 65536 rays 2401 and 2339. Not so with 512
+// slots (16384 rays 370 and 396) or beyond (65536 rays at depth 6: 2548 and
+// 2607).
 static inline bool forward_by_runs(const FusedParams& p)
 {
     if (p.ws.cap <= (1 << 18)) return true;
@@ -694,9 +701,10 @@ static inline bool forward_by_runs(const FusedParams& p)
 }
 
 // Launches a persistent tensor-core kernel with `most` CTAs an SM (by its TMEM
-// columns and launch bounds) or what shared memory leaves of them.
-static inline int launch_tc_persistent(void (*fn)(FusedParams), int threads, int smem, int most, cudaStream_t st,
-                                       const FusedParams& p)
+// columns and launch bounds) or what shared memory leaves of them. staged: the
+// planes are copied to shared memory.
+static inline int launch_tc_persistent(void (*fn)(FusedParams), int threads, int smem, int most, bool staged,
+                                       cudaStream_t st, const FusedParams& p)
 {
     int dev = 0, sms = 0, smem_sm = 0, per = 0;
     ATDF_CUDA_TRY(cudaGetDevice(&dev));
@@ -706,7 +714,7 @@ static inline int launch_tc_persistent(void (*fn)(FusedParams), int threads, int
     // staged planes want the whole carve-out; a forward by runs leaves the rest
     // of the L1 to the texels
     const int carveout =
-        most == 4 ? std::min(100, most * (smem + 1536) * 100 / smem_sm + 1) : (int)cudaSharedmemCarveoutMaxShared;
+        staged ? (int)cudaSharedmemCarveoutMaxShared : std::min(100, most * (smem + 1536) * 100 / smem_sm + 1);
     ATDF_CUDA_TRY(cudaFuncSetAttribute((const void*)fn, cudaFuncAttributePreferredSharedMemoryCarveout, carveout));
     ATDF_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, (const void*)fn, threads, smem));
     if (per < 1) return ATDF_ERR_UNSUPPORTED;

@@ -20,8 +20,8 @@
 // bytes a cycle and SM from L1/L2 as from shared memory, and vector
 // reductions into L2 add 4.2 floats a cycle and SM without waiting, where
 // shared-memory float atomics (a compare-and-swap loop) add 1.7 to 3.1. That
-// leaves shared memory to two blocks an SM, whose phases overlap, and lets
-// any block take any item: a slot's items need not share a block.
+// leaves room for two blocks an SM in the adjoint of two hidden layers and three
+// in the other kernels, whose phases overlap, and lets any block take any item: a slot's items need not share a block.
 #pragma once
 
 #include "fused_common.cuh"
@@ -294,40 +294,37 @@ __device__ __forceinline__ void decode_tile(float* sm, int rg, int cg, int cw, i
     using K = Cfg<C, MODE, H, NH>;
     using S = Smem<C, MODE, H, NH, false>;
     const int tid = threadIdx.x;
-                    uint64_t acc[8][4];
-                    layer0<C, MODE, H, NH, false>(sm, rg, cg, acc);
-                    // every warp has read all rows of x before any of them
-                    // gathers the geometry pass's next tile into it (two
-                    // hidden layers: the barrier after H0)
-                    if (NH == 1 && K::T < kGeo) __syncthreads();
-                    if (NH == 2) {
-    #pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            const float b = sm[S::b0 + cg + j * K::CG];
-    #pragma unroll
-                            for (int i = 0; i < 8; ++i)
-                                sm[S::h + (rg + i * K::RG) * K::HP + cg + j * K::CG] =
-                                    act_hidden(hact, sum2(acc[i][j]) + b, beta);
-                        }
-                        __syncthreads();
-                        zero2<8, 4>(acc);
-                        gemm_k<8, 4, H>(acc, sm + S::h + rg * K::HP, K::RG * K::HP, sm + S::w1 + cg * K::HP,
-                                        K::CG * K::HP);
-                    }
-                    // the last layer's sums over the thread's columns
-                    float z[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        const int c = cg + j * K::CG;
-                        const float b = sm[(NH == 2 ? S::b1 : S::b0) + c], wl = sm[S::wl + c];
-    #pragma unroll
-                        for (int i = 0; i < 8; ++i) z[i] = fmaf(act_hidden(hact, sum2(acc[i][j]) + b, beta), wl, z[i]);
-                    }
-    #pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        z[i] = sum_cols(z[i]);
-                        if ((tid & 6) == 0) sm[S::zp + cw * S::zrow + s0 + rg + i * K::RG] = z[i];
-                    }
+    uint64_t acc[8][4];
+    layer0<C, MODE, H, NH, false>(sm, rg, cg, acc);
+    // every warp has read all rows of x before any of them gathers the geometry
+    // pass's next tile into it (two hidden layers: the barrier after H0)
+    if (NH == 1 && K::T < kGeo) __syncthreads();
+    if (NH == 2) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float b = sm[S::b0 + cg + j * K::CG];
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                sm[S::h + (rg + i * K::RG) * K::HP + cg + j * K::CG] = act_hidden(hact, sum2(acc[i][j]) + b, beta);
+        }
+        __syncthreads();
+        zero2<8, 4>(acc);
+        gemm_k<8, 4, H>(acc, sm + S::h + rg * K::HP, K::RG * K::HP, sm + S::w1 + cg * K::HP, K::CG * K::HP);
+    }
+    // the last layer's sums over the thread's columns
+    float z[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int c = cg + j * K::CG;
+        const float b = sm[(NH == 2 ? S::b1 : S::b0) + c], wl = sm[S::wl + c];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) z[i] = fmaf(act_hidden(hact, sum2(acc[i][j]) + b, beta), wl, z[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        z[i] = sum_cols(z[i]);
+        if ((tid & 6) == 0) sm[S::zp + cw * S::zrow + s0 + rg + i * K::RG] = z[i];
+    }
 }
 
 template <int C, int MODE, int H, int NH>

@@ -1031,7 +1031,7 @@ static int launch_tc(void (*fn)(FusedParams), bool bwd, const FusedParams& p, cu
     int smem = (int)tcf::TCSmem(p.plane_off[3], p.gplane_off[3], bwd).total;
     if (smem > max_optin()) return ATDF_ERR_UNSUPPORTED;
     if (runs) smem = (int)tcf::TCSmem().total;
-    return launch_tc_persistent(fn, threads, smem, bwd ? 1 : runs ? 4 : 2, st, p);
+    return launch_tc_persistent(fn, threads, smem, bwd ? 1 : runs ? 4 : 2, !runs, st, p);
 }
 
 int launch_tc_forward(const FusedParams& p, cudaStream_t st)

@@ -1090,13 +1090,13 @@ bool tc24_supported(const atdf_field_t* f, const atdf_mlp_t* m)
 static int launch24(void (*fn)(FusedParams), bool bwd, const FusedParams& p, cudaStream_t st, bool runs = false)
 {
     int smem = (int)tc24::Smem24(p.plane_off[3], p.gplane_off[3], bwd).total;
-    int dev = 0, optin = 0, sms = 0;
+    int dev = 0, optin = 0;
     ATDF_CUDA_TRY(cudaGetDevice(&dev));
     ATDF_CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     if (smem > optin) return ATDF_ERR_UNSUPPORTED;
     if (runs) smem = (int)tc24::Smem24().total;
     const int threads = bwd ? tc24::kThreadsB : runs ? tc24::kRows : tc24::kThreadsF;
-    return launch_tc_persistent(fn, threads, smem, bwd ? 1 : runs ? 4 : 2, st, p);
+    return launch_tc_persistent(fn, threads, smem, bwd ? 1 : runs ? 4 : 2, !runs, st, p);
 }
 
 int launch_tc24_forward(const FusedParams& p, cudaStream_t st)

@@ -1,5 +1,5 @@
 // Register-tiled FP32 products of small matrices in shared memory, for the
-// decoder MLP on the CUDA cores (fused_simt.cuh, ops.cu).
+// decoder MLP on the CUDA cores (fused_simt.cuh, mlp.cu).
 //
 // Every operand is stored with the contraction index contiguous, so a thread
 // loads four of its values per row with one 16-byte load and multiplies them

@@ -269,8 +269,10 @@ int atdf_accumulate_loss_per_node(const float* per_ray_loss, int32_t channels, i
 
 /* The field and its decoder in one pass without gradients: out[i] = the
  * decoded density of point i in leaf node_id[i] (atdf_vm_features_forward then
- * atdf_mlp_forward). ATDF_ERR_UNSUPPORTED for shapes that the FP32 fused
- * projection does not take (compose the two entry points then). */
+ * atdf_mlp_forward). ATDF_ERR_UNSUPPORTED for channel counts, modes and decoders
+ * that the FP32 fused projection does not take and for planes or lines off a
+ * 16-byte boundary (compose the two entry points then). The projection's limit
+ * on the planes' size does not apply. */
 int atdf_field_density(const atdf_field_t* field, const atdf_mlp_t* mlp, const float* node_position_min,
                        const float* node_position_max, int64_t num_nodes, const float* position,
                        const int64_t* node_id, int64_t num_points, float* out, int32_t* dev_error,
