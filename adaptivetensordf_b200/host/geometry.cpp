@@ -79,6 +79,23 @@ static Tensor channels_last_copy(const Tensor& grid)
     return grid.permute({0, 2, 3, 1}).contiguous().permute({0, 3, 1, 2});
 }
 
+// The adjoint's channels-last kernel writes its gradient in that layout, and two
+// more passes over it (zeros and the copy to [N, C, H, W]) are what the strided
+// kernel, a thread per sample walking the channels, does without. For channels-
+// last grids (the others need 4 samples a texel for their copies as well) of up
+// to 2 M texels and 96 MB the passes hide behind the call: 4096 slots of 17^2, 16
+// channels, 1000 samples 93 us strided, 85 so; above, the strided kernel is the
+// faster one up to a sample per 10 + 2 C texels (16384 slots of 17^2 and 4 / 16 /
+// 32 channels level at 280 / 105 / 67 thousand samples; 1000 samples 79 / 128 /
+// 191 us strided and 107 / 256 / 462 so).
+static bool adjoint_in_channels_last(const Tensor& grid, int64_t samples)
+{
+    const int64_t texels = grid.size(0) * grid.size(2) * grid.size(3);
+    return samples > 0 && samples_in_channels_last(grid, samples) &&
+           (4 * samples >= texels || (texels <= (2 << 20) && grid.numel() <= (24 << 20)) ||
+            texels <= samples * (10 + 2 * grid.size(1)));
+}
+
 // Runs the allocations of a path that trades memory for speed; false where they
 // do not fit, and the caller takes the path that needs none of them.
 template <class Alloc>
@@ -129,7 +146,7 @@ class GridSample2DFn : public torch::autograd::Function<GridSample2DFn> {
         auto g = go[0].contiguous();
         auto guv = torch::zeros_like(u);
         auto err = ctx->saved_data["err"].toTensor();
-        if (samples_in_channels_last(grid, idx.size(0)) && idx.size(0) > 0) {
+        if (adjoint_in_channels_last(grid, idx.size(0))) {
             Tensor grid_read, g_read, ggrid, out;
             if (if_memory_allows([&] {
                     grid_read = channels_last_copy(grid);

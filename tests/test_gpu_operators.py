@@ -342,3 +342,25 @@ def test_decoder_rows_without_gradient(dims, value):
         res.append([t.grad.cpu().numpy() for t in leaf])
     for got, want in zip(res[1], res[0]):
         assert rel_err(got, want) < REL_TOL
+
+
+@pytest.mark.parametrize("S", [50, 7300 * 289 // 18 - 1, 7300 * 289 // 18 + 1])
+def test_grid_sample_adjoint_of_a_large_channels_last_grid(oracle, S):
+    """Both sides of the line from which a channels-last grid of more than 2 M
+    texels takes the channels-last adjoint: a sample per 10 + 2 C texels."""
+    import adaptivetensordf_b200 as ab
+
+    shape = (7300, 4, 17, 17)
+    rng = np.random.default_rng(S)
+    g = rng.normal(size=shape).astype(np.float32)
+    idx = rng.integers(0, shape[0], S)
+    uv = rng.uniform(-1.2, 1.2, (S, 2)).astype(np.float32)
+    go = rng.normal(size=(S, 4)).astype(np.float32)
+    gt = torch.from_numpy(g).cuda().contiguous(memory_format=torch.channels_last).requires_grad_(True)
+    ut = torch.from_numpy(uv).cuda().requires_grad_(True)
+    out = ab.IndirectGridSample2D(gt, torch.from_numpy(idx).cuda(), ut)
+    assert np.array_equal(out.detach().cpu().numpy(), oracle.grid_sample2d(g, idx, uv, np.float32))
+    gg, gu = torch.autograd.grad(out, [gt, ut], torch.from_numpy(go).cuda())
+    assert gg.is_contiguous()
+    assert rel_err(gg.cpu().numpy(), oracle.grid_sample2d_bwd(g, idx, uv, go, np.float64)[0]) < REL_TOL
+    assert np.array_equal(gu.cpu().numpy(), oracle.grid_sample2d_bwd(g, idx, uv, go, np.float32)[1])
