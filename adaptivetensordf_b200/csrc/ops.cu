@@ -296,18 +296,18 @@ __global__ void gs1_fwd_kernel(const float* __restrict__ grid, int64_t N, int64_
     }
 }
 
-// smem_sum: the grid's gradient fits in shared memory. Every sample adds to
-// one of few entries, so each block sums its own copy there and adds it once;
+// SMEM_SUM: the grid's gradient fits in shared memory. Many samples add to
+// few entries, so each block sums its own copy there and adds it once;
 // larger grids take global atomics.
+template <bool SMEM_SUM>
 __global__ void __launch_bounds__(256)
     gs1_bwd_kernel(const float* __restrict__ grid, int64_t N, int64_t C, int W, int64_t sN, int64_t sC, int64_t sW,
                    const int64_t* __restrict__ index, const float* __restrict__ uv, int64_t S,
-                   const float* __restrict__ gout, float* __restrict__ ggrid, float* __restrict__ guv, bool smem_sum,
-                   int32_t* err)
+                   const float* __restrict__ gout, float* __restrict__ ggrid, float* __restrict__ guv, int32_t* err)
 {
     extern __shared__ float s_sum[];
     const int64_t total = N * C * W;
-    if (smem_sum) {
+    if (SMEM_SUM) {
         for (int64_t j = threadIdx.x; j < total; j += blockDim.x) s_sum[j] = 0.0f;
         __syncthreads();
     }
@@ -319,7 +319,7 @@ __global__ void __launch_bounds__(256)
         }
         const Corner1 k = corners1(uv[i], W);
         const float* g = grid + n * sN;
-        float* gg = smem_sum ? s_sum + n * C * W : ggrid ? ggrid + n * C * W : nullptr;
+        float* gg = SMEM_SUM ? s_sum + n * C * W : ggrid ? ggrid + n * C * W : nullptr;
         float gix = 0.0f;
         const float a1 = __fsub_rn(k.fx1, k.ix), a0 = __fsub_rn(k.ix, k.fx0);
         for (int64_t c = 0; c < C; ++c) {
@@ -334,7 +334,7 @@ __global__ void __launch_bounds__(256)
         }
         if (guv) guv[i] = __fadd_rn(guv[i], __fdiv_rn(__fmul_rn(gix, (float)(W - 1)), 2.0f));
     }
-    if (!smem_sum) return;
+    if (!SMEM_SUM) return;
     __syncthreads();
     for (int64_t j = threadIdx.x; j < total; j += blockDim.x) {
         const float v = s_sum[j];
@@ -777,20 +777,23 @@ int atdf_grid_sample1d_backward(const float* grid, int64_t N, int64_t C, int64_t
         return ATDF_ERR_INVALID_ARGUMENT;
     if (S == 0) return ATDF_OK;
     // a block's copy of the gradient: up to 64 KB, so that three blocks share an
-    // SM, and fewer entries than samples to sum
-    const bool smem_sum = grad_grid && N * C * W * 4 <= 64 * 1024 && N * W <= S;
+    // SM, and enough samples to repay clearing and adding it: 16 channels, global
+    // and shared, 17 entries, 1000 samples 10 and 21 us, 4000: 19 and 21, 16000: 72
+    // and 23; 1000 entries, 4000 samples 12 and 16, 20000: 15 and 17, 64000: 38 and 19
+    const bool smem_sum = grad_grid && N * C * W * 4 <= 64 * 1024 && S >= std::max<int64_t>(4096, 24 * N * W);
+    const size_t smem = smem_sum ? (size_t)(N * C * W * 4) : 0;
+    auto kernel = smem_sum ? gs1_bwd_kernel<true> : gs1_bwd_kernel<false>;
     unsigned blocks = blocks_for(S);
     if (smem_sum) {
         int dev = 0, sms = 0, per = 0;
-        const int smem = (int)(N * C * W * 4);
-        if (const int e = allow_dynamic_shared((const void*)gs1_bwd_kernel, smem)) return e;
+        if (const int e = allow_dynamic_shared((const void*)kernel, (int)smem)) return e;
         ATDF_CUDA_TRY(cudaGetDevice(&dev));
         ATDF_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        ATDF_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, (const void*)gs1_bwd_kernel, 256, smem));
+        ATDF_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, (const void*)kernel, 256, smem));
         if (per > 0 && blocks > (unsigned)(sms * per)) blocks = (unsigned)(sms * per);
     }
-    gs1_bwd_kernel<<<blocks, 256, smem_sum ? (size_t)(N * C * W * 4) : 0, (cudaStream_t)stream>>>(
-        grid, N, C, (int)W, s[0], s[1], s[2], index, uv, S, grad_out, grad_grid, grad_uv, smem_sum, dev_error);
+    kernel<<<blocks, 256, smem, (cudaStream_t)stream>>>(grid, N, C, (int)W, s[0], s[1], s[2], index, uv, S, grad_out,
+                                                        grad_grid, grad_uv, dev_error);
     ATDF_LAUNCH_CHECK();
     return ATDF_OK;
 }

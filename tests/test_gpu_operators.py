@@ -364,3 +364,24 @@ def test_grid_sample_adjoint_of_a_large_channels_last_grid(oracle, S):
     assert gg.is_contiguous()
     assert rel_err(gg.cpu().numpy(), oracle.grid_sample2d_bwd(g, idx, uv, go, np.float64)[0]) < REL_TOL
     assert np.array_equal(gu.cpu().numpy(), oracle.grid_sample2d_bwd(g, idx, uv, go, np.float32)[1])
+
+
+@pytest.mark.parametrize("shape,S", [((2, 7, 33, 1), 4095), ((2, 7, 33, 1), 4096), ((2, 7, 33, 1), 30001),
+                                     ((1, 5, 700, 1), 16799), ((1, 5, 700, 1), 16800), ((1, 3, 6000, 1), 144000)])
+def test_grid_sample_line_sums(oracle, shape, S):
+    """The line gradient's sums on both sides of 4096 samples and 24 an entry
+    (shared memory from there on), and lines beyond 64 KB."""
+    import adaptivetensordf_b200 as ab
+
+    rng = np.random.default_rng(S)
+    g = rng.normal(size=shape).astype(np.float32)
+    idx = rng.integers(0, shape[0], S)
+    u = rng.uniform(-1.1, 1.1, (S, 1)).astype(np.float32)
+    go = rng.normal(size=(S, shape[1])).astype(np.float32)
+    gt, ut = torch.from_numpy(g).cuda().requires_grad_(True), torch.from_numpy(u).cuda().requires_grad_(True)
+    out = ab.IndirectGridSample1D(gt, torch.from_numpy(idx).cuda(), ut)
+    assert np.array_equal(out.detach().cpu().numpy(), oracle.grid_sample1d(g, idx, u, np.float32))
+    out.backward(torch.from_numpy(go).cuda())
+    # the FP32 oracle's weights: at thousands of entries they are rounded by 1e-4 by definition
+    assert rel_err(gt.grad.cpu().numpy(), oracle.grid_sample1d_bwd(g, idx, u, go, np.float32)[0]) < REL_TOL
+    assert np.array_equal(ut.grad.cpu().numpy(), oracle.grid_sample1d_bwd(g, idx, u, go, np.float32)[1])
